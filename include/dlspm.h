@@ -283,9 +283,9 @@ int dlspm_sddmm_csr_f32_host(dlspm_ctx *ctx, int M, int K, int N, int nnz,
 int dlspm_fused_sddmm_spmm_f32_host(dlspm_ctx *ctx, int M, int K, int N, int nnz,
                                     const int *row_offsets, const int *column_indices,
                                     const float *C, const float *B, const float *D, float *E);
-/* Batched SpMM with host pointers inside every dlspm_problem: pieces of up to 128 MiB are copied in,
- * run as one grouped launch and copied out on three streams, so the two copy directions and the
- * kernels overlap.  Arrays are copied one by one unless they are neighbours in ONE pinned host
+/* Batched SpMM with host pointers inside every dlspm_problem: pieces of 8 to 128 MiB (about a sixteenth
+ * of the batch; the whole of it up to 32 MiB) are copied in, run as one grouped launch and copied out
+ * on three streams, so the two copy directions and the kernels overlap.  Arrays are copied one by one unless they are neighbours in ONE pinned host
  * allocation in the order and spacing of the staging layout (per problem row_offsets,
  * column_indices, values, B, each padded to a multiple of 256 bytes, problems one after the other;
  * the C buffers likewise in problem order): such a run goes as a single copy, one per piece and
