@@ -2,7 +2,9 @@
 
 This package is plumbing for the tests and the benchmark: it loads the C-ABI shared library that
 `include/dlspm.h` declares and passes device pointers of torch tensors (or host pointers of numpy
-arrays) straight through.  There is no Python or CPU implementation of any kernel here; if the
+arrays) straight through.  The single-matrix calls on CUDA tensors go through a small native module
+(`csrc/py_call.cpp`), because their host time would otherwise exceed the kernels' on small problems;
+everything else is ctypes.  There is no Python or CPU implementation of any kernel here; if the
 shared library is missing, `load_library()` raises.
 
 The directory name contains a hyphen, so it is imported through `importlib` under the module name
@@ -11,14 +13,18 @@ The directory name contains a hyphen, so it is imported through `importlib` unde
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 import subprocess
+import sys
 from typing import Optional, Sequence
 
 import numpy as np
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG_DIR, "libdlspm.so")
+CALL_PATH = os.path.join(PKG_DIR, "_dlspm_call.so")
 HEADER_PATH = os.path.join(os.path.dirname(PKG_DIR), "include", "dlspm.h")
 
 OK = 0
@@ -153,7 +159,7 @@ def exported_names() -> Sequence[str]:
 
 def build(verbose: bool = False) -> None:
     """Compiles libdlspm.so and the drivers in-tree with nvcc for sm_100a (no GPU needed)."""
-    cmd = ["make", "-C", PKG_DIR, "-j", str(os.cpu_count() or 4), "all"]
+    cmd = ["make", "-C", PKG_DIR, "-j", str(os.cpu_count() or 4), "PYTHON=" + sys.executable, "all"]
     proc = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if verbose or proc.returncode != 0:
         print(proc.stdout)
@@ -175,6 +181,25 @@ def load_library() -> C.CDLL:
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+_call = None
+
+
+def _load_call():
+    """Loads the native module of the tensor-taking calls; raises if it has not been built."""
+    global _call
+    if _call is None:
+        load_library()
+        if not os.path.exists(CALL_PATH):
+            raise RuntimeError(f"{CALL_PATH} is missing: build it with `make -C {PKG_DIR}` (no fallback exists)")
+        import torch  # noqa: F401  (the module links against torch's libraries)
+
+        loader = importlib.machinery.ExtensionFileLoader("_dlspm_call", CALL_PATH)
+        spec = importlib.util.spec_from_file_location("_dlspm_call", CALL_PATH, loader=loader)
+        _call = importlib.util.module_from_spec(spec)
+        loader.exec_module(_call)
+    return _call
 
 
 def strerror(status: int) -> str:
@@ -226,7 +251,8 @@ def _stream_ptr(stream) -> Optional[int]:
     if stream is None:
         import torch
 
-        return torch.cuda.current_stream().cuda_stream or None
+        torch.cuda.init()
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()) or None
     if isinstance(stream, int):
         return stream or None
     return stream.cuda_stream or None
@@ -242,11 +268,14 @@ class Context:
         self.handle = _P()
         self.device = device
         _check(self.lib.dlspm_create(C.byref(self.handle), device), "dlspm_create")
+        self._call = _load_call()
+        self._address = self.handle.value
 
     def close(self) -> None:
         if self.handle:
             self.lib.dlspm_destroy(self.handle)
             self.handle = _P()
+            self._address = None
 
     def __del__(self):
         try:
@@ -271,53 +300,34 @@ class Context:
 
     # device-pointer entry points (torch CUDA tensors)
     def spmm(self, M, K, N, nnz, values, row_offsets, column_indices, B, Cout, stream=None) -> None:
-        import torch
-
-        _check(self.lib.dlspm_spmm_csr_f32(
-            self.handle, M, K, N, nnz, _dev_ptr(values, torch.float32, "values"),
-            _dev_ptr(row_offsets, torch.int32, "row_offsets"), _dev_ptr(column_indices, torch.int32, "column_indices"),
-            _dev_ptr(B, torch.float32, "B"), _dev_ptr(Cout, torch.float32, "C"), _stream_ptr(stream)),
-            "dlspm_spmm_csr_f32", self)
+        status = self._call.spmm(self._address, M, K, N, nnz, values, row_offsets, column_indices, B, Cout, stream)
+        if status:
+            _check(status, "dlspm_spmm_csr_f32", self)
 
     def sddmm(self, M, K, N, nnz, row_offsets, column_indices, lhs, rhs, out, stream=None) -> None:
-        import torch
-
-        _check(self.lib.dlspm_sddmm_csr_f32(
-            self.handle, M, K, N, nnz, _dev_ptr(row_offsets, torch.int32, "row_offsets"),
-            _dev_ptr(column_indices, torch.int32, "column_indices"), _dev_ptr(lhs, torch.float32, "lhs"),
-            _dev_ptr(rhs, torch.float32, "rhs"), _dev_ptr(out, torch.float32, "out"), _stream_ptr(stream)),
-            "dlspm_sddmm_csr_f32", self)
+        status = self._call.sddmm(self._address, M, K, N, nnz, row_offsets, column_indices, None, lhs, rhs, out, stream)
+        if status:
+            _check(status, "dlspm_sddmm_csr_f32", self)
 
     def sddmm_masked(self, M, K, N, nnz, row_offsets, column_indices, mask_values, lhs, rhs, out, stream=None) -> None:
         """out[p] = mask_values[p] * dot(lhs[i], rhs[col_p]); mask_values None means 1."""
-        import torch
-
-        _check(self.lib.dlspm_sddmm_csr_masked_f32(
-            self.handle, M, K, N, nnz, _dev_ptr(row_offsets, torch.int32, "row_offsets"),
-            _dev_ptr(column_indices, torch.int32, "column_indices"),
-            _dev_ptr(mask_values, torch.float32, "mask_values") if mask_values is not None else None,
-            _dev_ptr(lhs, torch.float32, "lhs"), _dev_ptr(rhs, torch.float32, "rhs"),
-            _dev_ptr(out, torch.float32, "out"), _stream_ptr(stream)), "dlspm_sddmm_csr_masked_f32", self)
+        status = self._call.sddmm(self._address, M, K, N, nnz, row_offsets, column_indices, mask_values, lhs, rhs, out,
+                                  stream)
+        if status:
+            _check(status, "dlspm_sddmm_csr_masked_f32", self)
 
     def fused(self, M, K, N, nnz, row_offsets, column_indices, Cq, Bk, Dv, Eo, stream=None) -> None:
-        import torch
-
-        _check(self.lib.dlspm_fused_sddmm_spmm_f32(
-            self.handle, M, K, N, nnz, _dev_ptr(row_offsets, torch.int32, "row_offsets"),
-            _dev_ptr(column_indices, torch.int32, "column_indices"), _dev_ptr(Cq, torch.float32, "C"),
-            _dev_ptr(Bk, torch.float32, "B"), _dev_ptr(Dv, torch.float32, "D"), _dev_ptr(Eo, torch.float32, "E"),
-            _stream_ptr(stream)), "dlspm_fused_sddmm_spmm_f32", self)
+        status = self._call.fused(self._address, M, K, N, nnz, row_offsets, column_indices, Cq, Bk, Dv, Eo, stream)
+        if status:
+            _check(status, "dlspm_fused_sddmm_spmm_f32", self)
 
     def attention(self, M, K, N, nnz, row_offsets, column_indices, Q, Kmat, V, O, scale=1.0, flags=0,
                   stream=None) -> None:
         """O = softmax_rows(scale * pattern .* (Q Kmat^T)) V (flags=ATTN_SOFTMAX) or the scaled chain."""
-        import torch
-
-        _check(self.lib.dlspm_fused_attention_f32(
-            self.handle, M, K, N, nnz, _dev_ptr(row_offsets, torch.int32, "row_offsets"),
-            _dev_ptr(column_indices, torch.int32, "column_indices"), _dev_ptr(Q, torch.float32, "Q"),
-            _dev_ptr(Kmat, torch.float32, "Kmat"), _dev_ptr(V, torch.float32, "V"), _dev_ptr(O, torch.float32, "O"),
-            float(scale), int(flags), _stream_ptr(stream)), "dlspm_fused_attention_f32", self)
+        status = self._call.attention(self._address, M, K, N, nnz, row_offsets, column_indices, Q, Kmat, V, O, scale,
+                                      flags, stream)
+        if status:
+            _check(status, "dlspm_fused_attention_f32", self)
 
     def plan_create(self, M, K, nnz, row_offsets, column_indices, stream=None) -> "Plan":
         import torch
@@ -330,13 +340,10 @@ class Context:
         return Plan(self, h, M)
 
     def spmm_planned(self, plan, N, values, row_offsets, column_indices, B, Cout, stream=None) -> None:
-        import torch
-
-        _check(self.lib.dlspm_spmm_csr_f32_planned(
-            self.handle, plan.handle, N, _dev_ptr(values, torch.float32, "values"),
-            _dev_ptr(row_offsets, torch.int32, "row_offsets"), _dev_ptr(column_indices, torch.int32, "column_indices"),
-            _dev_ptr(B, torch.float32, "B"), _dev_ptr(Cout, torch.float32, "C"), _stream_ptr(stream)),
-            "dlspm_spmm_csr_f32_planned", self)
+        status = self._call.spmm_planned(self._address, plan.handle.value, N, values, row_offsets, column_indices, B, Cout,
+                                         stream)
+        if status:
+            _check(status, "dlspm_spmm_csr_f32_planned", self)
 
     def spmm_batched(self, problems: "ProblemArray", stream=None) -> None:
         _check(self.lib.dlspm_spmm_batched_f32(self.handle, len(problems), problems.array, _stream_ptr(stream)),
