@@ -40,6 +40,7 @@ struct dlspm_ctx {
     cudaStream_t side_stream[kSideStreams];
     cudaEvent_t side_fork, side_join[kSideStreams];
     int side_ready;
+    int *mma_error;  // host memory mapped on the device: set by a tensor-core kernel whose bounded wait ran out
     long long host_copies;  // cudaMemcpyAsync calls issued by the pipelined host-buffer batch so far
 };
 
@@ -86,6 +87,18 @@ size_t dlspm_batched_table_bytes(int count);
 // asynchronously; the caller must not reuse it before the launch has finished.
 int dlspm_spmm_batched_at(dlspm_ctx *ctx, int count, const dlspm_problem *problems, void *tables, cudaStream_t st,
                           void *pinned = nullptr);
+
+// SpMM of one matrix on the tensor cores (spmm_mma.cu), and whether it is the faster way.
+bool dlspm_spmm_mma_pays_alone(const dlspm_ctx *ctx, int M, int K, int N, int nnz, int vec);
+int dlspm_spmm_mma(dlspm_ctx *ctx, int M, int K, int N, int nnz, const float *values, const int *row_offsets, const int *cols,
+                   const float *B, float *C, cudaStream_t st);
+
+// Whether the tensor cores are the faster way for one of many problems of a batch.
+bool dlspm_spmm_mma_pays(int M, int K, int N, int nnz);
+// Tables of a launch over `count` problems: their size, and their host image (returns the number of tiles).
+size_t dlspm_spmm_mma_table_bytes(int count);
+long long dlspm_spmm_mma_tables(int count, const dlspm_problem *problems, void *image);
+int dlspm_spmm_mma_launch_tables(dlspm_ctx *ctx, const void *tables, int count, long long tiles, int *error, cudaStream_t st);
 
 // Grouped SDDMM / fused launches with caller-provided table memory (sddmm_batch.cu).
 size_t dlspm_rows_batched_table_bytes(int count);

@@ -68,6 +68,13 @@ extern "C" int dlspm_create(dlspm_ctx **out, int device)
         delete ctx;
         return DLSPM_ERR_CUDA;
     }
+    if (cudaHostAlloc((void **)&ctx->mma_error, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        (void)cudaGetLastError();
+        cudaStreamDestroy(ctx->stream);
+        delete ctx;
+        return DLSPM_ERR_NOMEM;
+    }
+    *ctx->mma_error = 0;
     *out = ctx;
     return DLSPM_OK;
 }
@@ -80,6 +87,7 @@ extern "C" int dlspm_destroy(dlspm_ctx *ctx)
     if (ctx->stage) cudaFree(ctx->stage);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
+    if (ctx->mma_error) cudaFreeHost(ctx->mma_error);
     if (ctx->side_ready) {
         for (int i = 0; i < kSideStreams; i++) {
             cudaStreamDestroy(ctx->side_stream[i]);

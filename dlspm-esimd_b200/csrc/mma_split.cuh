@@ -1,0 +1,239 @@
+// fp32 products on the 5th-generation tensor cores: every fp32 number is split into three bf16 numbers
+// whose sum is the number itself (3 x 8 significand bits with signs cover the 24 of fp32), and of the nine
+// products of parts the six largest are formed,
+//     x*y = x1*y1 + (x1*y2 + x2*y1) + (x1*y3 + x2*y2 + x3*y1) + 2^-26 |x*y| or less,
+// by tcgen05.mma with fp32 accumulators in tensor memory.  Each part is rounded to nearest, so x2 and x3 are
+// at most 2^-9 and 2^-18 of x and the three products left out are below the rounding of one fp32 multiply.
+// Limits, which the kernels test for: |x| >= 2^-100 or zero (below that the third part would lose bits to
+// the range of bf16), and finite numbers whose first part does not round to infinity.
+//
+// This file holds the split, the instruction wrappers and the shared-memory operand descriptors.
+#pragma once
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "barrier.cuh"
+
+namespace dlspm {
+
+// ---- split ------------------------------------------------------------------------------------------
+
+// Running minimum of the magnitude bits of nonzero numbers (doubled, minus one; zero counts as large).
+__device__ __forceinline__ unsigned split_magnitude(float x, unsigned least)
+{
+    return __viaddmin_u32(__float_as_uint(x) << 1, 0xffffffffu, least);
+}
+constexpr unsigned kSplitLeast = (27u << 24) - 1u;  // of 2^-100: smaller values of split_magnitude are too small to split
+
+// Smallest magnitude of three numbers (one instruction, NaN ignored): below 2^-100, zeros are told from small numbers
+// by split_magnitude.
+__device__ __forceinline__ float min3_magnitude(float a, float b, float c)
+{
+    float r;
+    asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+constexpr float kSplitSmall = 7.888609052210118e-31f;  // 2^-100
+
+__device__ __forceinline__ uint32_t bf16x2_bits(float lo, float hi)
+{
+    const __nv_bfloat162 t = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&t);
+}
+
+// (x, y) -> the packed first, second and third parts.  The remainders are formed two at a time (both subtractions
+// are exact).
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t &p1, uint32_t &p2, uint32_t &p3)
+{
+    float2 r = make_float2(x, y);
+    const float2 minus = make_float2(-1.f, -1.f);
+    p1 = bf16x2_bits(r.x, r.y);
+    r = __ffma2_rn(make_float2(__uint_as_float(p1 << 16), __uint_as_float(p1 & 0xffff0000u)), minus, r);
+    p2 = bf16x2_bits(r.x, r.y);
+    r = __ffma2_rn(make_float2(__uint_as_float(p2 << 16), __uint_as_float(p2 & 0xffff0000u)), minus, r);
+    p3 = bf16x2_bits(r.x, r.y);
+}
+// One number alone, parts in the low halves.
+__device__ __forceinline__ void split_one(float x, uint32_t &p1, uint32_t &p2, uint32_t &p3)
+{
+    p1 = bf16x2_bits(x, 0.f);
+    x -= __uint_as_float(p1 << 16);
+    p2 = bf16x2_bits(x, 0.f);
+    x -= __uint_as_float(p2 << 16);
+    p3 = bf16x2_bits(x, 0.f);
+}
+
+// Sixteen bytes that are not read again by this block: kept out of L1, which these kernels leave 28 KiB.
+__device__ __forceinline__ float4 load_once(const float *p)
+{
+    float4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
+// Stores by shared-memory address.
+__device__ __forceinline__ void store_shared(uint32_t at, uint32_t x, uint32_t y)
+{
+    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void store_shared_half(uint32_t at, uint32_t x)
+{
+    asm volatile("{\n .reg .b16 lo, hi;\n mov.b32 {lo, hi}, %1;\n st.shared.b16 [%0], lo;\n}\n" ::"r"(at), "r"(x) : "memory");
+}
+__device__ __forceinline__ void store_shared_zero(uint32_t at)
+{
+    asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(at), "r"(0u) : "memory");
+}
+
+// ---- clusters ---------------------------------------------------------------------------------------
+
+__device__ __forceinline__ unsigned cluster_rank()
+{
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// Without an ordering of memory accesses: where only the blocks' lifetimes matter.
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Address of the same shared-memory object in another block of the cluster.
+__device__ __forceinline__ uint32_t cluster_map(uint32_t smem, unsigned rank)
+{
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ float cluster_load(uint32_t addr)
+{
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ unsigned cluster_load_u32(uint32_t addr)
+{
+    unsigned v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+// Arrives on a barrier of another block (address from cluster_map); earlier writes of this thread are visible
+// to whoever sees the phase complete.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar)
+{
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Bounded wait (a second or so) that gives up when `abort` is raised.  The warp is suspended inside the instruction
+// until the phase completes or the hint, 20 us, has passed: polling instead cost the other warps of the SM a third
+// of their issue slots.
+__device__ __forceinline__ bool mbar_wait_suspended(unsigned long long *bar, unsigned parity, volatile int *abort)
+{
+    const uint32_t a = smem_u32(bar);
+    for (unsigned i = 0; i < (1u << 16); i++) {
+        unsigned ok;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(ok)
+            : "r"(a), "r"(parity), "r"(20000u)
+            : "memory");
+        if (ok) return true;
+        if (*abort) return false;
+    }
+    return false;
+}
+
+// Work of the previous kernel in the stream is complete and visible from here on (launches that may start
+// before it has ended); and the next kernel may start its own preamble.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// True on one lane of a converged warp.
+__device__ __forceinline__ bool elect_one()
+{
+    unsigned p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
+}
+
+// ---- tensor memory and the multiply ------------------------------------------------------------------
+// PAIR: two blocks of a cluster (ranks 2i and 2i + 1) work on one tile of 256 rows; the even one issues.
+
+template <bool PAIR>
+__device__ __forceinline__ void tmem_alloc(uint32_t *slot, unsigned columns)
+{
+    if constexpr (PAIR) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(columns) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    } else {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(columns) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+}
+template <bool PAIR>
+__device__ __forceinline__ void tmem_free(uint32_t base, unsigned columns)
+{
+    if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(columns));
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(columns));
+}
+__device__ __forceinline__ void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+// Sixteen columns of this warp's 32 tensor-memory lanes; tmem_load_wait before the values are used.
+__device__ __forceinline__ void tmem_load16(uint32_t addr, float (&v)[16])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
+          "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+        : "r"(addr));
+}
+// Ties the loaded values to the wait, so that no use of them moves in front of it.
+__device__ __forceinline__ void tmem_load_wait(float (&v)[16])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]),
+                   "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15])
+                 :
+                 : "memory");
+}
+
+// Shared-memory operand descriptors.  Swizzled layouts repeat every 8 rows; byte offsets between repetitions:
+// `lead` and `stride` as in the canonical layouts of the PTX manual.
+constexpr uint64_t kSwizzle128 = 2, kSwizzle64 = 4;
+__device__ __forceinline__ uint64_t mma_descriptor(uint32_t smem, unsigned lead, unsigned stride, uint64_t swizzle)
+{
+    return (uint64_t)((smem & 0x3ffffu) >> 4) | ((uint64_t)(lead >> 4) << 16) | ((uint64_t)(stride >> 4) << 32) | (1ull << 46) |
+           (swizzle << 61);
+}
+// bf16 operands, fp32 accumulators, M x N tile; `a_mn`, `b_mn`: the operand's rows run along K (its M or N
+// dimension is the contiguous one).
+__host__ __device__ constexpr uint32_t mma_instruction(int M, int N, bool a_mn, bool b_mn)
+{
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(N >> 3) << 17) |
+           ((uint32_t)(M >> 4) << 24);
+}
+template <bool PAIR>
+__device__ __forceinline__ void mma_bf16(uint32_t acc, uint64_t a, uint64_t b, uint32_t instruction, bool add)
+{
+    if constexpr (PAIR)
+        asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(acc),
+                     "l"(a), "l"(b), "r"(instruction), "r"(add ? 1u : 0u)
+                     : "memory");
+    else
+        asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(acc),
+                     "l"(a), "l"(b), "r"(instruction), "r"(add ? 1u : 0u)
+                     : "memory");
+}
+// The barrier (of both blocks of the pair) receives one arrival when all multiplies issued so far are done.
+template <bool PAIR>
+__device__ __forceinline__ void mma_commit(unsigned long long *bar, unsigned pair_mask)
+{
+    if constexpr (PAIR)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+                     "h"((unsigned short)pair_mask)
+                     : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+}  // namespace dlspm

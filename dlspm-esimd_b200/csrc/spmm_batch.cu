@@ -373,22 +373,33 @@ __global__ void __launch_bounds__(256) batch_analyze_kernel(const BatchProblem *
 
 }  // namespace
 
-struct dlspm_batch {
-    dlspm_ctx *ctx;
-    // row-gather part
+// The device tables of one way of dealing a batch's problems out to the kernels.
+struct BatchParts {
+    // row-gather kernel
     int count;
-    GatherSplit split;            // fine and coarse launches over `problems`
-    BatchProblem *problems;       // device
-    long long *tile_start;        // device, count + 2 (fine part, coarse part)
-    // tiled part (denser problems)
+    GatherSplit split;             // fine and coarse launches over `problems`
+    BatchProblem *problems;        // device
+    long long *tile_start;         // device, count + 2 (fine part, coarse part)
+    // FMA tile kernel
     int tcount;
     long long ttiles;
-    TileProblem *tproblems;       // device
-    long long *ttile_start;       // device, tcount + 1
-    unsigned long long *counters; // device: [0] row-gather, [1] tiled
-    int *row_order_pool;          // device: row orders of all row-gather problems
-    int *error;                   // device: set by a kernel whose bounded wait ran out
-    double stats[4];              // 2*nnz*N and algorithmic bytes: row-gather part, tiled part
+    TileProblem *tproblems;        // device
+    long long *ttile_start;        // device, tcount + 1
+    // tensor-core kernel
+    int mcount;
+    long long mtiles;
+    void *mtables;                 // device (spmm_mma.cu)
+    double stats[4];               // 2*nnz*N and algorithmic bytes: row-gather part, tiled parts
+};
+
+struct dlspm_batch {
+    dlspm_ctx *ctx;
+    BatchParts usual;              // launches without strict mode
+    BatchParts strict;             // launches in strict mode (nothing on the tensor cores); same_parts: unused
+    bool same_parts;               // no problem of the batch suits the tensor cores
+    unsigned long long *counters;  // device: work counters of the row-gather launches
+    int *row_order_pool;           // device: row orders of all row-gather problems
+    int *error;                    // device: set by a kernel whose bounded wait ran out
 };
 
 namespace {
@@ -451,6 +462,93 @@ bool prefer_tiled(const dlspm_ctx *ctx, const dlspm_problem &q, int vec, bool so
         return !ctx->tile_min_density_set || ctx->tile_min_density_permille > 1000 ||
                density * 1000.0 >= (double)ctx->tile_min_density_permille;
     return density * 1000.0 >= (double)ctx->tile_min_density_permille && q.M >= 16 && q.N >= 64;
+}
+
+// Whether the automatic choice takes the tensor-core kernel for a problem.  The caller's density threshold, where one
+// is set, decides for the tiled kernels as a whole.
+bool prefer_mma(const dlspm_ctx *ctx, const dlspm_problem &q, int vec, bool sorted)
+{
+    if (ctx->spmm_kernel != 0 || vec != 4 || !sorted || q.nnz == 0) return false;
+    if (ctx->tile_min_density_set)
+        return (double)q.nnz / ((double)q.M * (double)q.K) * 1000.0 >= (double)ctx->tile_min_density_permille && q.M >= 16 && q.N >= 64;
+    return dlspm_spmm_mma_pays(q.M, q.K, q.N, q.nnz);
+}
+
+cudaError_t upload(void **dst, const void *src, size_t bytes)
+{
+    cudaError_t err = cudaMalloc(dst, std::max<size_t>(bytes, 16));
+    if (err == cudaSuccess && bytes) err = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
+    return err;
+}
+
+// Builds the tables for a batch whose analysed problems are `tab` (most work first).
+int build_parts(dlspm_ctx *ctx, const std::vector<BatchProblem> &tab, const std::vector<int> &flags, bool tensor, BatchParts &parts)
+{
+    std::vector<BatchProblem> gtab;
+    std::vector<long long> gstarts;
+    std::vector<TileProblem> ttab;
+    std::vector<long long> tstarts;
+    std::vector<dlspm_problem> mtab;
+    memset(&parts, 0, sizeof(parts));
+    for (size_t i = 0; i < tab.size(); i++) {
+        const BatchProblem &t = tab[i];
+        const dlspm_problem q{t.M, t.K, t.N, t.nnz, t.values, t.row_offsets, t.cols, t.B, t.C};
+        const double fl = 2.0 * (double)t.nnz * t.N;
+        const double by = 4.0 * (t.M + 1) + 8.0 * t.nnz + 4.0 * (double)t.K * t.N + 4.0 * (double)t.M * t.N;
+        const bool sorted = (flags[i] & 1) != 0;
+        const bool mma = tensor && prefer_mma(ctx, q, t.vec, sorted);
+        const bool tiled = !mma && prefer_tiled(ctx, q, t.vec, sorted);
+        parts.stats[mma || tiled ? 2 : 0] += fl;
+        parts.stats[mma || tiled ? 3 : 1] += by;
+        if (mma) {
+            mtab.push_back(q);
+        } else if (tiled) {
+            TileProblem tp;
+            tp.values = t.values; tp.row_offsets = t.row_offsets; tp.cols = t.cols; tp.B = t.B; tp.C = t.C;
+            tp.row_order = t.row_order;
+            tp.M = t.M; tp.K = t.K; tp.N = t.N;
+            tp.row_blocks = dlspm_ceil_div(t.M, kTileM);
+            tp.col_blocks = dlspm_ceil_div(t.N, kTileN);
+            tp.pad = 0;
+            ttab.push_back(tp);
+        } else {
+            gtab.push_back(t);
+        }
+    }
+    finish_gather_tables(gtab, gstarts, parts.split);
+    // A tile of the FMA tile kernel costs ceil(K / 32) equal steps: with the problems in order of
+    // decreasing K the fixed deal of tiles to thread blocks (block b takes tiles b, b + blocks, ...)
+    // hands every block the same mix, the longest tiles first.
+    std::stable_sort(ttab.begin(), ttab.end(), [](const TileProblem &x, const TileProblem &y) { return x.K > y.K; });
+    for (const TileProblem &tp : ttab) {
+        tstarts.push_back(parts.ttiles);
+        parts.ttiles += (long long)tp.row_blocks * tp.col_blocks;
+    }
+    tstarts.push_back(parts.ttiles);
+    parts.count = (int)gtab.size();
+    parts.tcount = (int)ttab.size();
+    parts.mcount = (int)mtab.size();
+    cudaError_t err = upload((void **)&parts.problems, gtab.data(), sizeof(BatchProblem) * gtab.size());
+    if (err == cudaSuccess) err = upload((void **)&parts.tile_start, gstarts.data(), sizeof(long long) * gstarts.size());
+    if (err == cudaSuccess) err = upload((void **)&parts.tproblems, ttab.data(), sizeof(TileProblem) * ttab.size());
+    if (err == cudaSuccess) err = upload((void **)&parts.ttile_start, tstarts.data(), sizeof(long long) * tstarts.size());
+    if (err != cudaSuccess) return dlspm_cuda_fail(ctx, err, "batch tables");
+    if (!mtab.empty()) {
+        std::vector<unsigned char> image(dlspm_spmm_mma_table_bytes(parts.mcount));
+        parts.mtiles = dlspm_spmm_mma_tables(parts.mcount, mtab.data(), image.data());
+        err = upload(&parts.mtables, image.data(), image.size());
+        if (err != cudaSuccess) return dlspm_cuda_fail(ctx, err, "batch tables");
+    }
+    return DLSPM_OK;
+}
+
+void free_parts(BatchParts &p)
+{
+    if (p.problems) cudaFree(p.problems);
+    if (p.tile_start) cudaFree(p.tile_start);
+    if (p.tproblems) cudaFree(p.tproblems);
+    if (p.ttile_start) cudaFree(p.ttile_start);
+    if (p.mtables) cudaFree(p.mtables);
 }
 
 }  // namespace
@@ -518,62 +616,13 @@ extern "C" int dlspm_batch_create(dlspm_ctx *ctx, int count, const dlspm_problem
         dlspm_batch_destroy(b);
         return DLSPM_ERR_CUDA;
     }
-    // pass 2: split into the tiled and the row-gather tables
-    std::vector<BatchProblem> gtab;
-    std::vector<long long> gstarts;
-    std::vector<TileProblem> ttab;
-    std::vector<long long> tstarts;
-    long long trun = 0;
-    for (size_t i = 0; i < n; i++) {
-        const BatchProblem &t = tab[i];
-        dlspm_problem q;
-        q.M = t.M; q.K = t.K; q.N = t.N;
-        q.nnz = t.nnz;
-        const double fl = 2.0 * (double)t.nnz * t.N;
-        const double by = 4.0 * (t.M + 1) + 8.0 * t.nnz + 4.0 * (double)t.K * t.N + 4.0 * (double)t.M * t.N;
-        const bool tiled = prefer_tiled(ctx, q, t.vec, flags[i] & 1);
-        b->stats[tiled ? 2 : 0] += fl;
-        b->stats[tiled ? 3 : 1] += by;
-        if (tiled) {
-            TileProblem tp;
-            tp.values = t.values; tp.row_offsets = t.row_offsets; tp.cols = t.cols; tp.B = t.B; tp.C = t.C;
-            tp.row_order = t.row_order;
-            tp.M = t.M; tp.K = t.K; tp.N = t.N;
-            tp.row_blocks = dlspm_ceil_div(t.M, kTileM);
-            tp.col_blocks = dlspm_ceil_div(t.N, kTileN);
-            tp.pad = 0;
-            ttab.push_back(tp);
-        } else {
-            gtab.push_back(t);
-        }
-    }
-    finish_gather_tables(gtab, gstarts, b->split);
-    // A tile of the tiled kernel costs ceil(K / 32) equal steps: with the problems in order of
-    // decreasing K the fixed deal of tiles to thread blocks (block b takes tiles b, b + blocks, ...)
-    // hands every block the same mix, the longest tiles first.
-    std::stable_sort(ttab.begin(), ttab.end(), [](const TileProblem &x, const TileProblem &y) { return x.K > y.K; });
-    for (const TileProblem &tp : ttab) {
-        tstarts.push_back(trun);
-        trun += (long long)tp.row_blocks * tp.col_blocks;
-    }
-    tstarts.push_back(trun);
-    b->count = (int)gtab.size();
-    b->tcount = (int)ttab.size();
-    b->ttiles = trun;
-    err = cudaMalloc(&b->problems, sizeof(BatchProblem) * std::max<size_t>(gtab.size(), 1));
-    if (err == cudaSuccess) err = cudaMalloc(&b->tile_start, sizeof(long long) * gstarts.size());
-    if (err == cudaSuccess) err = cudaMalloc(&b->tproblems, sizeof(TileProblem) * std::max<size_t>(ttab.size(), 1));
-    if (err == cudaSuccess) err = cudaMalloc(&b->ttile_start, sizeof(long long) * tstarts.size());
-    if (err == cudaSuccess && !gtab.empty())
-        err = cudaMemcpy(b->problems, gtab.data(), sizeof(BatchProblem) * gtab.size(), cudaMemcpyHostToDevice);
-    if (err == cudaSuccess) err = cudaMemcpy(b->tile_start, gstarts.data(), sizeof(long long) * gstarts.size(), cudaMemcpyHostToDevice);
-    if (err == cudaSuccess && !ttab.empty())
-        err = cudaMemcpy(b->tproblems, ttab.data(), sizeof(TileProblem) * ttab.size(), cudaMemcpyHostToDevice);
-    if (err == cudaSuccess) err = cudaMemcpy(b->ttile_start, tstarts.data(), sizeof(long long) * tstarts.size(), cudaMemcpyHostToDevice);
-    if (err != cudaSuccess) {
-        dlspm_cuda_fail(ctx, err, "batch tables");
+    // pass 2: deal the problems out to the kernels
+    rc = build_parts(ctx, tab, flags, true, b->usual);
+    b->same_parts = b->usual.mcount == 0;
+    if (!rc && !b->same_parts) rc = build_parts(ctx, tab, flags, false, b->strict);
+    if (rc) {
         dlspm_batch_destroy(b);
-        return DLSPM_ERR_CUDA;
+        return rc;
     }
     *out = b;
     return DLSPM_OK;
@@ -585,12 +634,17 @@ extern "C" int dlspm_batch_launch_part(dlspm_ctx *ctx, const dlspm_batch *batch,
     int rc = dlspm_use(ctx);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
+    const BatchParts &p = ctx->strict_fp32 && !batch->same_parts ? batch->strict : batch->usual;
     if (part != 1) {
-        rc = tile_launch_tables(ctx, batch->tproblems, batch->ttile_start, batch->error, batch->tcount, batch->ttiles, st);
+        if (p.mcount) {
+            rc = dlspm_spmm_mma_launch_tables(ctx, p.mtables, p.mcount, p.mtiles, batch->error, st);
+            if (rc) return rc;
+        }
+        rc = tile_launch_tables(ctx, p.tproblems, p.ttile_start, batch->error, p.tcount, p.ttiles, st);
         if (rc) return rc;
     }
     if (part != 2) {
-        rc = batch_launch_tables(ctx, batch->problems, batch->tile_start, batch->counters, batch->split, st);
+        rc = batch_launch_tables(ctx, p.problems, p.tile_start, batch->counters, p.split, st);
     }
     return rc;
 }
@@ -607,9 +661,9 @@ extern "C" int dlspm_batch_info(dlspm_ctx *ctx, const dlspm_batch *batch, int *g
     if (!ctx || !batch || batch->ctx != ctx) return DLSPM_ERR_INVALID_ARGUMENT;
     int rc = dlspm_use(ctx);
     if (rc) return rc;
-    if (gather_problems) *gather_problems = batch->count;
-    if (tiled_problems) *tiled_problems = batch->tcount;
-    if (stats4) memcpy(stats4, batch->stats, sizeof(batch->stats));
+    if (gather_problems) *gather_problems = batch->usual.count;
+    if (tiled_problems) *tiled_problems = batch->usual.tcount + batch->usual.mcount;
+    if (stats4) memcpy(stats4, batch->usual.stats, sizeof(batch->usual.stats));
     if (device_error) {
         DLSPM_CUDA_TRY(ctx, cudaDeviceSynchronize());
         DLSPM_CUDA_TRY(ctx, cudaMemcpy(device_error, batch->error, sizeof(int), cudaMemcpyDeviceToHost));
@@ -621,10 +675,8 @@ extern "C" int dlspm_batch_destroy(dlspm_batch *b)
 {
     if (!b) return DLSPM_OK;
     cudaSetDevice(b->ctx->device);
-    if (b->problems) cudaFree(b->problems);
-    if (b->tile_start) cudaFree(b->tile_start);
-    if (b->tproblems) cudaFree(b->tproblems);
-    if (b->ttile_start) cudaFree(b->ttile_start);
+    free_parts(b->usual);
+    free_parts(b->strict);
     if (b->counters) cudaFree(b->counters);
     if (b->row_order_pool) cudaFree(b->row_order_pool);
     if (b->error) cudaFree(b->error);

@@ -1,0 +1,726 @@
+// SpMM on the tensor cores, for patterns from a few percent nonzeros upwards: the sparse matrix is written
+// out densely, 64 columns at a time, in shared memory and multiplied with B by tcgen05.mma with both operands
+// split into three bf16 parts (mma_split.cuh), six products per fp32 product.
+//
+// Why: the row-gather kernel pays one L1 wavefront per FMA instruction and ends at 13 to 17 TFLOP/s of stored
+// entries, the FMA tile kernel at 45 TFLOP/s of dense arithmetic.  Six bf16 products per fp32 product leave
+// 1648 / 6 = 275 TFLOP/s of dense fp32-accurate arithmetic.
+//
+// A tile is 256 columns of C times up to 128 rows, computed by a PAIR of thread blocks (cta_group::2): the
+// columns of C are the tile's M dimension (tensor-memory lanes), the rows of the sparse matrix its N dimension.
+// With this orientation a warp's 32 lanes hold 32 neighbouring columns of C and plain 4-byte stores are
+// coalesced; and the row count of a tile can be any multiple of 16.  Each block of the pair converts its own
+// 128 columns of B and its own half of the rows, and the pair reads both halves of the rows.  (Tiles of 256 rows
+// need half the conversions of B per multiply, but the sums then take half of the registers of an SM, and the
+// eight operand warps that were left could not hide their latencies: 6000 cycles per 32 columns.)
+//
+// Sums: the product of the two first parts goes to one accumulator, the five small products to another.  The
+// tensor core does not round its sums to nearest, so an accumulator drifts with the number of additions: the
+// main one is added to fp32 registers every 64 columns of the sparse matrix, the small one once per tile (its
+// drift is relative to sums 2^-8 as large).
+//
+// Roles of the 28 warps of a block:
+//   8 sum warps       add finished accumulators to their registers and write C.
+//   16 operand warps  convert 64 rows of B and scatter the matching 64 columns of the sparse rows, eight lanes a
+//                     row, into one of three stages; both come from registers loaded one chunk ahead.
+//   1 issuing warp    (of the even block) issues 24 multiplies a chunk; in the odd block it relays barriers.
+// (registers are handed out in groups of four warps; the rest of the last group is idle)
+//
+// Rows whose columns are not strictly ascending, tiles with magnitudes that cannot be split, and sums that are
+// not finite are computed again from the CSR arrays with fp32 multiply-adds, so that such input gives what the
+// row-gather kernel gives.
+#pragma once
+#include "mma_split.cuh"
+#include "spmm_device.cuh"
+
+namespace dlspm {
+
+constexpr int kMmaChunk = 64;   // columns of the sparse matrix per stage, and per main accumulator
+constexpr int kMmaStages = 3;
+constexpr int kMmaCols = 128;   // columns of C per block, 256 per pair
+constexpr int kMmaRows = 64;    // rows of the sparse matrix per block at most, 128 per pair
+constexpr int kMmaMarkWords = 2 * kMmaRows / 32;
+constexpr int kMmaSumWarps = 8, kMmaOperandWarps = 16;
+constexpr int kMmaThreads = (kMmaSumWarps + kMmaOperandWarps + 4) * 32;
+constexpr int kMmaDensePlane = kMmaChunk * kMmaCols * 2;   // bytes of one part of one operand in a stage
+constexpr int kMmaSparsePlane = kMmaChunk * kMmaRows * 2;
+constexpr uint32_t kMmaSmallColumn = 256;  // tensor memory: two main accumulators, then two for the small products
+constexpr int kMmaRing = 16;    // tiles whose marks (rows to compute again) can be alive at once
+constexpr int kMmaRegsLaunch = 72, kMmaRegsSum = 88, kMmaRegsOperand = 72, kMmaRegsIssue = 40;
+static_assert(kMmaThreads * kMmaRegsLaunch <= 65536 &&
+                  kMmaSumWarps * 32 * kMmaRegsSum + kMmaOperandWarps * 32 * kMmaRegsOperand + 128 * kMmaRegsIssue <=
+                      kMmaThreads * kMmaRegsLaunch,
+              "register budgets exceed what the block is launched with");
+
+struct MmaProblem {
+    const float *values;
+    const int *row_offsets;
+    const int *cols;
+    const float *B;
+    float *C;
+    int M, K, N;
+    int block_rows;  // rows per tile, a multiple of 16 (half of them per block)
+    int row_blocks;  // ceil(M / block_rows)
+    int depth;       // entries of a row fetched ahead, in eights: 1 to 4
+};
+
+struct MmaSmem {
+    unsigned char dense[kMmaStages][3][kMmaDensePlane];    // B: rows of 64 of its columns, 128-byte swizzle
+    unsigned char sparse[kMmaStages][3][kMmaSparsePlane];  // A: rows of 64 columns, 128-byte swizzle
+    unsigned long long full[kMmaStages], empty[kMmaStages];  // operands written (both blocks) / multiplies done
+    unsigned long long sum_full[2], sum_empty[2];            // accumulators complete / added by all sum warps
+    unsigned long long drain;                                // multiplies still running when a wait ran out
+    unsigned again[kMmaRing][kMmaMarkWords];                  // rows of the tile to compute again
+    uint32_t tmem;
+    int abort;
+};
+constexpr size_t kMmaSmemBytes = sizeof(MmaSmem) + 1024;  // the swizzled planes start at a 1024-byte boundary
+static_assert(kMmaSmemBytes <= 232448, "shared memory of a block");
+
+// The tiles of one launch: of a table of problems (tile_start[i] = first tile of problem i), or of one problem.
+struct MmaArgs {
+    const MmaProblem *problems;
+    const long long *tile_start;
+    int count;
+    int splits;  // parts of K, each a pair of its own; more than one only with one tile per cluster
+    long long tiles;
+    MmaProblem one;  // used when problems is null
+    int *error;
+};
+
+struct MmaTile {
+    long long tile;
+    int prob;
+    const MmaProblem *p;
+    int row0, n0;       // first row and column of this block's part
+    int rows;           // rows per block of the pair
+    int chunk0, chunks; // its part of K
+};
+
+// A position in the ring of stages and the parity of its barriers' current phase.
+struct MmaStage {
+    int stage;
+    unsigned parity;
+    __device__ __forceinline__ void next()
+    {
+        if (++stage == kMmaStages) {
+            stage = 0;
+            parity ^= 1u;
+        }
+    }
+};
+
+template <bool TABLE>
+__device__ __forceinline__ bool mma_tile_load(MmaTile &t, const MmaArgs &a, unsigned rank)
+{
+    if (t.tile >= a.tiles) return false;
+    long long first = 0;
+    if constexpr (TABLE) {
+        int lo = t.prob, hi = a.count - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (__ldg(a.tile_start + mid) <= t.tile) lo = mid;
+            else hi = mid - 1;
+        }
+        t.prob = lo;
+        t.p = a.problems + lo;
+        first = __ldg(a.tile_start + lo);
+    } else {
+        t.p = &a.one;
+    }
+    const int i = (int)(t.tile - first);
+    const int cb = i / t.p->row_blocks, rb = i - cb * t.p->row_blocks;
+    t.rows = t.p->block_rows >> 1;
+    t.row0 = rb * t.p->block_rows;
+    t.n0 = cb * 2 * kMmaCols + (int)(rank & 1u) * kMmaCols;
+    const int all = (t.p->K + kMmaChunk - 1) / kMmaChunk;
+    const int part = (int)(rank >> 1);
+    t.chunk0 = (int)((long long)all * part / a.splits);
+    t.chunks = (int)((long long)all * (part + 1) / a.splits) - t.chunk0;
+    return true;
+}
+
+// First entry of the row at or behind column `col`.
+__device__ __forceinline__ int mma_lower_bound(const int *__restrict__ cols, int lo, int hi, int col)
+{
+    while (lo < hi) {
+        const int mid = lo + ((hi - lo) >> 1);
+        if (__ldg(cols + mid) < col) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// ---- operand warps ------------------------------------------------------------------------------------
+
+// What a lane needs to read B: byte offsets of its four columns in the chunk row that comes next, 16 rows further
+// and in the last row of B.  (Offsets instead of pointers: the base addresses stay in uniform registers.)
+struct MmaDense {
+    unsigned next, step, last;
+    unsigned d1, d2, d3;  // of the second to fourth column against the first (not WIDE)
+};
+
+// Half a chunk of B, rows k and k + 16 of 32 (k = warp), lane l columns 4l .. 4l + 3 of this block's 128.  Rows and
+// columns past the end of B repeat its last ones: no entry refers to such a row, and such a column is not stored.
+template <bool WIDE>
+__device__ __forceinline__ void mma_load_dense(float4 (&d)[2], MmaDense &b, const float *__restrict__ B)
+{
+    const char *base = reinterpret_cast<const char *>(B);
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const unsigned at = min(b.next, b.last);
+        b.next += b.step;
+        if constexpr (WIDE) {
+            d[i] = load_once(reinterpret_cast<const float *>(base + at));
+        } else {
+            d[i].x = __ldg(reinterpret_cast<const float *>(base + at));
+            d[i].y = __ldg(reinterpret_cast<const float *>(base + (at + b.d1)));
+            d[i].z = __ldg(reinterpret_cast<const float *>(base + (at + b.d2)));
+            d[i].w = __ldg(reinterpret_cast<const float *>(base + (at + b.d3)));
+        }
+    }
+}
+
+// Writes a half split to shared memory at `dst`: 64 columns are one 128-byte row of an 8-row block, the 16-byte
+// units of row r permuted by XOR with r.  Eight-row blocks along K are 1024 bytes apart, the two halves of 64
+// columns 8192.
+__device__ __forceinline__ void mma_store_dense(uint32_t dst, const float4 (&d)[2], unsigned &least)
+{
+    float small = 1.f;
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        small = min3_magnitude(small, d[i].x, d[i].y);
+        small = min3_magnitude(small, d[i].z, d[i].w);
+        uint32_t x1, x2, x3, y1, y2, y3;
+        split_pair(d[i].x, d[i].y, x1, x2, x3);
+        split_pair(d[i].z, d[i].w, y1, y2, y3);
+        store_shared(dst + i * 2048, x1, y1);
+        store_shared(dst + i * 2048 + kMmaDensePlane, x2, y2);
+        store_shared(dst + i * 2048 + 2 * kMmaDensePlane, x3, y3);
+    }
+    if (small < kSplitSmall) {  // a zero, or a number that cannot be split
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            least = split_magnitude(d[i].x, least);
+            least = split_magnitude(d[i].y, least);
+            least = split_magnitude(d[i].z, least);
+            least = split_magnitude(d[i].w, least);
+        }
+    }
+}
+
+// Entries q, q + 8, .. of a row; slots past its end hold a column that no chunk contains.
+template <int DEPTH>
+__device__ __forceinline__ void mma_load_pairs(int (&c)[DEPTH], float (&v)[DEPTH], int q, int end, const MmaProblem &p)
+{
+    const char *cols = reinterpret_cast<const char *>(p.cols), *values = reinterpret_cast<const char *>(p.values);
+    const unsigned at = 4u * (unsigned)q;
+#pragma unroll
+    for (int h = 0; h < DEPTH; h++) {
+        c[h] = 0x7fffffff;
+        if (q + 8 * h < end) {
+            c[h] = __ldg(reinterpret_cast<const int *>(cols + (at + 32u * h)));
+            v[h] = __ldg(reinterpret_cast<const float *>(values + (at + 32u * h)));
+        }
+    }
+}
+
+// One entry of the sparse matrix into a stage; `row` is the address of its row of the first part.
+__device__ __forceinline__ void mma_store_entry(uint32_t row, int col, float v, int swizzle, bool live)
+{
+    uint32_t p1, p2, p3;
+    split_one(v, p1, p2, p3);
+    const uint32_t e = row + ((col * 2) ^ swizzle);
+    if (live) {
+        store_shared_half(e, p1);
+        store_shared_half(e + kMmaSparsePlane, p2);
+        store_shared_half(e + 2 * kMmaSparsePlane, p3);
+    }
+}
+
+__device__ __forceinline__ void mma_mark_again(MmaSmem &sm, int ring, int bit, unsigned rank)
+{
+    // the marks of a tile are kept in both blocks of the pair
+    atomicOr(&sm.again[ring][bit >> 5], 1u << (bit & 31));
+    const uint32_t other = cluster_map(smem_u32(&sm.again[ring][bit >> 5]), rank ^ 1u);
+    asm volatile("red.relaxed.cluster.shared::cluster.or.b32 [%0], %1;" ::"r"(other), "r"(1u << (bit & 31)) : "memory");
+}
+
+// One tile: every lane group of eight lanes owns one row of it, 4 * warp + group, and walks it once.  DEPTH: entries
+// of a row fetched ahead, in eights.  CHECK: columns may be out of order (with a table they were looked at when it
+// was made).
+template <int DEPTH, bool CHECK, bool WIDE>
+__device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, const MmaTile &t, unsigned rank, int warp, int lane,
+                                                 int ring, MmaStage &st)
+{
+    volatile int *abort = &sm.abort;
+    const MmaProblem &p = *t.p;
+    const int l8 = lane & 7, group = lane & 24, own = warp * 4 + (lane >> 3);
+    const int swizzle = (own & 7) << 4;
+    const bool row_warp = warp * 4 < t.rows;  // this warp has rows in the tile
+    int cursor = 0, end = 0;
+    {
+        const int row = t.row0 + (int)(rank & 1u) * t.rows + own;
+        if (own < t.rows && row < p.M) {
+            const int start = __ldg(p.row_offsets + row), stop = __ldg(p.row_offsets + row + 1);
+            cursor = start;
+            end = stop;
+            if (a.splits > 1) {
+                const int part = (int)(rank >> 1);
+                if (part > 0) cursor = mma_lower_bound(p.cols, start, stop, t.chunk0 * kMmaChunk);
+                if (part + 1 < a.splits) end = mma_lower_bound(p.cols, start, stop, (t.chunk0 + t.chunks) * kMmaChunk);
+            }
+        }
+    }
+    int k0 = t.chunk0 * kMmaChunk;
+    MmaDense b;
+    {
+        const int n = min(t.n0 + 4 * lane, WIDE ? p.N - 4 : p.N - 1);
+        b.next = 4u * ((unsigned)(k0 + warp) * (unsigned)p.N + (unsigned)n);
+        b.step = 64u * (unsigned)p.N;
+        b.last = 4u * ((unsigned)(p.K - 1) * (unsigned)p.N + (unsigned)n);
+        if constexpr (!WIDE) {
+            b.d1 = 4u * (unsigned)min(1, p.N - 1 - n);
+            b.d2 = 4u * (unsigned)min(2, p.N - 1 - n);
+            b.d3 = 4u * (unsigned)min(3, p.N - 1 - n);
+        }
+    }
+    const uint32_t dense_at = smem_u32(&sm.dense[0][0][0]) + (lane >> 4) * 8192 + (warp >> 3) * 1024 + (warp & 7) * 128 +
+                              ((((lane & 15) >> 1) ^ (warp & 7)) << 4) + (lane & 1) * 8;
+    const uint32_t sparse_at = smem_u32(&sm.sparse[0][0][0]) + own * 128;
+    float4 dense[2];
+    unsigned least = 0xffffffffu;
+    bool bad = false, ok = true;  // bad: the lane group's row has columns out of order
+    // One chunk: its entries are in (c, v), the next chunk's are fetched into (cn, vn).
+    auto step = [&](int (&c)[DEPTH], float (&v)[DEPTH], int (&cn)[DEPTH], float (&vn)[DEPTH]) {
+        ok = mbar_wait_suspended(&sm.empty[st.stage], st.parity ^ 1u, abort);  // passes at once in the first round
+        if (!ok) return;
+        const uint32_t row = sparse_at + st.stage * (3 * kMmaSparsePlane);
+        const uint32_t dst = dense_at + st.stage * (3 * kMmaDensePlane);
+        if (row_warp) {
+            // this warp's four rows: zeros in all three parts
+            const uint32_t z = row + l8 * 16;
+            store_shared_zero(z);
+            store_shared_zero(z + kMmaSparsePlane);
+            store_shared_zero(z + 2 * kMmaSparsePlane);
+            __syncwarp();
+            // how many of the entries at hand belong to this chunk (they are the first of them: columns ascend)
+            int used = 0;
+#pragma unroll
+            for (int h = 0; h < DEPTH; h++)
+                used += __popc((__ballot_sync(0xffffffffu, (unsigned)(c[h] - k0) < (unsigned)kMmaChunk) >> group) & 0xffu);
+            cursor += used;
+            bool more = used == 8 * DEPTH;
+            while (__any_sync(0xffffffffu, more)) {  // more entries than were fetched ahead: eight at a time
+                const int q = cursor + l8;
+                bool take = false;
+                if (more && q < end) {
+                    const int col = __ldg(p.cols + q), before = CHECK ? __ldg(p.cols + q - 1) : -1;
+                    const float x = __ldg(p.values + q);
+                    take = (unsigned)(col - k0) < (unsigned)kMmaChunk;
+                    if (take) {
+                        if (CHECK && col <= before) bad = true;
+                        least = split_magnitude(x, least);
+                        mma_store_entry(row, col - k0, x, swizzle, true);
+                    }
+                }
+                const int got = __popc((__ballot_sync(0xffffffffu, take) >> group) & 0xffu);
+                cursor += got;
+                more = got == 8;
+            }
+            if constexpr (DEPTH <= 2) mma_load_pairs(cn, vn, cursor + l8, end, p);
+        }
+        mma_store_dense(dst, dense, least);
+        mma_load_dense<WIDE>(dense, b, p.B);
+        if (row_warp) {
+            int last = -1;  // column in front of the first entry at hand (entries of earlier chunks are in order)
+#pragma unroll
+            for (int h = 0; h < DEPTH; h++) {
+                const int col = c[h] - k0;
+                const bool live = (unsigned)col < (unsigned)kMmaChunk;
+                if constexpr (CHECK) {
+                    int before = __shfl_up_sync(0xffffffffu, col, 1, 8);
+                    if (l8 == 0) before = last;
+                    if (h + 1 < DEPTH) last = __shfl_sync(0xffffffffu, col, 7, 8);
+                    bad = bad || (live && col <= before);
+                }
+                if (live) least = split_magnitude(v[h], least);
+                mma_store_entry(row, col, v[h], swizzle, live);
+            }
+            if constexpr (DEPTH > 2) mma_load_pairs(c, v, cursor + l8, end, p);
+        }
+        mma_store_dense(dst + 4096, dense, least);
+        mma_load_dense<WIDE>(dense, b, p.B);
+        k0 += kMmaChunk;
+    };
+    // Hands a stage over; `marks`: the tile's last one.
+    auto hand_over = [&](bool marks) {
+        if (marks) {
+            if (CHECK && cursor != end) bad = true;  // entries out of order were never reached
+            const bool all = __any_sync(0xffffffffu, least < kSplitLeast);
+            if (__any_sync(0xffffffffu, bad) || all) {
+                if (bad && own < t.rows) mma_mark_again(sm, ring, (int)(rank & 1u) * t.rows + own, rank);
+                if (all)
+                    for (int r = lane; r < 2 * t.rows; r += 32) mma_mark_again(sm, ring, r, rank);
+            }
+        }
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.full[st.stage]);
+        st.next();
+    };
+    int c0[DEPTH];
+    float v0[DEPTH];
+    mma_load_pairs(c0, v0, cursor + l8, end, p);
+    mma_load_dense<WIDE>(dense, b, p.B);
+    if constexpr (DEPTH <= 2) {
+        // two chunks a turn with the register sets exchanged: copying one to the other would wait for its loads
+        int c1[DEPTH];
+        float v1[DEPTH];
+        for (int i = 0; i < t.chunks; i += 2) {
+            step(c0, v0, c1, v1);
+            if (!ok) return false;
+            hand_over(i + 1 == t.chunks);
+            if (i + 1 < t.chunks) {
+                step(c1, v1, c0, v0);
+                if (!ok) return false;
+                hand_over(i + 2 == t.chunks);
+            }
+        }
+    } else {
+        // (no registers for a second set; the entries of a dense chunk are fetched behind the last one's)
+        for (int i = 0; i < t.chunks; i++) {
+            step(c0, v0, c0, v0);
+            if (!ok) return false;
+            hand_over(i + 1 == t.chunks);
+        }
+    }
+    return true;
+}
+
+template <bool TABLE, bool WIDE>
+__device__ __forceinline__ bool mma_operands(MmaSmem &sm, const MmaArgs &a, unsigned rank, int warp, int lane)
+{
+    MmaTile t;
+    t.tile = blockIdx.x / (2u * (unsigned)a.splits);
+    t.prob = 0;
+    const unsigned stride = gridDim.x / (2u * (unsigned)a.splits);
+    MmaStage st{0, 0u};
+    int ring = 0;
+    while (mma_tile_load<TABLE>(t, a, rank)) {
+        bool ok;
+        if (t.p->depth == 1) ok = mma_operand_tile<1, !TABLE, WIDE>(sm, a, t, rank, warp, lane, ring, st);
+        else if (t.p->depth == 2) ok = mma_operand_tile<2, !TABLE, WIDE>(sm, a, t, rank, warp, lane, ring, st);
+        else ok = mma_operand_tile<5, !TABLE, WIDE>(sm, a, t, rank, warp, lane, ring, st);
+        if (!ok) return false;
+        ring = (ring + 1) % kMmaRing;
+        t.tile += stride;
+    }
+    return true;
+}
+
+// ---- issuing warp (of the even block) ----------------------------------------------------------
+
+// The whole warp walks the chunks, one lane issues (the instructions take their operands from uniform registers,
+// which the compiler can only use where control flow is uniform).
+template <bool TABLE>
+__device__ __forceinline__ bool mma_issue(MmaSmem &sm, const MmaArgs &a, unsigned rank, bool issuer)
+{
+    volatile int *abort = &sm.abort;
+    MmaTile t;
+    t.tile = blockIdx.x / (2u * (unsigned)a.splits);
+    t.prob = 0;
+    const unsigned stride = gridDim.x / (2u * (unsigned)a.splits);
+    const unsigned pair_mask = 3u << rank;
+    const uint32_t tmem = sm.tmem;
+    // parts (of B, of A) of the five small products
+    const int part_b[5] = {2, 1, 1, 0, 0}, part_a[5] = {0, 1, 0, 2, 1};
+    const uint64_t dense0 = mma_descriptor(smem_u32(&sm.dense[0][0][0]), 8192, 1024, kSwizzle128);
+    const uint64_t sparse0 = mma_descriptor(smem_u32(&sm.sparse[0][0][0]), 0, 1024, kSwizzle128);
+    constexpr uint64_t kDense = kMmaDensePlane >> 4, kSparse = kMmaSparsePlane >> 4;
+    unsigned g = 0, done = 0;  // chunks (one main accumulator each) and tiles so far
+    while (mma_tile_load<TABLE>(t, a, rank)) {
+        const uint32_t instruction = mma_instruction(256, 2 * t.rows, true, false);
+        const uint32_t small = tmem + kMmaSmallColumn + (done & 1u) * 128u;
+        for (int c = 0; c < t.chunks; c++, g++) {
+            const int s = (int)(g % kMmaStages);
+            // (the accumulator of the small products was read together with the tile's last main one)
+            if (g >= 2u && !mbar_wait_suspended(&sm.sum_empty[g & 1u], ((g >> 1) - 1u) & 1u, abort)) return false;
+            if (!mbar_wait_suspended(&sm.full[s], (g / kMmaStages) & 1u, abort)) return false;
+            tmem_fence_after();
+            const uint32_t main = tmem + (g & 1u) * 128u;
+            const uint64_t dense = dense0 + s * (3 * kDense), sparse = sparse0 + s * (3 * kSparse);
+            if (issuer) {
+#pragma unroll
+                for (int ks = 0; ks < kMmaChunk / 16; ks++) {
+                    const uint64_t d = dense + ks * (2048 >> 4), x = sparse + ks * (32 >> 4);
+#pragma unroll
+                    for (int j = 0; j < 5; j++)
+                        mma_bf16<true>(small, d + part_b[j] * kDense, x + part_a[j] * kSparse, instruction, c + j + ks > 0);
+                    mma_bf16<true>(main, d, x, instruction, ks > 0);
+                }
+                mma_commit<true>(&sm.empty[s], pair_mask);
+                mma_commit<true>(&sm.sum_full[g & 1u], pair_mask);
+            }
+            __syncwarp();
+        }
+        done++;
+        t.tile += stride;
+    }
+    return true;
+}
+
+// ---- relay (odd block) ------------------------------------------------------------------------------------
+
+// Passes the odd block's barriers on to the even block's, one arrival per phase: a remote arrival orders all
+// memory accesses of its thread first, which would hold up a warp with loads in flight.
+template <bool TABLE>
+__device__ __forceinline__ bool mma_relay(MmaSmem &sm, const MmaArgs &a, unsigned rank, bool sums)
+{
+    volatile int *abort = &sm.abort;
+    MmaTile t;
+    t.tile = blockIdx.x / (2u * (unsigned)a.splits);
+    t.prob = 0;
+    const unsigned stride = gridDim.x / (2u * (unsigned)a.splits);
+    const unsigned slots = sums ? 2u : (unsigned)kMmaStages;
+    unsigned long long *own = sums ? sm.sum_empty : sm.full;
+    const uint32_t other = cluster_map(smem_u32(own), rank ^ 1u);
+    unsigned g = 0;
+    while (mma_tile_load<TABLE>(t, a, rank)) {
+        for (int c = 0; c < t.chunks; c++, g++) {
+            if (!mbar_wait_suspended(&own[g % slots], (g / slots) & 1u, abort)) return false;
+            mbar_arrive_cluster(other + (g % slots) * 8u);
+        }
+        t.tile += stride;
+    }
+    return true;
+}
+
+// ---- sum warps --------------------------------------------------------------------------------------------
+
+__device__ __forceinline__ void sum_warps_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kMmaSumWarps * 32) : "memory"); }
+
+// Row `row` of C, this block's 128 columns from n0, by one warp from the CSR arrays.
+__device__ __forceinline__ void mma_row_again(const MmaProblem &p, int row, int n0, int lane)
+{
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int q = __ldg(p.row_offsets + row), end = __ldg(p.row_offsets + row + 1); q < end; q++) {
+        const float v = __ldg(p.values + q);
+        const float *b = p.B + (size_t)__ldg(p.cols + q) * (size_t)p.N + n0 + lane;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (n0 + lane + 32 * i < p.N) acc[i] = fmaf(v, __ldg(b + 32 * i), acc[i]);
+    }
+    float *c = p.C + (size_t)row * (size_t)p.N + n0 + lane;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        if (n0 + lane + 32 * i < p.N) c[32 * i] = acc[i];
+}
+
+// Marks the columns of the accumulators (rows of the sparse matrix) in which some lane holds a sum that is not
+// finite.  `first` is the row of acc[0].
+template <int COUNT>
+__device__ __forceinline__ void mma_mark_not_finite(MmaSmem &sm, int ring, const float (&acc)[COUNT], int first, int lane)
+{
+    float probe[2] = {0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < COUNT; j++) probe[j & 1] = fmaf(acc[j], 0.f, probe[j & 1]);
+    if (!__any_sync(0xffffffffu, probe[0] + probe[1] != 0.f)) return;  // NaN compares unequal
+#pragma unroll
+    for (int j = 0; j < COUNT; j++)
+        if (__any_sync(0xffffffffu, fmaf(acc[j], 0.f, 0.f) != 0.f) && lane == 0)
+            atomicOr(&sm.again[ring][(first + j) >> 5], 1u << ((first + j) & 31));
+}
+
+// Adds 64 columns of an accumulator to the warp's registers (those of them that the tile has).
+__device__ __forceinline__ void mma_add(float (&acc)[kMmaRows], uint32_t addr, int columns)
+{
+#pragma unroll
+    for (int j = 0; j < kMmaRows; j += 16) {
+        if (j < columns) {
+            float v[16];
+            tmem_load16(addr + j, v);
+            tmem_load_wait(v);
+#pragma unroll
+            for (int x = 0; x < 16; x += 2) {
+                const float2 sum = __fadd2_rn(make_float2(acc[j + x], acc[j + x + 1]), make_float2(v[x], v[x + 1]));
+                acc[j + x] = sum.x;
+                acc[j + x + 1] = sum.y;
+            }
+        }
+    }
+}
+
+// Warp w: tensor-memory lanes 32 * (w % 4) .. + 31 (columns of C), accumulator columns 64 * (w / 4) .. + 63
+// (rows of the sparse matrix).
+template <bool TABLE>
+__device__ __forceinline__ bool mma_sums(MmaSmem &sm, const MmaArgs &a, unsigned rank, int warp, int lane)
+{
+    volatile int *abort = &sm.abort;
+    MmaTile t;
+    t.tile = blockIdx.x / (2u * (unsigned)a.splits);
+    t.prob = 0;
+    const unsigned stride = gridDim.x / (2u * (unsigned)a.splits);
+    const int half = (warp >> 2) * kMmaRows, quarter = warp & 3;
+    const uint32_t tmem = sm.tmem + ((uint32_t)quarter << 21) + (uint32_t)half;
+    unsigned q = 0, done = 0;
+    int ring = 0;
+    while (mma_tile_load<TABLE>(t, a, rank)) {
+        const int tile_rows = 2 * t.rows;
+        float acc[kMmaRows];
+#pragma unroll
+        for (int j = 0; j < kMmaRows; j++) acc[j] = 0.f;
+        for (int i = 0; i < t.chunks; i++, q++) {
+            if (!mbar_wait_suspended(&sm.sum_full[q & 1u], (q >> 1) & 1u, abort)) return false;
+            tmem_fence_after();
+            mma_add(acc, tmem + (q & 1u) * 128u, tile_rows - half);
+            if (i + 1 == t.chunks) mma_add(acc, tmem + kMmaSmallColumn + (done & 1u) * 128u, tile_rows - half);
+            tmem_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.sum_empty[q & 1u]);
+        }
+        done++;
+        const int n = t.n0 + 32 * quarter + lane;
+        if (a.splits > 1) {
+            // partial sums to shared memory (the stages are free: this was the last tile); the blocks of the
+            // cluster that hold the same columns add them up behind a cluster barrier, in mma_combine
+            float *part = reinterpret_cast<float *>(&sm.dense[0][0][0]);
+#pragma unroll
+            for (int j = 0; j < kMmaRows; j++) part[(half + j) * kMmaCols + 32 * quarter + lane] = acc[j];
+            return true;
+        }
+        mma_mark_not_finite(sm, ring, acc, half, lane);
+        if (n < t.p->N) {
+            float *c = t.p->C + (size_t)(t.row0 + half) * (size_t)t.p->N + n;
+            const int rows = min(tile_rows, t.p->M - t.row0) - half;
+#pragma unroll
+            for (int j = 0; j < kMmaRows; j++)
+                if (j < rows) __stcs(c + (size_t)j * (size_t)t.p->N, acc[j]);
+        }
+        sum_warps_barrier();
+        unsigned any = 0;
+        for (int w = 0; w < kMmaMarkWords; w++) any |= *(volatile unsigned *)&sm.again[ring][w];
+        if (any) {
+            for (int j = warp; j < tile_rows; j += kMmaSumWarps)
+                if (((*(volatile unsigned *)&sm.again[ring][j >> 5] >> (j & 31)) & 1u) && t.row0 + j < t.p->M)
+                    mma_row_again(*t.p, t.row0 + j, t.n0, lane);
+            sum_warps_barrier();
+            if (warp == 0 && lane < kMmaMarkWords) sm.again[ring][lane] = 0u;
+        }
+        ring = (ring + 1) % kMmaRing;
+        t.tile += stride;
+    }
+    return true;
+}
+
+// splits > 1: adds the partial sums of the tile over the parts of K, in order.  Block part p takes the rows of
+// the tile's p-th share.
+template <bool TABLE>
+__device__ __forceinline__ void mma_combine(MmaSmem &sm, const MmaArgs &a, unsigned rank, int warp, int lane)
+{
+    MmaTile t;
+    t.tile = blockIdx.x / (2u * (unsigned)a.splits);
+    t.prob = 0;
+    mma_tile_load<TABLE>(t, a, rank);
+    const int tile_rows = 2 * t.rows, part = (int)(rank >> 1);
+    const int per = (tile_rows + a.splits - 1) / a.splits;
+    const int first = part * per, last = min(min(first + per, tile_rows), t.p->M - t.row0);
+    const uint32_t sums = smem_u32(&sm.dense[0][0][0]);
+    uint32_t again = 0;  // lane w < 4: word w of the marks of all parts
+    if (lane < kMmaMarkWords)
+        for (int s = 0; s < a.splits; s++)
+            again |= cluster_load_u32(cluster_map(smem_u32(&sm.again[0][lane]), (unsigned)(2 * s) | (rank & 1u)));
+    for (int j = first + warp; j < last; j += kMmaSumWarps) {
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int s = 0; s < a.splits; s++) {
+            const uint32_t from = cluster_map(sums + (uint32_t)(j * kMmaCols + lane) * 4u, (unsigned)(2 * s) | (rank & 1u));
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i] += cluster_load(from + 128u * i);
+        }
+        float probe = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) probe = fmaf(v[i], 0.f, probe);
+        const unsigned word = __shfl_sync(0xffffffffu, again, j >> 5);
+        if (__any_sync(0xffffffffu, probe != 0.f) || ((word >> (j & 31)) & 1u)) {
+            mma_row_again(*t.p, t.row0 + j, t.n0, lane);
+        } else {
+            float *c = t.p->C + (size_t)(t.row0 + j) * (size_t)t.p->N + t.n0 + lane;
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (t.n0 + lane + 32 * i < t.p->N) c[32 * i] = v[i];
+        }
+    }
+}
+
+// Grid: clusters of 2 * splits blocks; cluster i takes the tiles i, i + clusters, ...  error[0] is set to 1 if a
+// bounded wait ran out.
+// TABLE: the tiles of a table of problems; otherwise of the one problem among the arguments (whose fields then cost
+// no registers).  WIDE: rows of B are 16-byte aligned.
+template <bool TABLE, bool WIDE>
+__global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_constant__ MmaArgs a)
+{
+    extern __shared__ unsigned char smem_raw[];
+    MmaSmem &sm = *reinterpret_cast<MmaSmem *>(smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned rank = cluster_rank();
+    constexpr int kIssueWarp = kMmaSumWarps + kMmaOperandWarps;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kMmaStages; s++) {
+            mbar_init(&sm.full[s], kMmaOperandWarps + (rank & 1u ? 0u : 1u));  // even block: plus the odd one's relay
+            mbar_init(&sm.empty[s], 1);
+        }
+        for (int b = 0; b < 2; b++) {
+            mbar_init(&sm.sum_full[b], 1);
+            mbar_init(&sm.sum_empty[b], kMmaSumWarps + (rank & 1u ? 0u : 1u));
+        }
+        mbar_init(&sm.drain, 1);
+        sm.abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (threadIdx.x < kMmaRing * kMmaMarkWords) (&sm.again[0][0])[threadIdx.x] = 0u;
+    if (warp == kIssueWarp) tmem_alloc<true>(&sm.tmem, 512);
+    tmem_fence_before();
+    __syncthreads();
+    // (the warps that set the shared memory up also publish it)
+    if (warp < kMmaSumWarps) cluster_arrive();
+    else cluster_arrive_relaxed();
+    grid_dependency_wait();
+    cluster_wait();
+    tmem_fence_after();
+    bool ok = true;
+    if (warp < kMmaSumWarps) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kMmaRegsSum));
+        ok = mma_sums<TABLE>(sm, a, rank, warp, lane);
+    } else if (warp < kIssueWarp) {
+        if (kMmaRegsOperand != kMmaRegsLaunch) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kMmaRegsOperand));
+        ok = mma_operands<TABLE, WIDE>(sm, a, rank, warp - kMmaSumWarps, lane);
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kMmaRegsIssue));
+        if (warp == kIssueWarp && (rank & 1u) == 0u) {
+            const bool issuer = elect_one();
+            ok = mma_issue<TABLE>(sm, a, rank, issuer);
+            if (!ok && issuer) {  // multiplies in flight get a bounded chance to end before the tensor memory is freed
+                mma_commit<true>(&sm.drain, 1u << rank);
+                (void)mbar_wait(&sm.drain, 0u);
+            }
+        }
+        if (warp <= kIssueWarp + 1 && (rank & 1u) && lane == 0) ok = mma_relay<TABLE>(sm, a, rank, warp != kIssueWarp);
+    }
+    if (!ok) {
+        *(volatile int *)&sm.abort = 1;
+        *(volatile int *)a.error = 1;
+    }
+    __syncwarp();
+    if (a.splits > 1) {
+        cluster_arrive();
+        cluster_wait();
+        if (warp < kMmaSumWarps && *(volatile int *)&sm.abort == 0) mma_combine<TABLE>(sm, a, rank, warp, lane);
+    }
+    // no block leaves while another one of its cluster may still read its memory or arrive on its barriers
+    tmem_fence_before();
+    cluster_arrive_relaxed();
+    cluster_wait();
+    if (warp == kIssueWarp) tmem_free<true>(sm.tmem, 512);
+}
+
+}  // namespace dlspm

@@ -32,6 +32,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "barrier.cuh"
+
 namespace dlspm {
 
 constexpr int kTileN = 256, kTileK = 32;
@@ -58,7 +60,6 @@ constexpr int kTileStages = 4;                   // B chunks in flight
 // Registers are handed out to a block in units of four warps, so the producer warp costs a whole
 // group of four: the block is launched with 20 warps, of which three leave at once.
 constexpr int kTileThreads = (kTileConsumers + 4) * 32;
-constexpr unsigned kWaitLimit = 1u << 20;  // polls of an mbarrier (a quarter of a microsecond apart) before the kernel gives up
 
 struct TileProblem {
     const float *values;
@@ -86,33 +87,6 @@ struct TileSmem {
     int abort;                                             // set by a thread whose bounded wait ran out
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned parity)
-{
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait: false after kWaitLimit polls (the caller records the failure and leaves).
-__device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned parity)
-{
-    for (unsigned i = 0; i < kWaitLimit; i++)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
-}
 __device__ __forceinline__ void bulk_copy_g2s(void *dst, const void *src, unsigned bytes, unsigned long long *bar)
 {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
@@ -125,25 +99,6 @@ __device__ __forceinline__ void cp_async_4(void *dst, const void *src)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-__device__ __forceinline__ void mbar_arrive(unsigned long long *bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// Bounded wait that also gives up when another thread of the block has raised `abort`.
-__device__ __forceinline__ bool mbar_wait_or_abort(unsigned long long *bar, unsigned parity, volatile int *abort)
-{
-    for (unsigned i = 0; i < kWaitLimit; i++) {
-        if (mbar_try_wait(bar, parity)) return true;
-        // a waiting warp must not take issue slots from the warps that compute
-        if (i >= 4u) __nanosleep(i < 64u ? 64u : 256u);
-        if ((i & 63u) == 63u && *abort) return false;
-    }
-    return false;
-}
 
 // The (tile, chunk) steps of one block in order: tiles blockIdx.x, blockIdx.x + gridDim.x, ... of the
 // launch.  Producer and consumers walk the same sequence independently; `g` numbers the chunks of

@@ -68,20 +68,21 @@ typedef enum dlspm_option {
      * reference CPU loop (SPMM/spmm-esimd-fromfile.cpp:63-83, built without FMA contraction)
      * bit for bit.  0 (default): fused multiply-add. */
     DLSPM_OPT_STRICT_FP32 = 0,
-    /* SpMM kernel choice in prepared batches: 0 = automatic (density threshold below), 1 = row-gather
-     * kernel only, 2 and 3 = shared-memory tiled kernel wherever it applies (N % 4 == 0, aligned dense
-     * operands, strictly ascending columns in every row; restricted by the threshold below only if
-     * the caller has set one).  3 is the form the automatic choice uses: absent entries are
-     * multiplied as zeros, except in chunks of B that hold an infinity or a NaN, which run under the
-     * presence masks, so that a non-finite value of B reaches exactly the rows that reference it, as
-     * in the reference loop.  2 runs every chunk under the masks (slower; kept for tests).  All
-     * choices give the same bits on the same input (apart from the sign of a zero sum, see the
-     * kernel). */
+    /* SpMM kernel choice in prepared batches: 0 = automatic, 1 = row-gather kernel only, 2 and 3 = shared-memory
+     * tiled kernel (fp32 multiply-adds) wherever it applies (N % 4 == 0, aligned dense operands, strictly ascending
+     * columns in every row; restricted by the threshold below only if the caller has set one).  3: absent entries are
+     * multiplied as zeros, except in chunks of B that hold an infinity or a NaN, which run under the presence
+     * masks, so that a non-finite value of B reaches exactly the rows that reference it, as in the reference loop.
+     * 2 runs every chunk under the masks (slower; kept for tests).  1, 2 and 3 give the same bits on the same input
+     * (apart from the sign of a zero sum, see the kernel).  The automatic choice takes, problem by problem, the
+     * row-gather kernel or the tensor cores (from about 5 % nonzeros where the matrix is large; every fp32 product
+     * from six bf16 products of its operands' exact three-part splits, sums in fp32, errors below those of the other
+     * kernels; the tiled kernel above for problems from 45 % nonzeros that do not suit them).  In strict mode
+     * (DLSPM_OPT_STRICT_FP32) it stays on the kernels whose order of additions is the reference's. */
     DLSPM_OPT_SPMM_KERNEL = 1,
-    /* Threshold of the automatic choice, in thousandths: the tiled kernel is taken for problems
-     * whose fraction of nonzeros is at least value/1000.  Default 450: on B200 the tiled kernel
-     * reaches 22.5 TFLOP/s on half-full problems against 15.8 for the row-gather kernel, and loses
-     * at 30 % nonzeros (13.9 against 17).  1001 = never; -1 = back to the default, as if never set. */
+    /* Threshold of the automatic choice, in thousandths: the tiled kernels (tensor cores, fp32 tile kernel) are taken
+     * for problems whose fraction of nonzeros is at least value/1000.  1001 = never; -1 = back to the default, an
+     * estimate of both times from the problem's sizes and nonzeros. */
     DLSPM_OPT_TILE_MIN_DENSITY = 2,
     /* 1: every entry point that takes a CSR pattern validates it before it launches anything
      * (row offsets start at 0, end at nnz, never decrease, no row longer than K, every column index

@@ -1,0 +1,121 @@
+"""GPU parity of the tensor-core SpMM (csrc/spmm_mma.cuh) against the CPU oracle at the edges of its tiles: 128 rows,
+256 columns, 64 columns of the sparse matrix per step, eight lanes per row."""
+import numpy as np
+import pytest
+
+from cases import csr_bernoulli, csr_from_lengths, csr_rowlen_normal, dense, shuffle_rows_columns
+from conftest import TOL, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+def batch_run(pkg, ctx, dev, M, K, N, ro, ci, vals, B):
+    """One problem as a prepared batch that takes the tensor cores whatever its density."""
+    import torch
+
+    ctx.set_option(pkg.OPT_TILE_MIN_DENSITY, 0)
+    try:
+        arr = pkg.ProblemArray(1)
+        guard = 64
+        buf = torch.full((M * N + 2 * guard,), float("nan"), device=dev)
+        arr.set(0, M, K, N, int(ci.size), to_dev(vals, dev), to_dev(ro, dev), to_dev(ci, dev), to_dev(B, dev),
+                buf[guard:guard + M * N])
+        batch = ctx.batch_create(arr)
+        batch.launch()
+        torch.cuda.synchronize()
+        info = batch.info(check_device=True)
+        batch.close()
+    finally:
+        ctx.set_option(pkg.OPT_TILE_MIN_DENSITY, -1)
+    assert info == (0, 1, 0)
+    out = buf.cpu().numpy()
+    assert np.isnan(out[:guard]).all() and np.isnan(out[guard + M * N:]).all(), "wrote outside C"
+    return out[guard:guard + M * N].reshape(M, N)
+
+
+def lone_run(ctx, dev, M, K, N, ro, ci, vals, B):
+    import torch
+
+    out = torch.full((M, N), float("nan"), device=dev)
+    ctx.spmm(M, K, N, int(ci.size), to_dev(vals, dev), to_dev(ro, dev), to_dev(ci, dev), to_dev(B, dev), out)
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+def check(oracle, ro, ci, vals, B, M, N, out, tol=TOL / 50):
+    assert not np.isnan(out).any()
+    bad, worst = oracle.violations(oracle.spmm(vals, ro, ci, B, M, N), out, oracle.spmm_scale(vals, ro, ci, B, M, N), tol)
+    assert bad == 0, worst
+
+
+@pytest.mark.parametrize("M,K,N,density", [(16, 64, 64, 0.3), (17, 1, 64, 1.0), (64, 63, 132, 0.5), (127, 65, 256, 0.1), (128, 64, 260, 0.9),
+                                           (129, 127, 252, 0.02), (300, 200, 516, 0.25), (31, 1000, 128, 1.0), (1000, 129, 68, 0.4)])
+def test_tile_edges(pkg, oracle, ctx, dev, M, K, N, density):
+    seed = M + K + N
+    ro, ci = csr_bernoulli(pkg, M, K, density, seed)
+    vals = pkg.gen_dense_host(int(ci.size), seed, 2)
+    B = dense(pkg, K, N, seed, 10)
+    check(oracle, ro, ci, vals, B, M, N, batch_run(pkg, ctx, dev, M, K, N, ro, ci, vals, B))
+
+
+def test_row_lengths_around_the_lane_group(pkg, oracle, ctx, dev):
+    """Empty and full rows, and rows of up to 64 entries inside one step in front of rows with none."""
+    K, N = 256, 64
+    lengths = [0, 1, 7, 8, 9, 15, 16, 17, 31, 33, 39, 40, 41, 63, 64, 65, 128, 255, 256, 0, 0, 3]
+    ro, ci = csr_from_lengths(pkg, K, lengths, seed=3)
+    ci[ro[12]:ro[13]] = np.arange(20, 20 + lengths[12])  # all in one step
+    ci[ro[14]:ro[15]] = np.arange(64, 64 + lengths[14])
+    vals = pkg.gen_dense_host(int(ci.size), 3, 2)
+    B = dense(pkg, K, N, 3, 10)
+    out = batch_run(pkg, ctx, dev, len(lengths), K, N, ro, ci, vals, B)
+    check(oracle, ro, ci, vals, B, len(lengths), N, out)
+    assert (out[[0, 19, 20]] == 0).all()
+
+
+@pytest.mark.parametrize("M,K,N,density,order", [(1024, 2048, 512, 0.3, "sorted"), (1000, 2000, 510, 0.4, "sorted"),
+                                                 (1024, 2048, 512, 0.3, "shuffled"), (2048, 512, 1028, 0.3, "doubled"),
+                                                 (900, 4100, 301, 0.5, "sorted")])
+def test_lone_launches(pkg, oracle, ctx, dev, M, K, N, density, order):
+    """With and without parts of K in blocks of their own, aligned and ragged widths; columns out of order and
+    repeated columns are found by the kernel."""
+    seed = M + N
+    ro, ci = csr_rowlen_normal(pkg, M, K, 1.0 - density, seed)
+    if order == "shuffled":
+        ci = shuffle_rows_columns(ro, ci, seed)
+    if order == "doubled":
+        ci[ro[5] + 1] = ci[ro[5]]
+        ci[ro[70] + 9] = ci[ro[70] + 8]
+    vals = pkg.gen_dense_host(int(ci.size), seed, 2)
+    B = dense(pkg, K, N, seed, 10)
+    check(oracle, ro, ci, vals, B, M, N, lone_run(ctx, dev, M, K, N, ro, ci, vals, B))
+
+
+@pytest.mark.parametrize("where", ["infinite", "tiny", "huge"])
+def test_numbers_that_cannot_be_split(pkg, oracle, ctx, dev, where):
+    """Infinities and NaN reach the rows that refer to them and no others; magnitudes at the ends of the range keep
+    their precision."""
+    M, K, N = 300, 200, 512
+    ro, ci = csr_rowlen_normal(pkg, M, K, 0.5, 4242)
+    vals = pkg.gen_dense_host(int(ci.size), 4242, 2)
+    B = dense(pkg, K, N, 4242, 10).copy()
+    if where == "infinite":
+        used = 130
+        B[used, 5], B[used, 300] = np.nan, -np.inf
+        out = batch_run(pkg, ctx, dev, M, K, N, ro, ci, vals, B)
+        refers = np.array([used in ci[ro[i]:ro[i + 1]] for i in range(M)])
+        assert refers.any() and not refers.all()
+        assert np.isfinite(out[~refers]).all()
+        assert np.isnan(out[refers][:, 5]).all() and np.isinf(out[refers][:, 300]).all()
+        B[used, 5] = B[used, 300] = 0
+        want = oracle.spmm(vals, ro, ci, B, M, N)
+        keep = np.ones(N, bool)
+        keep[[5, 300]] = False
+        assert np.allclose(out[:, keep], want[:, keep], rtol=1e-4, atol=1e-4)
+        return
+    if where == "tiny":
+        vals = (vals * np.float32(1e-36)).astype(np.float32)
+        B *= np.float32(1e20)
+    else:
+        B[7, 3] = np.float32(3.4e38)  # rounds to infinity as bf16
+        vals *= np.float32(1e-3)
+    check(oracle, ro, ci, vals, B, M, N, batch_run(pkg, ctx, dev, M, K, N, ro, ci, vals, B))
