@@ -18,6 +18,7 @@
 
 #include "common.cuh"
 #include "fused_device.cuh"
+#include "launch.cuh"
 #include "sddmm_device.cuh"
 
 using namespace dlspm;
@@ -40,6 +41,7 @@ fused_rows_kernel(const int *__restrict__ row_offsets, const int *__restrict__ c
                   const float *__restrict__ c, const float *__restrict__ b, const float *__restrict__ d,
                   float *__restrict__ e, int M, int chunks, float scale)
 {
+    kernel_begin();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row = blockIdx.x * kWarps + warp;
     if (row >= M) return;
@@ -84,6 +86,7 @@ fused_rows_split_kernel(const int *__restrict__ row_offsets, const int *__restri
                         const float *__restrict__ c, const float *__restrict__ b, const float *__restrict__ d,
                         float *__restrict__ e, int M, int chunks, float scale, int split_shift)
 {
+    kernel_begin();
     extern __shared__ float4 part[];  // [kWarps][G * R]
     __shared__ float stat[kWarps][2];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -181,6 +184,7 @@ fused_generic_kernel(const int *__restrict__ row_offsets, const int *__restrict_
                      const float *__restrict__ c, const float *__restrict__ b, const float *__restrict__ d,
                      float *__restrict__ e, int M, int N, float scale)
 {
+    kernel_begin();
     constexpr int U = 4;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row = blockIdx.x * kWarps + warp;
@@ -245,6 +249,7 @@ fused_rows_scalar_kernel(const int *__restrict__ row_offsets, const int *__restr
                          const float *__restrict__ c, const float *__restrict__ b, const float *__restrict__ d,
                          float *__restrict__ e, int M, int N, float scale)
 {
+    kernel_begin();
     constexpr int NG = 32 / G;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row = blockIdx.x * kWarps + warp;
@@ -329,9 +334,9 @@ void launch_scalar(const int *ro, const int *ci, const float *c, const float *b,
 {
     const unsigned blocks = (unsigned)dlspm_ceil_div(M, kWarps);
     const int per_lane = dlspm_ceil_div(N, G);
-    if (per_lane <= 2) fused_rows_scalar_kernel<G, 2, MODE><<<blocks, kWarps * 32, 0, st>>>(ro, ci, c, b, d, e, M, N, scale);
-    else if (per_lane <= 4) fused_rows_scalar_kernel<G, 4, MODE><<<blocks, kWarps * 32, 0, st>>>(ro, ci, c, b, d, e, M, N, scale);
-    else fused_rows_scalar_kernel<G, 8, MODE><<<blocks, kWarps * 32, 0, st>>>(ro, ci, c, b, d, e, M, N, scale);
+    if (per_lane <= 2) launch_overlapped(fused_rows_scalar_kernel<G, 2, MODE>, blocks, kWarps * 32, 0, st, ro, ci, c, b, d, e, M, N, scale);
+    else if (per_lane <= 4) launch_overlapped(fused_rows_scalar_kernel<G, 4, MODE>, blocks, kWarps * 32, 0, st, ro, ci, c, b, d, e, M, N, scale);
+    else launch_overlapped(fused_rows_scalar_kernel<G, 8, MODE>, blocks, kWarps * 32, 0, st, ro, ci, c, b, d, e, M, N, scale);
 }
 
 // Patterns of one to a few waves of thread blocks, as in the SDDMM launcher: two or four warps per row
@@ -375,13 +380,12 @@ void launch_fast(const int *ro, const int *ci, const float *c, const float *b, c
     if (split_shift > 0) {
         const long long warps = (long long)M << split_shift;
         const size_t smem = sizeof(float4) * (size_t)kWarps * G * R;
-        fused_rows_split_kernel<G, R, MODE><<<(unsigned)((warps + kWarps - 1) / kWarps), kWarps * 32, smem, st>>>(
-            ro, ci, c, b, d, e, M, chunks, scale, split_shift);
+        launch_overlapped(fused_rows_split_kernel<G, R, MODE>, (unsigned)((warps + kWarps - 1) / kWarps), kWarps * 32, smem, st, ro, ci, c, b, d, e, M, chunks, scale, split_shift);
         return;
     }
     if constexpr (G == 32 && R == 4) {
         if ((long long)M > 2LL * kWarps * sm_count) {  // more rows than two resident blocks per SM hold
-            fused_rows_kernel<G, R, MODE, true><<<dlspm_ceil_div(M, kWarps), kWarps * 32, 0, st>>>(ro, ci, c, b, d, e, M, chunks, scale);
+            launch_overlapped(fused_rows_kernel<G, R, MODE, true>, dlspm_ceil_div(M, kWarps), kWarps * 32, 0, st, ro, ci, c, b, d, e, M, chunks, scale);
             return;
         }
     }
@@ -390,17 +394,17 @@ void launch_fast(const int *ro, const int *ci, const float *c, const float *b, c
         const long long blocks = dlspm_ceil_div(M, kWarps);
         const long long w6 = (blocks + 6LL * sm_count - 1) / (6LL * sm_count), w8 = (blocks + 8LL * sm_count - 1) / (8LL * sm_count);
         if ((double)w8 * 8.0 * 1.07 < (double)w6 * 6.0) {
-            fused_rows_kernel<G, R, MODE, true><<<(unsigned)blocks, kWarps * 32, 0, st>>>(ro, ci, c, b, d, e, M, chunks, scale);
+            launch_overlapped(fused_rows_kernel<G, R, MODE, true>, (unsigned)blocks, kWarps * 32, 0, st, ro, ci, c, b, d, e, M, chunks, scale);
             return;
         }
     }
     if constexpr (G == 4 && R == 2) {
         if (wide) {  // rows of 32 floats, 32-byte aligned operands, a long launch: 256-bit loads
-            fused_rows_kernel<G, R, MODE, false, true><<<dlspm_ceil_div(M, kWarps), kWarps * 32, 0, st>>>(ro, ci, c, b, d, e, M, chunks, scale);
+            launch_overlapped(fused_rows_kernel<G, R, MODE, false, true>, dlspm_ceil_div(M, kWarps), kWarps * 32, 0, st, ro, ci, c, b, d, e, M, chunks, scale);
             return;
         }
     }
-    fused_rows_kernel<G, R, MODE><<<dlspm_ceil_div(M, kWarps), kWarps * 32, 0, st>>>(ro, ci, c, b, d, e, M, chunks, scale);
+    launch_overlapped(fused_rows_kernel<G, R, MODE>, dlspm_ceil_div(M, kWarps), kWarps * 32, 0, st, ro, ci, c, b, d, e, M, chunks, scale);
 }
 
 // Warps per row (as a shift) for a pattern with few rows, by the rule of the SDDMM kernel: share
@@ -461,7 +465,7 @@ int fused_launch(dlspm_ctx *ctx, int M, int K, int N, int nnz, const int *row_of
         else if (N <= 128) launch_scalar<16, MODE>(row_offsets, column_indices, C, B, D, E, M, N, scale, st);
         else launch_scalar<32, MODE>(row_offsets, column_indices, C, B, D, E, M, N, scale, st);
     } else {
-        fused_generic_kernel<MODE><<<dlspm_ceil_div(M, kWarps), kWarps * 32, 0, st>>>(row_offsets, column_indices, C, B, D, E, M, N, scale);
+        launch_overlapped(fused_generic_kernel<MODE>, dlspm_ceil_div(M, kWarps), kWarps * 32, 0, st, row_offsets, column_indices, C, B, D, E, M, N, scale);
     }
     DLSPM_CUDA_TRY(ctx, cudaGetLastError());
     return DLSPM_OK;

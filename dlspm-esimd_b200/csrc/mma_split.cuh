@@ -14,6 +14,7 @@
 #include <stdint.h>
 
 #include "barrier.cuh"
+#include "launch.cuh"
 
 namespace dlspm {
 
@@ -141,11 +142,6 @@ __device__ __forceinline__ bool mbar_wait_suspended(unsigned long long *bar, uns
     }
     return false;
 }
-
-// Work of the previous kernel in the stream is complete and visible from here on (launches that may start
-// before it has ended); and the next kernel may start its own preamble.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // True on one lane of a converged warp.
 __device__ __forceinline__ bool elect_one()

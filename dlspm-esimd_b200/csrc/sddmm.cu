@@ -9,6 +9,7 @@
 #include <cstdint>
 
 #include "common.cuh"
+#include "launch.cuh"
 #include "sddmm_device.cuh"
 
 using namespace dlspm;
@@ -30,6 +31,7 @@ sddmm_rows_kernel(const int *__restrict__ row_offsets, const int *__restrict__ c
                   const float *__restrict__ lhs, const float *__restrict__ rhs, float *__restrict__ out,
                   int M, int chunks, const float *__restrict__ mask, int split_shift, int k_shift)
 {
+    kernel_begin();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // (1 << split_shift) * (1 << k_shift) warps share a row: the passes of 32 nonzeros are dealt
     // out in turn, and within a pass a warp takes every (1 << k_shift)-th nonzero of each lane
@@ -79,6 +81,7 @@ sddmm_rows_long_kernel(const int *__restrict__ row_offsets, const int *__restric
                        const float *__restrict__ lhs, const float *__restrict__ rhs, float *__restrict__ out,
                        int M, int chunks, const float *__restrict__ mask, int k_shift)
 {
+    kernel_begin();
     constexpr int G = 32, kSeg = G * R;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // 1 << k_shift warps share a row, each taking every (1 << k_shift)-th nonzero of a pass
@@ -115,6 +118,7 @@ sddmm_generic_kernel(const int *__restrict__ row_offsets, const int *__restrict_
                      const float *__restrict__ lhs, const float *__restrict__ rhs, float *__restrict__ out,
                      int M, int N, const float *__restrict__ mask)
 {
+    kernel_begin();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row = blockIdx.x * kWarps + warp;
     if (row >= M) return;
@@ -163,6 +167,7 @@ sddmm_rows_scalar_kernel(const int *__restrict__ row_offsets, const int *__restr
                          const float *__restrict__ lhs, const float *__restrict__ rhs, float *__restrict__ out,
                          int M, int N, const float *__restrict__ mask, int split_shift)
 {
+    kernel_begin();
     constexpr int NG = 32 / G;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // 1 << split_shift warps share a row and take its passes in turn (patterns with few rows)
@@ -212,9 +217,9 @@ void launch_scalar(const int *ro, const int *ci, const float *lhs, const float *
 {
     const unsigned blocks = (unsigned)((((long long)M << split_shift) + kWarps - 1) / kWarps);
     const int per_lane = dlspm_ceil_div(N, G);
-    if (per_lane <= 2) sddmm_rows_scalar_kernel<G, 2><<<blocks, kWarps * 32, 0, st>>>(ro, ci, lhs, rhs, out, M, N, mask, split_shift);
-    else if (per_lane <= 4) sddmm_rows_scalar_kernel<G, 4><<<blocks, kWarps * 32, 0, st>>>(ro, ci, lhs, rhs, out, M, N, mask, split_shift);
-    else sddmm_rows_scalar_kernel<G, 8><<<blocks, kWarps * 32, 0, st>>>(ro, ci, lhs, rhs, out, M, N, mask, split_shift);
+    if (per_lane <= 2) launch_overlapped(sddmm_rows_scalar_kernel<G, 2>, blocks, kWarps * 32, 0, st, ro, ci, lhs, rhs, out, M, N, mask, split_shift);
+    else if (per_lane <= 4) launch_overlapped(sddmm_rows_scalar_kernel<G, 4>, blocks, kWarps * 32, 0, st, ro, ci, lhs, rhs, out, M, N, mask, split_shift);
+    else launch_overlapped(sddmm_rows_scalar_kernel<G, 8>, blocks, kWarps * 32, 0, st, ro, ci, lhs, rhs, out, M, N, mask, split_shift);
 }
 
 // Patterns of one to a few waves of thread blocks: the last wave is often nearly empty (6144 rows are
@@ -268,20 +273,20 @@ void launch_fast(const int *ro, const int *ci, const float *lhs, const float *rh
         // the capped build pays when it saves a wave of thread blocks (eight instead of six per SM)
         const long long w6 = (blocks + 6LL * sm_count - 1) / (6LL * sm_count), w8 = (blocks + 8LL * sm_count - 1) / (8LL * sm_count);
         if (k_shift == 0 && (double)w8 * 8.0 * 1.07 < (double)w6 * 6.0) {
-            sddmm_rows_kernel<G, R, false, true><<<blocks, kWarps * 32, 0, st>>>(ro, ci, lhs, rhs, out, M, chunks, mask, split_shift, 0);
+            launch_overlapped(sddmm_rows_kernel<G, R, false, true>, blocks, kWarps * 32, 0, st, ro, ci, lhs, rhs, out, M, chunks, mask, split_shift, 0);
             return;
         }
     }
     if constexpr (G == 4 && R == 2) {
         if (wide && k_shift == 0) {
-            sddmm_rows_kernel<G, R, false, false, true><<<blocks, kWarps * 32, 0, st>>>(ro, ci, lhs, rhs, out, M, chunks, mask, split_shift, 0);
+            launch_overlapped(sddmm_rows_kernel<G, R, false, false, true>, blocks, kWarps * 32, 0, st, ro, ci, lhs, rhs, out, M, chunks, mask, split_shift, 0);
             return;
         }
     }
     if (k_shift > 0)
-        sddmm_rows_kernel<G, R, true><<<blocks, kWarps * 32, 0, st>>>(ro, ci, lhs, rhs, out, M, chunks, mask, split_shift, k_shift);
+        launch_overlapped(sddmm_rows_kernel<G, R, true>, blocks, kWarps * 32, 0, st, ro, ci, lhs, rhs, out, M, chunks, mask, split_shift, k_shift);
     else
-        sddmm_rows_kernel<G, R, false><<<blocks, kWarps * 32, 0, st>>>(ro, ci, lhs, rhs, out, M, chunks, mask, split_shift, 0);
+        launch_overlapped(sddmm_rows_kernel<G, R, false>, blocks, kWarps * 32, 0, st, ro, ci, lhs, rhs, out, M, chunks, mask, split_shift, 0);
 }
 
 // Warps per row (as a shift) for a pattern with few rows: one warp per row would leave most of the
@@ -376,19 +381,19 @@ int sddmm_launch(dlspm_ctx *ctx, int M, int K, int N, int nnz, const int *row_of
         // segments below that
         const int kshift = sddmm_k_shift(ctx, M, nnz, 0, 0.0);
         const unsigned lblocks = (unsigned)((((long long)M << kshift) + kWarps - 1) / kWarps);
-        if (N > 2048 && kshift > 0) sddmm_rows_long_kernel<4, true><<<lblocks, kWarps * 32, 0, st>>>(row_offsets, column_indices, lhs, rhs, out_values, M, N / 4, mask, kshift);
-        else if (N > 2048) sddmm_rows_long_kernel<4, false><<<lblocks, kWarps * 32, 0, st>>>(row_offsets, column_indices, lhs, rhs, out_values, M, N / 4, mask, 0);
-        else if (kshift > 0) sddmm_rows_long_kernel<8, true><<<lblocks, kWarps * 32, 0, st>>>(row_offsets, column_indices, lhs, rhs, out_values, M, N / 4, mask, kshift);
-        else sddmm_rows_long_kernel<8, false><<<lblocks, kWarps * 32, 0, st>>>(row_offsets, column_indices, lhs, rhs, out_values, M, N / 4, mask, 0);
+        if (N > 2048 && kshift > 0) launch_overlapped(sddmm_rows_long_kernel<4, true>, lblocks, kWarps * 32, 0, st, row_offsets, column_indices, lhs, rhs, out_values, M, N / 4, mask, kshift);
+        else if (N > 2048) launch_overlapped(sddmm_rows_long_kernel<4, false>, lblocks, kWarps * 32, 0, st, row_offsets, column_indices, lhs, rhs, out_values, M, N / 4, mask, 0);
+        else if (kshift > 0) launch_overlapped(sddmm_rows_long_kernel<8, true>, lblocks, kWarps * 32, 0, st, row_offsets, column_indices, lhs, rhs, out_values, M, N / 4, mask, kshift);
+        else launch_overlapped(sddmm_rows_long_kernel<8, false>, lblocks, kWarps * 32, 0, st, row_offsets, column_indices, lhs, rhs, out_values, M, N / 4, mask, 0);
     } else if (N <= 256) {  // no 128-bit loads: the group layout with scalar elements
         const int shift = sddmm_split_shift(ctx, M, nnz);
         if (N <= 64) launch_scalar<8>(row_offsets, column_indices, lhs, rhs, out_values, M, N, mask, shift, st);
         else if (N <= 128) launch_scalar<16>(row_offsets, column_indices, lhs, rhs, out_values, M, N, mask, shift, st);
         else launch_scalar<32>(row_offsets, column_indices, lhs, rhs, out_values, M, N, mask, shift, st);
     } else if (vec == 2) {
-        sddmm_generic_kernel<2><<<blocks, kWarps * 32, 0, st>>>(row_offsets, column_indices, lhs, rhs, out_values, M, N, mask);
+        launch_overlapped(sddmm_generic_kernel<2>, blocks, kWarps * 32, 0, st, row_offsets, column_indices, lhs, rhs, out_values, M, N, mask);
     } else {
-        sddmm_generic_kernel<1><<<blocks, kWarps * 32, 0, st>>>(row_offsets, column_indices, lhs, rhs, out_values, M, N, mask);
+        launch_overlapped(sddmm_generic_kernel<1>, blocks, kWarps * 32, 0, st, row_offsets, column_indices, lhs, rhs, out_values, M, N, mask);
     }
     DLSPM_CUDA_TRY(ctx, cudaGetLastError());
     return DLSPM_OK;

@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "launch.cuh"
 #include "spmm_device.cuh"
 
 using namespace dlspm;
@@ -31,6 +32,7 @@ struct SpmmArgs {
 template <int VEC, int U, bool STRICT, int J>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_rows_kernel(const SpmmArgs a)
 {
+    kernel_begin();
     __shared__ int2 stage[kWarpsPerCta][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long tile = blockIdx.x;
@@ -51,6 +53,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_rows_kernel(const Spmm
 template <int VEC, int U, int S>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_rows_split_kernel(const SpmmArgs a)
 {
+    kernel_begin();
     __shared__ int2 stage[kWarpsPerCta][32];
     __shared__ float part[kWarpsPerCta][U][32 * VEC];
     constexpr int kRows = kWarpsPerCta / S;
@@ -79,7 +82,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_rows_split_kernel(cons
             if (p < end) cv = make_int2(__ldg(a.cols + p), __float_as_int(__ldg(a.values + p)));
             stage[warp][lane] = cv;
             __syncwarp();
-            spmm_accumulate_staged<VEC, U, false, kLoneBatch<U>>(stage[warp], min(32, end - base), a.B, a.N, cidx, acc);
+            spmm_accumulate_staged<VEC, U, false, kLoneBatch<VEC, U>>(stage[warp], min(32, end - base), a.B, a.N, cidx, acc);
             __syncwarp();
         }
     }
@@ -108,7 +111,7 @@ template <int VEC, int U, int S>
 void launch_rows_split(SpmmArgs a, int slabs, cudaStream_t st)
 {
     a.row_groups = dlspm_ceil_div(a.M, kWarpsPerCta / S);
-    spmm_rows_split_kernel<VEC, U, S><<<(unsigned)((long long)a.row_groups * slabs), kWarpsPerCta * 32, 0, st>>>(a);
+    launch_overlapped(spmm_rows_split_kernel<VEC, U, S>, (unsigned)((long long)a.row_groups * slabs), kWarpsPerCta * 32, 0, st, a);
 }
 
 // Narrow dense operand (N <= 64 floats, 16-byte aligned rows): a full warp per row would leave most
@@ -119,6 +122,7 @@ void launch_rows_split(SpmmArgs a, int slabs, cudaStream_t st)
 template <int LANES, bool STRICT>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_subwarp_kernel(const SpmmArgs a)
 {
+    kernel_begin();
     constexpr int kRowsPerWarp = 32 / LANES;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane / LANES, t = lane % LANES;
@@ -167,6 +171,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_subwarp_kernel(const S
 template <int LANES>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_subwarp_shared_kernel(const SpmmArgs a)
 {
+    kernel_begin();
     constexpr int kGroups = 32 / LANES;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane / LANES, t = lane % LANES;
@@ -211,7 +216,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_subwarp_shared_kernel(
 template <int LANES>
 void launch_subwarp_shared(const SpmmArgs &a, cudaStream_t st)
 {
-    spmm_subwarp_shared_kernel<LANES><<<(unsigned)dlspm_ceil_div(a.M, kWarpsPerCta), kWarpsPerCta * 32, 0, st>>>(a);
+    launch_overlapped(spmm_subwarp_shared_kernel<LANES>, (unsigned)dlspm_ceil_div(a.M, kWarpsPerCta), kWarpsPerCta * 32, 0, st, a);
 }
 
 template <int LANES>
@@ -219,28 +224,28 @@ void launch_subwarp(const SpmmArgs &a, bool strict, cudaStream_t st)
 {
     const int rows_per_block = kWarpsPerCta * (32 / LANES);
     const unsigned blocks = (unsigned)dlspm_ceil_div(a.M, rows_per_block);
-    if (strict) spmm_subwarp_kernel<LANES, true><<<blocks, kWarpsPerCta * 32, 0, st>>>(a);
-    else spmm_subwarp_kernel<LANES, false><<<blocks, kWarpsPerCta * 32, 0, st>>>(a);
+    if (strict) launch_overlapped(spmm_subwarp_kernel<LANES, true>, blocks, kWarpsPerCta * 32, 0, st, a);
+    else launch_overlapped(spmm_subwarp_kernel<LANES, false>, blocks, kWarpsPerCta * 32, 0, st, a);
 }
 
 template <int VEC, int U>
 void launch_rows(const SpmmArgs &a, int slabs, bool strict, cudaStream_t st)
 {
     const long long tiles = (long long)a.row_groups * slabs;
-    dim3 grid((unsigned)tiles), block(kWarpsPerCta * 32);
+    const unsigned grid = (unsigned)tiles, block = kWarpsPerCta * 32;
     // The narrow slabs exist in two builds: with the batched loads (74 to 76 registers, three
     // resident blocks) for launches of a few waves, where the latency chain of a warp counts, and
     // with the plain loop (32 and 44 registers) for long launches, where occupancy hides it.
     // Measured: one-chunk slabs, 32768 x 8192 (9 waves) 0.71 -> 0.61 ms with the plain loop but
     // 8192 x 8192 (2.3 waves) 0.19 -> 0.20 ms; two-chunk slabs, 32768 x 2048 413 -> 338 us.
     const int waves = U == 1 ? 6 : 2;
-    const bool lone = kLoneBatch<U> > 0 && tiles <= (long long)waves * 3 * a.sm_count;
+    const bool lone = kLoneBatch<VEC, U> > 0 && tiles <= (long long)waves * 3 * a.sm_count;
     if (lone) {
-        if (strict) spmm_rows_kernel<VEC, U, true, kLoneBatch<U>><<<grid, block, 0, st>>>(a);
-        else spmm_rows_kernel<VEC, U, false, kLoneBatch<U>><<<grid, block, 0, st>>>(a);
+        if (strict) launch_overlapped(spmm_rows_kernel<VEC, U, true, kLoneBatch<VEC, U>>, grid, block, 0, st, a);
+        else launch_overlapped(spmm_rows_kernel<VEC, U, false, kLoneBatch<VEC, U>>, grid, block, 0, st, a);
     } else {
-        if (strict) spmm_rows_kernel<VEC, U, true, 0><<<grid, block, 0, st>>>(a);
-        else spmm_rows_kernel<VEC, U, false, 0><<<grid, block, 0, st>>>(a);
+        if (strict) launch_overlapped(spmm_rows_kernel<VEC, U, true, 0>, grid, block, 0, st, a);
+        else launch_overlapped(spmm_rows_kernel<VEC, U, false, 0>, grid, block, 0, st, a);
     }
 }
 

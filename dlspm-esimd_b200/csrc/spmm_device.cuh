@@ -124,13 +124,14 @@ __device__ __forceinline__ void spmm_accumulate_staged(const int2 *stage, int cn
 }
 
 // Nonzeros taken at once by a lone launch (0: the plain unrolled loop): 8 loads in flight per lane
-// for the one- and two-chunk slabs.  Measured on lone matrices of 256 to 2048 rows: 512 x 512 at
+// for the one- and two-chunk slabs of 16-byte loads.  Measured on lone matrices of 256 to 2048 rows: 512 x 512 at
 // 10 %, N = 128 went from 7.7 to 5.2 us, 1024 x 1024 at 30 % from 20.5 to 17.5 us; 16 nonzeros at
-// once (one-chunk) or 8 (two-chunk) lost again through registers.  The grouped launch keeps the
+// once (one-chunk) or 8 (two-chunk) lost again through registers.  Narrower loads need fewer registers each, so more
+// of them are in flight.  The grouped launch keeps the
 // plain loop for every width: it holds all three widths in one kernel, its occupancy is what
 // hides the latency there, and the batched loads would cost it registers.
-template <int U>
-constexpr int kLoneBatch = U == 1 ? 8 : U == 2 ? 4 : 0;
+template <int VEC, int U>
+constexpr int kLoneBatch = VEC == 4 ? (U == 1 ? 8 : U == 2 ? 4 : 0) : VEC == 2 ? (U == 1 ? 16 : U == 2 ? 8 : 4) : (U == 4 ? 8 : 16);
 
 // The (column, value) pair of nonzero start + lane of a row, (0, 0) beyond its end: what the first
 // staging step of spmm_warp_row_slab loads.  A caller that walks several rows can ask for the next
