@@ -41,7 +41,7 @@ fused_rows_kernel(const int *__restrict__ row_offsets, const int *__restrict__ c
                   const float *__restrict__ c, const float *__restrict__ b, const float *__restrict__ d,
                   float *__restrict__ e, int M, int chunks, float scale)
 {
-    kernel_begin();
+    grid_dependency_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row = blockIdx.x * kWarps + warp;
     if (row >= M) return;
@@ -86,7 +86,7 @@ fused_rows_split_kernel(const int *__restrict__ row_offsets, const int *__restri
                         const float *__restrict__ c, const float *__restrict__ b, const float *__restrict__ d,
                         float *__restrict__ e, int M, int chunks, float scale, int split_shift)
 {
-    kernel_begin();
+    grid_dependency_wait();
     extern __shared__ float4 part[];  // [kWarps][G * R]
     __shared__ float stat[kWarps][2];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -184,7 +184,7 @@ fused_generic_kernel(const int *__restrict__ row_offsets, const int *__restrict_
                      const float *__restrict__ c, const float *__restrict__ b, const float *__restrict__ d,
                      float *__restrict__ e, int M, int N, float scale)
 {
-    kernel_begin();
+    grid_dependency_wait();
     constexpr int U = 4;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row = blockIdx.x * kWarps + warp;
@@ -249,7 +249,7 @@ fused_rows_scalar_kernel(const int *__restrict__ row_offsets, const int *__restr
                          const float *__restrict__ c, const float *__restrict__ b, const float *__restrict__ d,
                          float *__restrict__ e, int M, int N, float scale)
 {
-    kernel_begin();
+    grid_dependency_wait();
     constexpr int NG = 32 / G;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row = blockIdx.x * kWarps + warp;

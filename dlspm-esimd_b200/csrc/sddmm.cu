@@ -31,7 +31,7 @@ sddmm_rows_kernel(const int *__restrict__ row_offsets, const int *__restrict__ c
                   const float *__restrict__ lhs, const float *__restrict__ rhs, float *__restrict__ out,
                   int M, int chunks, const float *__restrict__ mask, int split_shift, int k_shift)
 {
-    kernel_begin();
+    grid_dependency_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // (1 << split_shift) * (1 << k_shift) warps share a row: the passes of 32 nonzeros are dealt
     // out in turn, and within a pass a warp takes every (1 << k_shift)-th nonzero of each lane
@@ -61,12 +61,14 @@ sddmm_rows_kernel(const int *__restrict__ row_offsets, const int *__restrict__ c
             const float r = sddmm_pass<G, R, true>(a, rhs4, chunks, col, g, t, kmask, ksub);
             if (p < end && (t & kmask) == ksub) out[p] = mask ? __ldg(mask + p) * r : r;
         } else {
-            // nonzeros dealt to the lane groups in turn: this lane ends up with nonzero `q` of the row
+            // nonzeros dealt to the lane groups in turn: this lane ends up with nonzero `q` of the row, whose factor
+            // is asked for in front of the gathers (behind them its latency came on top of every pass)
+            const int q = base + sddmm_dealt_slot(G, g, t);
+            const float factor = mask && q < end ? __ldg(mask + q) : 1.f;
             float r;
             if constexpr (WIDE) r = sddmm_pass_dealt_wide(a, rhs4, col, g, t);
             else r = sddmm_pass_dealt<G, R>(a, rhs4, chunks, col, g, t);
-            const int q = base + sddmm_dealt_slot(G, g, t);
-            if (q < end) out[q] = mask ? __ldg(mask + q) * r : r;
+            if (q < end) out[q] = factor * r;
         }
     }
 }
@@ -81,7 +83,7 @@ sddmm_rows_long_kernel(const int *__restrict__ row_offsets, const int *__restric
                        const float *__restrict__ lhs, const float *__restrict__ rhs, float *__restrict__ out,
                        int M, int chunks, const float *__restrict__ mask, int k_shift)
 {
-    kernel_begin();
+    grid_dependency_wait();
     constexpr int G = 32, kSeg = G * R;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // 1 << k_shift warps share a row, each taking every (1 << k_shift)-th nonzero of a pass
@@ -118,7 +120,7 @@ sddmm_generic_kernel(const int *__restrict__ row_offsets, const int *__restrict_
                      const float *__restrict__ lhs, const float *__restrict__ rhs, float *__restrict__ out,
                      int M, int N, const float *__restrict__ mask)
 {
-    kernel_begin();
+    grid_dependency_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row = blockIdx.x * kWarps + warp;
     if (row >= M) return;
@@ -167,7 +169,7 @@ sddmm_rows_scalar_kernel(const int *__restrict__ row_offsets, const int *__restr
                          const float *__restrict__ lhs, const float *__restrict__ rhs, float *__restrict__ out,
                          int M, int N, const float *__restrict__ mask, int split_shift)
 {
-    kernel_begin();
+    grid_dependency_wait();
     constexpr int NG = 32 / G;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // 1 << split_shift warps share a row and take its passes in turn (patterns with few rows)
@@ -265,7 +267,11 @@ void launch_fast(const int *ro, const int *ci, const float *lhs, const float *rh
             }
             per_sm = n > 0 ? n : 4;
         }
-        split_shift = sddmm_wave_shift(((long long)M + kWarps - 1) / kWarps, (long long)per_sm * sm_count, avg_row);
+        const long long blocks = ((long long)M + kWarps - 1) / kWarps;
+        // (the two-chunk layout has a build for eight resident blocks, below: what fits one wave of it is not shared;
+        // the warps then walk through the columns side by side and meet in L1.  8192 x 8192, N = 64, 98 -> 91 us.)
+        if (!(G == 8 && R == 2 && blocks > (long long)per_sm * sm_count && blocks <= 8LL * sm_count))
+            split_shift = sddmm_wave_shift(blocks, (long long)per_sm * sm_count, avg_row);
     }
     const long long warps = (long long)M << (split_shift + k_shift);
     const unsigned blocks = (unsigned)((warps + kWarps - 1) / kWarps);

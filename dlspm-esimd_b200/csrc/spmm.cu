@@ -32,7 +32,7 @@ struct SpmmArgs {
 template <int VEC, int U, bool STRICT, int J>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_rows_kernel(const SpmmArgs a)
 {
-    kernel_begin();
+    grid_dependency_wait();
     __shared__ int2 stage[kWarpsPerCta][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long tile = blockIdx.x;
@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_rows_kernel(const Spmm
 template <int VEC, int U, int S>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_rows_split_kernel(const SpmmArgs a)
 {
-    kernel_begin();
+    grid_dependency_wait();
     __shared__ int2 stage[kWarpsPerCta][32];
     __shared__ float part[kWarpsPerCta][U][32 * VEC];
     constexpr int kRows = kWarpsPerCta / S;
@@ -122,7 +122,7 @@ void launch_rows_split(SpmmArgs a, int slabs, cudaStream_t st)
 template <int LANES, bool STRICT>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_subwarp_kernel(const SpmmArgs a)
 {
-    kernel_begin();
+    grid_dependency_wait();
     constexpr int kRowsPerWarp = 32 / LANES;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane / LANES, t = lane % LANES;
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_subwarp_kernel(const S
 template <int LANES>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_subwarp_shared_kernel(const SpmmArgs a)
 {
-    kernel_begin();
+    grid_dependency_wait();
     constexpr int kGroups = 32 / LANES;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane / LANES, t = lane % LANES;

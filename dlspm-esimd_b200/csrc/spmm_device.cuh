@@ -93,26 +93,60 @@ __device__ __forceinline__ void spmm_accumulate_staged(const int2 *stage, int cn
             }
         }
     } else {
-        for (int j = 0; j < cnt; j += J) {
+        // Lanes beyond the width load its last columns and do not store their sums; whole chunks beyond it are
+        // skipped.  A full batch is free of tests (with them a row of N = 49 cost 39 instructions per nonzero).
+        int at[U];
+        bool in[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            at[u] = min(cidx[u], N - VEC);
+            in[u] = u == 0 || __any_sync(0xffffffffu, cidx[u] < N);
+        }
+        int j = 0;
+        for (; j + J <= cnt; j += J) {
             float b[J][U][VEC];
             float a[J];
 #pragma unroll
             for (int jj = 0; jj < J; jj++) {
+                const int2 e = stage[j + jj];
+                a[jj] = __int_as_float(e.y);
+                const float *brow = B + (size_t)e.x * (size_t)N;
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (in[u]) load_vec<VEC>(brow + at[u], b[jj][u]);
+            }
+#pragma unroll
+            for (int jj = 0; jj < J; jj++) {
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if (in[u]) {
+#pragma unroll
+                        for (int v = 0; v < VEC; v++) acc[u][v] = mad<STRICT>(a[jj], b[jj][u][v], acc[u][v]);
+                    }
+                }
+            }
+        }
+        // the rest, in batches of a quarter
+        constexpr int T = J / 4;
+        for (; j < cnt; j += T) {
+            float b[T][U][VEC];
+            float a[T];
+#pragma unroll
+            for (int jj = 0; jj < T; jj++) {
                 const bool live = j + jj < cnt;
                 const int2 e = stage[(j + jj) & 31];
                 a[jj] = __int_as_float(e.y);
                 const float *brow = B + (size_t)e.x * (size_t)N;
 #pragma unroll
-                for (int u = 0; u < U; u++) {
-                    if (live && cidx[u] < N) load_vec<VEC>(brow + cidx[u], b[jj][u]);
-                }
+                for (int u = 0; u < U; u++)
+                    if (live && in[u]) load_vec<VEC>(brow + at[u], b[jj][u]);
             }
 #pragma unroll
-            for (int jj = 0; jj < J; jj++) {
+            for (int jj = 0; jj < T; jj++) {
                 if (j + jj < cnt) {
 #pragma unroll
                     for (int u = 0; u < U; u++) {
-                        if (cidx[u] < N) {
+                        if (in[u]) {
 #pragma unroll
                             for (int v = 0; v < VEC; v++) acc[u][v] = mad<STRICT>(a[jj], b[jj][u][v], acc[u][v]);
                         }

@@ -659,7 +659,6 @@ __device__ __forceinline__ void mma_combine(MmaSmem &sm, const MmaArgs &a, unsig
 template <bool TABLE, bool WIDE>
 __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_constant__ MmaArgs a)
 {
-    grid_dependency_launch();
     extern __shared__ unsigned char smem_raw[];
     MmaSmem &sm = *reinterpret_cast<MmaSmem *>(smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
