@@ -100,6 +100,17 @@ size_t dlspm_spmm_mma_table_bytes(int count);
 long long dlspm_spmm_mma_tables(int count, const dlspm_problem *problems, void *image);
 int dlspm_spmm_mma_launch_tables(dlspm_ctx *ctx, const void *tables, int count, long long tiles, int *error, cudaStream_t st);
 
+// SDDMM of one pattern on the tensor cores (sddmm_mma.cu), and whether it is the faster way: alone, or as one of many
+// problems of a grouped call.
+bool dlspm_sddmm_mma_pays_alone(const dlspm_ctx *ctx, int M, int K, int N, int nnz, int vec);
+void dlspm_sddmm_mma_choose(int count, const dlspm_sddmm_problem *problems, unsigned char *chosen);
+int dlspm_sddmm_mma(dlspm_ctx *ctx, int M, int K, int N, int nnz, const int *row_offsets, const int *cols, const float *mask,
+                    const float *lhs, const float *rhs, float *out, cudaStream_t st);
+// Tables of a launch over `count` problems: their size, and their host image (returns the number of strips).
+size_t dlspm_sddmm_mma_table_bytes(int count);
+long long dlspm_sddmm_mma_tables(int count, const dlspm_sddmm_problem *problems, void *image);
+int dlspm_sddmm_mma_launch_tables(dlspm_ctx *ctx, const void *tables, int count, long long strips, cudaStream_t st);
+
 // Grouped SDDMM / fused launches with caller-provided table memory (sddmm_batch.cu).
 size_t dlspm_rows_batched_table_bytes(int count);
 int dlspm_sddmm_batched_at(dlspm_ctx *ctx, int count, const dlspm_sddmm_problem *problems, void *tables, void *pinned,

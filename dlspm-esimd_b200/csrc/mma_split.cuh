@@ -193,6 +193,25 @@ __device__ __forceinline__ void tmem_load_wait(float (&v)[16])
                  : "memory");
 }
 
+// Adds 64 columns of an accumulator to the warp's registers (those of them below `columns`).
+__device__ __forceinline__ void tmem_add(float (&acc)[64], uint32_t addr, int columns)
+{
+#pragma unroll
+    for (int j = 0; j < 64; j += 16) {
+        if (j < columns) {
+            float v[16];
+            tmem_load16(addr + j, v);
+            tmem_load_wait(v);
+#pragma unroll
+            for (int x = 0; x < 16; x += 2) {
+                const float2 sum = __fadd2_rn(make_float2(acc[j + x], acc[j + x + 1]), make_float2(v[x], v[x + 1]));
+                acc[j + x] = sum.x;
+                acc[j + x + 1] = sum.y;
+            }
+        }
+    }
+}
+
 // Shared-memory operand descriptors.  Swizzled layouts repeat every 8 rows; byte offsets between repetitions:
 // `lead` and `stride` as in the canonical layouts of the PTX manual.
 constexpr uint64_t kSwizzle128 = 2, kSwizzle64 = 4;

@@ -316,10 +316,15 @@ size_t padded256(size_t n) { return (n + 255) & ~(size_t)255; }
 }  // namespace
 
 // Bytes of device memory the tables of a grouped SDDMM / fused launch of `count` problems need.
-size_t dlspm_rows_batched_table_bytes(int count)
+static size_t rows_table_bytes(int count)
 {
     return padded256(sizeof(RowProblem) * (size_t)count) + (size_t)kClasses * 256 +
            padded256(sizeof(long long) * ((size_t)count + kClasses)) + 256 * (size_t)kClasses + 256;
+}
+
+size_t dlspm_rows_batched_table_bytes(int count)
+{
+    return rows_table_bytes(count) + padded256(dlspm_sddmm_mma_table_bytes(count));  // behind them those of the tensor cores
 }
 
 namespace {
@@ -424,18 +429,23 @@ int dlspm_sddmm_batched_at(dlspm_ctx *ctx, int count, const dlspm_sddmm_problem 
                            cudaStream_t st)
 {
     std::vector<HostEntry> by_class[kClasses];
+    std::vector<dlspm_sddmm_problem> dense;  // for the tensor cores
     for (int i = 0; i < count; i++) {
         const dlspm_sddmm_problem &q = problems[i];
         if (q.M < 0 || q.K < 0 || q.N < 0 || q.nnz < 0 || (q.M > 0 && !q.row_offsets) ||
             (q.nnz > 0 && (!q.column_indices || !q.out_values)) || (q.nnz > 0 && q.N > 0 && (!q.lhs || !q.rhs)))
             return DLSPM_ERR_INVALID_ARGUMENT;
     }
+    std::vector<unsigned char> chosen((size_t)count);
+    dlspm_sddmm_mma_choose(count, problems, chosen.data());
     for (int i = 0; i < count; i++) {
         const dlspm_sddmm_problem &q = problems[i];
         if (q.M == 0 || q.nnz == 0) continue;
         int G = 0, R = 0;
         const bool wide = q.N > 0 && dlspm_vec_width(q.N, q.lhs, q.rhs) == 4;
-        if (wide) {
+        if (chosen[(size_t)i]) {
+            dense.push_back(q);
+        } else if (wide) {
             HostEntry e;
             e.p = RowProblem{q.row_offsets, q.column_indices, q.lhs, q.rhs, nullptr, q.mask_values, q.out_values, q.M, q.N / 4, 0};
             e.avg_row = (double)q.nnz / (double)q.M;
@@ -451,6 +461,19 @@ int dlspm_sddmm_batched_at(dlspm_ctx *ctx, int count, const dlspm_sddmm_problem 
                                                 q.lhs, q.rhs, q.out_values, st);
             if (rc) return rc;
         }
+    }
+    if (!dense.empty()) {
+        const size_t at = rows_table_bytes(count), bytes = dlspm_sddmm_mma_table_bytes((int)dense.size());
+        std::vector<unsigned char> local;
+        void *image = pinned ? (char *)pinned + at : nullptr;
+        if (!image) {
+            local.resize(bytes);
+            image = local.data();
+        }
+        const long long strips = dlspm_sddmm_mma_tables((int)dense.size(), dense.data(), image);
+        DLSPM_CUDA_TRY(ctx, cudaMemcpyAsync((char *)tables + at, image, bytes, cudaMemcpyHostToDevice, st));
+        const int rc = dlspm_sddmm_mma_launch_tables(ctx, (char *)tables + at, (int)dense.size(), strips, st);
+        if (rc) return rc;
     }
     choose_sharing(ctx, by_class);
     return rows_batched_at<kOpSddmm>(ctx, by_class, tables, pinned, st);

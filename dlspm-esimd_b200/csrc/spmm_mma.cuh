@@ -532,25 +532,6 @@ __device__ __forceinline__ void mma_mark_not_finite(MmaSmem &sm, int ring, const
             atomicOr(&sm.again[ring][(first + j) >> 5], 1u << ((first + j) & 31));
 }
 
-// Adds 64 columns of an accumulator to the warp's registers (those of them that the tile has).
-__device__ __forceinline__ void mma_add(float (&acc)[kMmaRows], uint32_t addr, int columns)
-{
-#pragma unroll
-    for (int j = 0; j < kMmaRows; j += 16) {
-        if (j < columns) {
-            float v[16];
-            tmem_load16(addr + j, v);
-            tmem_load_wait(v);
-#pragma unroll
-            for (int x = 0; x < 16; x += 2) {
-                const float2 sum = __fadd2_rn(make_float2(acc[j + x], acc[j + x + 1]), make_float2(v[x], v[x + 1]));
-                acc[j + x] = sum.x;
-                acc[j + x + 1] = sum.y;
-            }
-        }
-    }
-}
-
 // Warp w: tensor-memory lanes 32 * (w % 4) .. + 31 (columns of C), accumulator columns 64 * (w / 4) .. + 63
 // (rows of the sparse matrix).
 template <bool TABLE>
@@ -573,8 +554,8 @@ __device__ __forceinline__ bool mma_sums(MmaSmem &sm, const MmaArgs &a, unsigned
         for (int i = 0; i < t.chunks; i++, q++) {
             if (!mbar_wait_suspended(&sm.sum_full[q & 1u], (q >> 1) & 1u, abort)) return false;
             tmem_fence_after();
-            mma_add(acc, tmem + (q & 1u) * 128u, tile_rows - half);
-            if (i + 1 == t.chunks) mma_add(acc, tmem + kMmaSmallColumn + (done & 1u) * 128u, tile_rows - half);
+            tmem_add(acc, tmem + (q & 1u) * 128u, tile_rows - half);
+            if (i + 1 == t.chunks) tmem_add(acc, tmem + kMmaSmallColumn + (done & 1u) * 128u, tile_rows - half);
             tmem_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.sum_empty[q & 1u]);
