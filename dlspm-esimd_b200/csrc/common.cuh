@@ -95,10 +95,14 @@ int dlspm_spmm_mma(dlspm_ctx *ctx, int M, int K, int N, int nnz, const float *va
 
 // Whether the tensor cores are the faster way for one of many problems of a batch.
 bool dlspm_spmm_mma_pays(int M, int K, int N, int nnz);
-// Tables of a launch over `count` problems: their size, and their host image (returns the number of tiles).
+// Tables of a launch over `count` problems: their size, and their host image.
+struct dlspm_mma_parts {
+    int deep, rest;  // problems of the two builds
+    long long deep_tiles, rest_tiles;
+};
 size_t dlspm_spmm_mma_table_bytes(int count);
-long long dlspm_spmm_mma_tables(int count, const dlspm_problem *problems, void *image);
-int dlspm_spmm_mma_launch_tables(dlspm_ctx *ctx, const void *tables, int count, long long tiles, int *error, cudaStream_t st);
+dlspm_mma_parts dlspm_spmm_mma_tables(int count, const dlspm_problem *problems, void *image);
+int dlspm_spmm_mma_launch_tables(dlspm_ctx *ctx, const void *tables, const dlspm_mma_parts &parts, int *error, cudaStream_t st);
 
 // SDDMM of one pattern on the tensor cores (sddmm_mma.cu), and whether it is the faster way: alone, or as one of many
 // problems of a grouped call.

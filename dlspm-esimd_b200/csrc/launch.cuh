@@ -15,6 +15,9 @@ namespace dlspm {
 // Work of the kernels in front in the stream is complete and visible from here on.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The next launch in the stream may be set up from here on (by default: from the end of the block on).
+__device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Launches `kernel` (which begins with grid_dependency_wait); errors are left for cudaGetLastError.
 template <typename... Params, typename... Args>
 inline void launch_overlapped(void (*kernel)(Params...), unsigned blocks, unsigned threads, size_t shared, cudaStream_t st, Args... args)

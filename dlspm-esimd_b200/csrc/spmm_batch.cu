@@ -387,7 +387,7 @@ struct BatchParts {
     long long *ttile_start;        // device, tcount + 1
     // tensor-core kernel
     int mcount;
-    long long mtiles;
+    dlspm_mma_parts mparts;
     void *mtables;                 // device (spmm_mma.cu)
     double stats[4];               // 2*nnz*N and algorithmic bytes: row-gather part, tiled parts
 };
@@ -535,7 +535,7 @@ int build_parts(dlspm_ctx *ctx, const std::vector<BatchProblem> &tab, const std:
     if (err != cudaSuccess) return dlspm_cuda_fail(ctx, err, "batch tables");
     if (!mtab.empty()) {
         std::vector<unsigned char> image(dlspm_spmm_mma_table_bytes(parts.mcount));
-        parts.mtiles = dlspm_spmm_mma_tables(parts.mcount, mtab.data(), image.data());
+        parts.mparts = dlspm_spmm_mma_tables(parts.mcount, mtab.data(), image.data());
         err = upload(&parts.mtables, image.data(), image.size());
         if (err != cudaSuccess) return dlspm_cuda_fail(ctx, err, "batch tables");
     }
@@ -637,7 +637,7 @@ extern "C" int dlspm_batch_launch_part(dlspm_ctx *ctx, const dlspm_batch *batch,
     const BatchParts &p = ctx->strict_fp32 && !batch->same_parts ? batch->strict : batch->usual;
     if (part != 1) {
         if (p.mcount) {
-            rc = dlspm_spmm_mma_launch_tables(ctx, p.mtables, p.mcount, p.mtiles, batch->error, st);
+            rc = dlspm_spmm_mma_launch_tables(ctx, p.mtables, p.mparts, batch->error, st);
             if (rc) return rc;
         }
         rc = tile_launch_tables(ctx, p.tproblems, p.ttile_start, batch->error, p.tcount, p.ttiles, st);

@@ -37,6 +37,7 @@ namespace dlspm {
 
 constexpr int kMmaChunk = 64;   // columns of the sparse matrix per stage, and per main accumulator
 constexpr int kMmaStages = 3;
+constexpr int kMmaDepth = 5;    // entries of a row fetched ahead, in eights, of the usual build at most (the deep one: 8)
 constexpr int kMmaCols = 128;   // columns of C per block, 256 per pair
 constexpr int kMmaRows = 64;    // rows of the sparse matrix per block at most, 128 per pair
 constexpr int kMmaMarkWords = 2 * kMmaRows / 32;
@@ -61,7 +62,7 @@ struct MmaProblem {
     int M, K, N;
     int block_rows;  // rows per tile, a multiple of 16 (half of them per block)
     int row_blocks;  // ceil(M / block_rows)
-    int depth;       // entries of a row fetched ahead, in eights: 1 to 4
+    int depth;       // entries of a row fetched ahead, in eights: 1 to 8
 };
 
 struct MmaSmem {
@@ -85,6 +86,8 @@ struct MmaArgs {
     int splits;  // parts of K, each a pair of its own; more than one only with one tile per cluster
     long long tiles;
     MmaProblem one;  // used when problems is null
+    int before_next;  // the launch behind this one in the stream (with `beside`) may start on SMs as they become free
+    int beside;       // this launch needs nothing of the one in front of it and waits for its end at its own end only
     int *error;
 };
 
@@ -297,6 +300,7 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
         if (!ok) return;
         const uint32_t row = sparse_at + st.stage * (3 * kMmaSparsePlane);
         const uint32_t dst = dense_at + st.stage * (3 * kMmaDensePlane);
+        int turns = 0;  // eights of entries at hand of which some row uses one
         if (row_warp) {
             // this warp's four rows: zeros in all three parts
             const uint32_t z = row + l8 * 16;
@@ -307,8 +311,11 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
             // how many of the entries at hand belong to this chunk (they are the first of them: columns ascend)
             int used = 0;
 #pragma unroll
-            for (int h = 0; h < DEPTH; h++)
-                used += __popc((__ballot_sync(0xffffffffu, (unsigned)(c[h] - k0) < (unsigned)kMmaChunk) >> group) & 0xffu);
+            for (int h = 0; h < DEPTH; h++) {
+                const unsigned m = __ballot_sync(0xffffffffu, (unsigned)(c[h] - k0) < (unsigned)kMmaChunk);
+                used += __popc((m >> group) & 0xffu);
+                if (DEPTH > 5 && m) turns = h + 1;
+            }
             cursor += used;
             bool more = used == 8 * DEPTH;
             while (__any_sync(0xffffffffu, more)) {  // more entries than were fetched ahead: eight at a time
@@ -336,6 +343,7 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
             int last = -1;  // column in front of the first entry at hand (entries of earlier chunks are in order)
 #pragma unroll
             for (int h = 0; h < DEPTH; h++) {
+                if (DEPTH > 5 && h >= turns) break;  // the whole warp
                 const int col = c[h] - k0;
                 const bool live = (unsigned)col < (unsigned)kMmaChunk;
                 if constexpr (CHECK) {
@@ -398,7 +406,7 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
     return true;
 }
 
-template <bool TABLE, bool WIDE>
+template <bool TABLE, bool WIDE, bool DEEP>
 __device__ __forceinline__ bool mma_operands(MmaSmem &sm, const MmaArgs &a, unsigned rank, int warp, int lane)
 {
     MmaTile t;
@@ -409,9 +417,13 @@ __device__ __forceinline__ bool mma_operands(MmaSmem &sm, const MmaArgs &a, unsi
     int ring = 0;
     while (mma_tile_load<TABLE>(t, a, rank)) {
         bool ok;
-        if (t.p->depth == 1) ok = mma_operand_tile<1, !TABLE, WIDE>(sm, a, t, rank, warp, lane, ring, st);
-        else if (t.p->depth == 2) ok = mma_operand_tile<2, !TABLE, WIDE>(sm, a, t, rank, warp, lane, ring, st);
-        else ok = mma_operand_tile<5, !TABLE, WIDE>(sm, a, t, rank, warp, lane, ring, st);
+        if constexpr (DEEP) {
+            ok = mma_operand_tile<8, !TABLE, WIDE>(sm, a, t, rank, warp, lane, ring, st);
+        } else {
+            if (t.p->depth == 1) ok = mma_operand_tile<1, !TABLE, WIDE>(sm, a, t, rank, warp, lane, ring, st);
+            else if (t.p->depth == 2) ok = mma_operand_tile<2, !TABLE, WIDE>(sm, a, t, rank, warp, lane, ring, st);
+            else ok = mma_operand_tile<5, !TABLE, WIDE>(sm, a, t, rank, warp, lane, ring, st);
+        }
         if (!ok) return false;
         ring = (ring + 1) % kMmaRing;
         t.tile += stride;
@@ -636,8 +648,9 @@ __device__ __forceinline__ void mma_combine(MmaSmem &sm, const MmaArgs &a, unsig
 // Grid: clusters of 2 * splits blocks; cluster i takes the tiles i, i + clusters, ...  error[0] is set to 1 if a
 // bounded wait ran out.
 // TABLE: the tiles of a table of problems; otherwise of the one problem among the arguments (whose fields then cost
-// no registers).  WIDE: rows of B are 16-byte aligned.
-template <bool TABLE, bool WIDE>
+// no registers).  WIDE: rows of B are 16-byte aligned.  DEEP: the build for problems with more than 40 entries of a
+// row ahead (in one build with the others its registers cost those 10 to 20 %).
+template <bool TABLE, bool WIDE, bool DEEP>
 __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_constant__ MmaArgs a)
 {
     extern __shared__ unsigned char smem_raw[];
@@ -665,7 +678,8 @@ __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_c
     // (the warps that set the shared memory up also publish it)
     if (warp < kMmaSumWarps) cluster_arrive();
     else cluster_arrive_relaxed();
-    grid_dependency_wait();
+    if (!a.beside) grid_dependency_wait();
+    if (a.before_next) grid_dependency_launch();
     cluster_wait();
     tmem_fence_after();
     bool ok = true;
@@ -674,7 +688,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_c
         ok = mma_sums<TABLE>(sm, a, rank, warp, lane);
     } else if (warp < kIssueWarp) {
         if (kMmaRegsOperand != kMmaRegsLaunch) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kMmaRegsOperand));
-        ok = mma_operands<TABLE, WIDE>(sm, a, rank, warp - kMmaSumWarps, lane);
+        ok = mma_operands<TABLE, WIDE, DEEP>(sm, a, rank, warp - kMmaSumWarps, lane);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kMmaRegsIssue));
         if (warp == kIssueWarp && (rank & 1u) == 0u) {
@@ -702,6 +716,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_c
     cluster_arrive_relaxed();
     cluster_wait();
     if (warp == kIssueWarp) tmem_free<true>(sm.tmem, 512);
+    if (a.beside) grid_dependency_wait();
 }
 
 }  // namespace dlspm
