@@ -88,13 +88,21 @@ size_t dlspm_batched_table_bytes(int count);
 int dlspm_spmm_batched_at(dlspm_ctx *ctx, int count, const dlspm_problem *problems, void *tables, cudaStream_t st,
                           void *pinned = nullptr);
 
+// Reports a bounded wait that ran out in an earlier tensor-core launch of the context.
+static inline int dlspm_mma_check(dlspm_ctx *ctx)
+{
+    if (*(volatile int *)ctx->mma_error == 0) return DLSPM_OK;
+    *(volatile int *)ctx->mma_error = 0;
+    return DLSPM_ERR_TIMEOUT;
+}
+
 // SpMM of one matrix on the tensor cores (spmm_mma.cu), and whether it is the faster way.
 bool dlspm_spmm_mma_pays_alone(const dlspm_ctx *ctx, int M, int K, int N, int nnz, int vec);
 int dlspm_spmm_mma(dlspm_ctx *ctx, int M, int K, int N, int nnz, const float *values, const int *row_offsets, const int *cols,
                    const float *B, float *C, cudaStream_t st);
 
-// Whether the tensor cores are the faster way for one of many problems of a batch.
-bool dlspm_spmm_mma_pays(int M, int K, int N, int nnz);
+// Which problems of a batch the tensor cores are the faster way for.
+void dlspm_spmm_mma_choose(int count, const dlspm_problem *problems, unsigned char *chosen);
 // Tables of a launch over `count` problems: their size, and their host image.
 struct dlspm_mma_parts {
     int deep, rest;  // problems of the two builds
@@ -102,7 +110,17 @@ struct dlspm_mma_parts {
 };
 size_t dlspm_spmm_mma_table_bytes(int count);
 dlspm_mma_parts dlspm_spmm_mma_tables(int count, const dlspm_problem *problems, void *image);
-int dlspm_spmm_mma_launch_tables(dlspm_ctx *ctx, const void *tables, const dlspm_mma_parts &parts, int *error, cudaStream_t st);
+// `sorted`: every row's columns are known to ascend.
+int dlspm_spmm_mma_launch_tables(dlspm_ctx *ctx, const void *tables, const dlspm_mma_parts &parts, bool sorted, int *error,
+                                 cudaStream_t st);
+// The same for a caller that builds its tables entry by entry, those of the deep build first: writes a table entry and
+// returns its tiles; whether a chosen problem's depth is that of the deep build; `starts` as dlspm_spmm_mma_tables lays it
+// out (first tiles and total of the deep part, then of the others).
+constexpr size_t kMmaEntryBytes = 64;
+long long dlspm_spmm_mma_entry(const dlspm_problem &q, void *at);
+bool dlspm_spmm_mma_deep(int depth);
+int dlspm_spmm_mma_launch_at(dlspm_ctx *ctx, const void *tables, const long long *starts, const dlspm_mma_parts &parts, bool sorted,
+                             int *error, cudaStream_t st);
 
 // SDDMM of one pattern on the tensor cores (sddmm_mma.cu), and whether it is the faster way: alone, or as one of many
 // problems of a grouped call.

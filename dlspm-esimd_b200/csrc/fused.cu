@@ -43,7 +43,7 @@ fused_rows_kernel(const int *__restrict__ row_offsets, const int *__restrict__ c
 {
     grid_dependency_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = blockIdx.x * kWarps + warp;
+    const int row = blockIdx.x * (blockDim.x >> 5) + warp;
     if (row >= M) return;
     const int g = lane / G, t = lane % G;
     const float4 *c4 = reinterpret_cast<const float4 *>(c) + (size_t)row * (size_t)chunks;
@@ -383,9 +383,13 @@ void launch_fast(const int *ro, const int *ci, const float *c, const float *b, c
         launch_overlapped(fused_rows_split_kernel<G, R, MODE>, (unsigned)((warps + kWarps - 1) / kWarps), kWarps * 32, smem, st, ro, ci, c, b, d, e, M, chunks, scale, split_shift);
         return;
     }
+    // Launches of a few waves in blocks of four rows: the SMs then differ by less (4096 rows are 3.5 blocks of eight per
+    // SM: 40.9 -> 39.3 us at d = 64; 5353 rows, d = 224: 123 -> 102 us).  Longer launches keep eight, whose rows meet
+    // in L1 (16384 rows, d = 128, with four: 217 -> 222 us).
+    const int warps = (long long)M <= 40LL * kWarps * sm_count / 10 ? 4 : kWarps;
     if constexpr (G == 32 && R == 4) {
         if ((long long)M > 2LL * kWarps * sm_count) {  // more rows than two resident blocks per SM hold
-            launch_overlapped(fused_rows_kernel<G, R, MODE, true>, dlspm_ceil_div(M, kWarps), kWarps * 32, 0, st, ro, ci, c, b, d, e, M, chunks, scale);
+            launch_overlapped(fused_rows_kernel<G, R, MODE, true>, dlspm_ceil_div(M, warps), warps * 32, 0, st, ro, ci, c, b, d, e, M, chunks, scale);
             return;
         }
     }
@@ -394,17 +398,17 @@ void launch_fast(const int *ro, const int *ci, const float *c, const float *b, c
         const long long blocks = dlspm_ceil_div(M, kWarps);
         const long long w6 = (blocks + 6LL * sm_count - 1) / (6LL * sm_count), w8 = (blocks + 8LL * sm_count - 1) / (8LL * sm_count);
         if ((double)w8 * 8.0 * 1.07 < (double)w6 * 6.0) {
-            launch_overlapped(fused_rows_kernel<G, R, MODE, true>, (unsigned)blocks, kWarps * 32, 0, st, ro, ci, c, b, d, e, M, chunks, scale);
+            launch_overlapped(fused_rows_kernel<G, R, MODE, true>, dlspm_ceil_div(M, warps), warps * 32, 0, st, ro, ci, c, b, d, e, M, chunks, scale);
             return;
         }
     }
     if constexpr (G == 4 && R == 2) {
         if (wide) {  // rows of 32 floats, 32-byte aligned operands, a long launch: 256-bit loads
-            launch_overlapped(fused_rows_kernel<G, R, MODE, false, true>, dlspm_ceil_div(M, kWarps), kWarps * 32, 0, st, ro, ci, c, b, d, e, M, chunks, scale);
+            launch_overlapped(fused_rows_kernel<G, R, MODE, false, true>, dlspm_ceil_div(M, warps), warps * 32, 0, st, ro, ci, c, b, d, e, M, chunks, scale);
             return;
         }
     }
-    launch_overlapped(fused_rows_kernel<G, R, MODE>, dlspm_ceil_div(M, kWarps), kWarps * 32, 0, st, ro, ci, c, b, d, e, M, chunks, scale);
+    launch_overlapped(fused_rows_kernel<G, R, MODE>, dlspm_ceil_div(M, warps), warps * 32, 0, st, ro, ci, c, b, d, e, M, chunks, scale);
 }
 
 // Warps per row (as a shift) for a pattern with few rows, by the rule of the SDDMM kernel: share

@@ -83,14 +83,6 @@ PickCost pick_cost(const dlspm_sddmm_problem &q)
 
 size_t pick_starts_offset(int count) { return (sizeof(PickProblem) * (size_t)count + 255) & ~(size_t)255; }
 
-// Reports a bounded wait that ran out in an earlier launch.
-int pick_check(dlspm_ctx *ctx)
-{
-    if (*(volatile int *)ctx->mma_error == 0) return DLSPM_OK;
-    *(volatile int *)ctx->mma_error = 0;
-    return DLSPM_ERR_TIMEOUT;
-}
-
 }  // namespace
 
 // Which problems of a grouped call the tensor cores are faster for, against 7.3 TFLOP/s of the gather kernels; none of
@@ -109,7 +101,7 @@ void dlspm_sddmm_mma_choose(int count, const dlspm_sddmm_problem *problems, unsi
         gather += c.gather_us;
         longest = std::max(longest, c.strip_us);
     }
-    if (all + 0.5 * longest + 10.0 >= 0.8 * gather) std::fill(chosen, chosen + count, (unsigned char)0);
+    if (count > kPickCheckMost || all + 0.5 * longest + 10.0 >= 0.8 * gather) std::fill(chosen, chosen + count, (unsigned char)0);
 }
 
 // A pattern on its own, against 4 us and 8 TFLOP/s (3 without 16-byte loads).  Measured, gather / tensor cores in us:
@@ -126,7 +118,7 @@ bool dlspm_sddmm_mma_pays_alone(const dlspm_ctx *ctx, int M, int K, int N, int n
 int dlspm_sddmm_mma(dlspm_ctx *ctx, int M, int K, int N, int nnz, const int *row_offsets, const int *cols, const float *mask,
                     const float *lhs, const float *rhs, float *out, cudaStream_t st)
 {
-    const int rc = pick_check(ctx);
+    const int rc = dlspm_mma_check(ctx);
     if (rc) return rc;
     PickArgs a = {};
     a.one = PickProblem{row_offsets, cols, lhs, rhs, mask, out, M, K, N, 0, 0, 0};
@@ -165,7 +157,7 @@ long long dlspm_sddmm_mma_tables(int count, const dlspm_sddmm_problem *problems,
 
 int dlspm_sddmm_mma_launch_tables(dlspm_ctx *ctx, const void *tables, int count, long long strips, cudaStream_t st)
 {
-    const int rc = pick_check(ctx);
+    const int rc = dlspm_mma_check(ctx);
     if (rc) return rc;
     PickArgs a = {};
     a.problems = (const PickProblem *)tables;

@@ -37,6 +37,7 @@ static_assert(kPickThreads * kPickRegsLaunch <= 65536 &&
                   32 * (kPickSumWarps * kPickRegsSum + kPickOperandWarps * kPickRegsOperand + kPickWarps * kPickRegsPick + 4 * kPickRegsIssue) <=
                       kPickThreads * kPickRegsLaunch,
               "register budgets exceed what the block is launched with");
+constexpr int kPickCheckMost = 8192;         // problems of a launch at most
 constexpr uint32_t kPickSmallColumn = 256;  // tensor memory: two main accumulators, then two for the small products
 constexpr int kPickRing = 16;               // tiles whose mark (numbers that cannot be split) can be alive at once
 
@@ -63,6 +64,7 @@ struct PickSmem {
     unsigned long long tile_full[2], tile_empty[2];            // halves of `tile` written / read by all pick warps
     unsigned long long drain;                                  // multiplies still running when a wait ran out
     unsigned slow[kPickRing];                                  // the tile holds numbers that cannot be split
+    unsigned unsorted[kPickCheckMost / 32];                    // problems whose columns do not ascend
     uint32_t tmem;
     int abort;
 };
@@ -124,6 +126,17 @@ __device__ __forceinline__ bool pick_strip_load(PickStrip &s, const PickArgs &a,
     s.tiles = max(middle - begin, pick_boundary(*s.p, 2 * pair + 2) - middle);
     s.chunks = (s.p->N + kPickInner - 1) / kPickInner;
     return true;
+}
+
+// The same, past strips of problems that were computed at the start of the kernel.
+template <bool TABLE>
+__device__ __forceinline__ bool pick_strip_next(PickStrip &s, const PickArgs &a, const PickSmem &sm, unsigned rank)
+{
+    while (pick_strip_load<TABLE>(s, a, rank)) {
+        if (!TABLE || !((sm.unsorted[s.prob >> 5] >> (s.prob & 31)) & 1u)) return true;
+        s.at += gridDim.x >> 1;
+    }
+    return false;
 }
 
 struct PickStage {
@@ -212,7 +225,7 @@ __device__ __forceinline__ bool pick_operands(PickSmem &sm, const PickArgs &a, u
     PickStrip s;
     s.at = blockIdx.x >> 1;
     s.prob = 0;
-    bool have = pick_strip_load<TABLE>(s, a, rank);
+    bool have = pick_strip_next<TABLE>(s, a, sm, rank);
     int tile = 0, chunk = 0;
     auto load = [&] {
         const unsigned N = (unsigned)s.p->N;
@@ -238,7 +251,7 @@ __device__ __forceinline__ bool pick_operands(PickSmem &sm, const PickArgs &a, u
             if (++tile == s.tiles) {
                 tile = 0;
                 s.at += gridDim.x >> 1;
-                have = pick_strip_load<TABLE>(s, a, rank);
+                have = pick_strip_next<TABLE>(s, a, sm, rank);
             }
         }
         if (have) load();
@@ -269,7 +282,7 @@ __device__ __forceinline__ bool pick_issue(PickSmem &sm, const PickArgs &a, unsi
     constexpr uint64_t kRhs = kPickRhsPlane >> 4, kLhs = kPickLhsPlane >> 4;
     unsigned g = 0, done = 0;  // chunks (one main accumulator each) and tiles so far
     PickStage st{0, 0u};
-    while (pick_strip_load<TABLE>(s, a, rank)) {
+    while (pick_strip_next<TABLE>(s, a, sm, rank)) {
         const uint32_t instruction = mma_instruction(256, 2 * s.rows, false, false);
         for (int tile = 0; tile < s.tiles; tile++, done++) {
             const uint32_t small = tmem + kPickSmallColumn + (done & 1u) * 128u;
@@ -313,7 +326,7 @@ __device__ __forceinline__ bool pick_relay(PickSmem &sm, const PickArgs &a, unsi
     unsigned long long *own = sums ? sm.sum_empty : sm.full;
     const uint32_t other = cluster_map(smem_u32(own), rank ^ 1u);
     unsigned g = 0;
-    while (pick_strip_load<TABLE>(s, a, rank)) {
+    while (pick_strip_next<TABLE>(s, a, sm, rank)) {
         for (int c = 0; c < s.tiles * s.chunks; c++, g++) {
             if (!mbar_wait_suspended(&own[g % slots], (g / slots) & 1u, abort)) return false;
             mbar_arrive_cluster(other + (g % slots) * 8u);
@@ -337,7 +350,7 @@ __device__ __forceinline__ bool pick_sums(PickSmem &sm, const PickArgs &a, unsig
     const int half = (warp >> 2) * kPickRows, quarter = warp & 3;
     const uint32_t tmem = sm.tmem + ((uint32_t)quarter << 21) + (uint32_t)half;
     unsigned g = 0, done = 0;
-    while (pick_strip_load<TABLE>(s, a, rank)) {
+    while (pick_strip_next<TABLE>(s, a, sm, rank)) {
         const int columns = 2 * s.rows - half;
         for (int tile = 0; tile < s.tiles; tile++, done++) {
             float acc[kPickRows];
@@ -367,13 +380,23 @@ __device__ __forceinline__ bool pick_sums(PickSmem &sm, const PickArgs &a, unsig
 // ---- pick warps -------------------------------------------------------------------------------------------
 
 // Entries q .. of row `row`, as many as are left of four, eight lanes an entry, from the operands.
+template <bool WIDE>
 __device__ __forceinline__ void pick_four(const PickProblem &p, int row, int q, int left, int lane)
 {
     const int e = lane >> 3;
     float sum = 0.f;
     if (e < left) {
         const float *x = p.lhs + (size_t)row * (size_t)p.N, *y = p.rhs + (size_t)__ldg(p.cols + q + e) * (size_t)p.N;
-        for (int k = lane & 7; k < p.N; k += 8) sum = fmaf(__ldg(x + k), __ldg(y + k), sum);
+        if constexpr (WIDE) {
+#pragma unroll 4
+            for (int k = 4 * (lane & 7); k < p.N; k += 32) {
+                const float4 a = __ldg(reinterpret_cast<const float4 *>(x + k)), b = __ldg(reinterpret_cast<const float4 *>(y + k));
+                sum = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, sum))));
+            }
+        } else {
+#pragma unroll 4
+            for (int k = lane & 7; k < p.N; k += 8) sum = fmaf(__ldg(x + k), __ldg(y + k), sum);
+        }
     }
 #pragma unroll
     for (int d = 4; d >= 1; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
@@ -417,7 +440,7 @@ __device__ __forceinline__ void pick_fetch(int *to, const int *__restrict__ cols
 // Rows warp, warp + 8, .. of the strip; lane r (< 16) holds the cursor of the warp's r-th row and the end of its
 // part.  Of every row 32 entries are at hand in shared memory, fetched one tile ahead (a lane reads only what it
 // fetched itself).
-template <bool TABLE>
+template <bool TABLE, bool WIDE>
 __device__ __forceinline__ bool pick_entries(PickSmem &sm, const PickArgs &a, unsigned rank, int warp, int lane)
 {
     constexpr int kRows = 2 * kPickRows / kPickWarps, kTurn = kRows / 2;
@@ -427,7 +450,7 @@ __device__ __forceinline__ bool pick_entries(PickSmem &sm, const PickArgs &a, un
     s.at = blockIdx.x >> 1;
     s.prob = 0;
     unsigned done = 0;
-    while (pick_strip_load<TABLE>(s, a, rank)) {
+    while (pick_strip_next<TABLE>(s, a, sm, rank)) {
         const PickProblem &p = *s.p;
         int cursor = 0, end = 0;
         {
@@ -489,7 +512,7 @@ __device__ __forceinline__ bool pick_entries(PickSmem &sm, const PickArgs &a, un
                             const unsigned d = (unsigned)(ahead[r][lane] - j0);
                             const int count = __clz(__brev(__ballot_sync(0xffffffffu, d >= (unsigned)kPickCols)));
                             __syncwarp();
-                            for (int e = 0; e < count; e += 4) pick_four(p, s.row0 + warp + kPickWarps * r, at + e, count - e, lane);
+                            for (int e = 0; e < count; e += 4) pick_four<WIDE>(p, s.row0 + warp + kPickWarps * r, at + e, count - e, lane);
                         }
                     }
                     __syncwarp();
@@ -509,12 +532,40 @@ __device__ __forceinline__ bool pick_entries(PickSmem &sm, const PickArgs &a, un
         for (int r = 0; r < kRows; r++) {
             const int stop = __shfl_sync(0xffffffffu, end, r);
             for (int q = __shfl_sync(0xffffffffu, cursor, r); q < stop; q += 4)
-                pick_four(p, s.row0 + warp + kPickWarps * r, q, stop - q, lane);
+                pick_four<WIDE>(p, s.row0 + warp + kPickWarps * r, q, stop - q, lane);
         }
         s.at += gridDim.x >> 1;
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     return true;
+}
+
+// ---- columns out of order ---------------------------------------------------------------------------------------
+
+// Looks at eight entries each of 32 rows.  Entries out of order that this does not find are computed one by one; a pattern
+// whose rows are out of order as a rule would take ten times as long that way as with the loop below.
+__device__ __forceinline__ bool pick_looks_sorted(const PickProblem &p, int lane)
+{
+    const int row = (int)((long long)p.M * lane / 32);
+    const int start = __ldg(p.row_offsets + row), end = __ldg(p.row_offsets + row + 1);
+    const int from = start + (end - start) / 2;
+    int c[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) c[i] = from + i < end ? __ldg(p.cols + from + i) : 0x7fffffff;
+    bool ok = true;
+#pragma unroll
+    for (int i = 1; i < 8; i++) ok = ok && (c[i] > c[i - 1] || from + i >= end);
+    return __all_sync(0xffffffffu, ok);
+}
+
+// A whole problem entry by entry, by all warps of the launch.
+template <bool WIDE>
+__device__ __forceinline__ void pick_all(const PickProblem &p, int warp, int lane)
+{
+    for (int row = (int)blockIdx.x * (kPickThreads / 32) + warp; row < p.M; row += (int)gridDim.x * (kPickThreads / 32)) {
+        const int end = __ldg(p.row_offsets + row + 1);
+        for (int q = __ldg(p.row_offsets + row); q < end; q += 4) pick_four<WIDE>(p, row, q, end - q, lane);
+    }
 }
 
 // Grid: pairs of blocks; pair i takes the strips i, i + pairs, ...  error[0] is set to 1 if a bounded wait ran out.
@@ -553,8 +604,22 @@ __global__ void __launch_bounds__(kPickThreads, 1) sddmm_mma_kernel(const __grid
     grid_dependency_wait();
     cluster_wait();
     tmem_fence_after();
-    bool ok = true;
-    if (warp < kPickSumWarps) {
+    bool ok = true, done = false;
+    if constexpr (TABLE) {
+        for (int i = threadIdx.x; i < (a.count + 31) / 32; i += kPickThreads) sm.unsorted[i] = 0u;
+        __syncthreads();
+        for (int i = warp; i < a.count; i += kPickThreads / 32)
+            if (!pick_looks_sorted(a.problems[i], lane) && lane == 0) atomicOr(&sm.unsorted[i >> 5], 1u << (i & 31));
+        __syncthreads();
+        for (int w = 0; w < (a.count + 31) / 32; w++)
+            for (unsigned m = sm.unsorted[w]; m; m &= m - 1u) pick_all<WIDE>(a.problems[32 * w + __ffs(m) - 1], warp, lane);
+    } else {
+        done = !pick_looks_sorted(a.one, lane);
+        if (done) pick_all<WIDE>(a.one, warp, lane);
+    }
+    if (done) {
+        // nothing left to do
+    } else if (warp < kPickSumWarps) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPickRegsSum));
         ok = pick_sums<TABLE>(sm, a, rank, warp, lane);
     } else if (warp < kFirstPick) {
@@ -562,7 +627,7 @@ __global__ void __launch_bounds__(kPickThreads, 1) sddmm_mma_kernel(const __grid
         ok = pick_operands<TABLE, WIDE>(sm, a, rank, warp - kPickSumWarps, lane);
     } else if (warp < kIssueWarp) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPickRegsPick));
-        ok = pick_entries<TABLE>(sm, a, rank, warp - kFirstPick, lane);
+        ok = pick_entries<TABLE, WIDE>(sm, a, rank, warp - kFirstPick, lane);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPickRegsIssue));
         if (warp == kIssueWarp && (rank & 1u) == 0u) {

@@ -464,14 +464,25 @@ bool prefer_tiled(const dlspm_ctx *ctx, const dlspm_problem &q, int vec, bool so
     return density * 1000.0 >= (double)ctx->tile_min_density_permille && q.M >= 16 && q.N >= 64;
 }
 
-// Whether the automatic choice takes the tensor-core kernel for a problem.  The caller's density threshold, where one
+// Whether the automatic choice may take the tensor-core kernel for a problem.  The caller's density threshold, where one
 // is set, decides for the tiled kernels as a whole.
-bool prefer_mma(const dlspm_ctx *ctx, const dlspm_problem &q, int vec, bool sorted)
+bool mma_eligible(const dlspm_ctx *ctx, const dlspm_problem &q, int vec)
 {
-    if (ctx->spmm_kernel != 0 || vec != 4 || !sorted || q.nnz == 0) return false;
-    if (ctx->tile_min_density_set)
-        return (double)q.nnz / ((double)q.M * (double)q.K) * 1000.0 >= (double)ctx->tile_min_density_permille && q.M >= 16 && q.N >= 64;
-    return dlspm_spmm_mma_pays(q.M, q.K, q.N, q.nnz);
+    if (ctx->spmm_kernel != 0 || vec != 4 || q.nnz == 0) return false;
+    return !ctx->tile_min_density_set ||
+           ((double)q.nnz / ((double)q.M * (double)q.K) * 1000.0 >= (double)ctx->tile_min_density_permille && q.M >= 16 && q.N >= 64);
+}
+
+// The problems of a one-shot grouped launch that go to the tensor cores (chosen[i]: depth, or 0).  Strict mode keeps the
+// order of additions of the row-gather kernel.
+void choose_one_shot(const dlspm_ctx *ctx, int count, const dlspm_problem *problems, unsigned char *chosen)
+{
+    for (int i = 0; i < count; i++) {
+        const dlspm_problem &q = problems[i];
+        chosen[i] = !ctx->strict_fp32 && !ctx->tile_min_density_set && q.M > 0 && q.N > 0 &&
+                    mma_eligible(ctx, q, dlspm_vec_width(q.N, q.B, q.C));
+    }
+    dlspm_spmm_mma_choose(count, problems, chosen);
 }
 
 cudaError_t upload(void **dst, const void *src, size_t bytes)
@@ -490,13 +501,21 @@ int build_parts(dlspm_ctx *ctx, const std::vector<BatchProblem> &tab, const std:
     std::vector<long long> tstarts;
     std::vector<dlspm_problem> mtab;
     memset(&parts, 0, sizeof(parts));
+    std::vector<dlspm_problem> all;
+    std::vector<unsigned char> chosen(tab.size());
     for (size_t i = 0; i < tab.size(); i++) {
         const BatchProblem &t = tab[i];
-        const dlspm_problem q{t.M, t.K, t.N, t.nnz, t.values, t.row_offsets, t.cols, t.B, t.C};
+        all.push_back(dlspm_problem{t.M, t.K, t.N, t.nnz, t.values, t.row_offsets, t.cols, t.B, t.C});
+        chosen[i] = tensor && (flags[i] & 1) && mma_eligible(ctx, all[i], t.vec);
+    }
+    if (!ctx->tile_min_density_set) dlspm_spmm_mma_choose((int)all.size(), all.data(), chosen.data());
+    for (size_t i = 0; i < tab.size(); i++) {
+        const BatchProblem &t = tab[i];
+        const dlspm_problem &q = all[i];
         const double fl = 2.0 * (double)t.nnz * t.N;
         const double by = 4.0 * (t.M + 1) + 8.0 * t.nnz + 4.0 * (double)t.K * t.N + 4.0 * (double)t.M * t.N;
         const bool sorted = (flags[i] & 1) != 0;
-        const bool mma = tensor && prefer_mma(ctx, q, t.vec, sorted);
+        const bool mma = chosen[i] != 0;
         const bool tiled = !mma && prefer_tiled(ctx, q, t.vec, sorted);
         parts.stats[mma || tiled ? 2 : 0] += fl;
         parts.stats[mma || tiled ? 3 : 1] += by;
@@ -637,7 +656,7 @@ extern "C" int dlspm_batch_launch_part(dlspm_ctx *ctx, const dlspm_batch *batch,
     const BatchParts &p = ctx->strict_fp32 && !batch->same_parts ? batch->strict : batch->usual;
     if (part != 1) {
         if (p.mcount) {
-            rc = dlspm_spmm_mma_launch_tables(ctx, p.mtables, p.mparts, batch->error, st);
+            rc = dlspm_spmm_mma_launch_tables(ctx, p.mtables, p.mparts, true, batch->error, st);
             if (rc) return rc;
         }
         rc = tile_launch_tables(ctx, p.tproblems, p.ttile_start, batch->error, p.tcount, p.ttiles, st);
@@ -690,7 +709,7 @@ size_t dlspm_batched_table_bytes(int count)
 {
     const size_t tab = (sizeof(BatchProblem) * (size_t)count + 255) & ~(size_t)255;
     const size_t st = (sizeof(long long) * ((size_t)count + 2) + 255) & ~(size_t)255;
-    return tab + st + 256;
+    return tab + st + 256 + ((dlspm_spmm_mma_table_bytes(count) + 255) & ~(size_t)255);  // those of the tensor cores last
 }
 
 // One-shot grouped launch with its tables placed at `tables` (device memory of at least
@@ -701,7 +720,32 @@ int dlspm_spmm_batched_at(dlspm_ctx *ctx, int count, const dlspm_problem *proble
     std::vector<BatchProblem> tab;
     std::vector<long long> starts;
     GatherSplit split;
-    int rc = build_tables(ctx, count, problems, tab, starts, split);
+    for (int i = 0; i < count; i++) {
+        const dlspm_problem &q = problems[i];
+        const int bad = check_spmm_args(q.M, q.K, q.N, q.nnz, q.values, q.row_offsets, q.column_indices, q.B, q.C);
+        if (bad) return bad;
+    }
+    std::vector<unsigned char> chosen((size_t)count);
+    choose_one_shot(ctx, count, problems, chosen.data());
+    std::vector<dlspm_problem> dense, others;
+    for (int i = 0; i < count; i++) (chosen[(size_t)i] ? dense : others).push_back(problems[i]);
+    if (!dense.empty()) {
+        int rc = dlspm_mma_check(ctx);
+        if (rc) return rc;
+        const size_t at = dlspm_batched_table_bytes(count) - ((dlspm_spmm_mma_table_bytes(count) + 255) & ~(size_t)255);
+        const size_t bytes = dlspm_spmm_mma_table_bytes((int)dense.size());
+        std::vector<unsigned char> local;
+        void *image = pinned ? (char *)pinned + at : nullptr;
+        if (!image) {
+            local.resize(bytes);
+            image = local.data();
+        }
+        const dlspm_mma_parts parts = dlspm_spmm_mma_tables((int)dense.size(), dense.data(), image);
+        DLSPM_CUDA_TRY(ctx, cudaMemcpyAsync((char *)tables + at, image, bytes, cudaMemcpyHostToDevice, st));
+        rc = dlspm_spmm_mma_launch_tables(ctx, (char *)tables + at, parts, false, ctx->mma_error, st);
+        if (rc) return rc;
+    }
+    int rc = build_tables(ctx, (int)others.size(), others.data(), tab, starts, split);
     if (rc) return rc;
     if (tab.empty()) return DLSPM_OK;
     const size_t tab_bytes = sizeof(BatchProblem) * tab.size();
@@ -755,11 +799,12 @@ namespace {
 constexpr int kStaticMaxProblems = 1024;
 constexpr size_t kStaticTableBytes = sizeof(BatchProblem) * kStaticMaxProblems;
 constexpr size_t kStaticStartsOff = (kStaticTableBytes + 255) & ~(size_t)255;
-constexpr size_t kStaticStartsBytes = sizeof(long long) * (kStaticMaxProblems + 1);
+constexpr size_t kStaticStartsBytes = sizeof(long long) * (kStaticMaxProblems + 3);  // tile indexes of the two kernels
 constexpr size_t kStaticCounterOff = (kStaticStartsOff + kStaticStartsBytes + 255) & ~(size_t)255;
 constexpr size_t kStaticScratchBytes = kStaticCounterOff + 256;
 // the size quoted in the header and the documentation
 static_assert(sizeof(BatchProblem) == 80 && kStaticScratchBytes == 90624, "update the documented size of the static scratch");
+static_assert(kMmaEntryBytes <= sizeof(BatchProblem), "entries of either kernel fit the table");
 
 // Problem table, tile index and work counter of dlspm_spmm_batched_f32_static.  In host code this
 // name is only a handle for cudaGetSymbolAddress, never an address a kernel can use.
@@ -790,8 +835,8 @@ constexpr int kStaticChunk = 32;  // table entries built on the stack and copied
 
 }  // namespace
 
-// Host memory: none from the heap, and about 5 KiB of stack (a 2 KiB order array of 16-bit indices
-// and one chunk of kStaticChunk table entries), so the call also fits the small stacks of plug-in
+// Host memory: none from the heap, and about 6 KiB of stack (a 2 KiB order array of 16-bit indices,
+// a 1 KiB array of choices and one chunk of kStaticChunk table entries), so the call also fits the small stacks of plug-in
 // and real-time threads.  The table is sent in chunks; every cudaMemcpyAsync here has a pageable
 // source of a few KiB, which the runtime copies out before it returns, so the chunk buffer can be
 // reused at once.  Because of these copies the call cannot be recorded into a CUDA graph: on a
@@ -815,8 +860,10 @@ extern "C" int dlspm_spmm_batched_f32_static(dlspm_ctx *ctx, int count, const dl
     rc = static_scratch_address(ctx, &base);
     if (rc) return rc;
 
-    // Same order as the allocating entry point: decreasing nnz*N, the lower index first on ties.
+    // Same order as the allocating entry point: the problems of the row-gather kernel by decreasing nnz*N, the lower
+    // index first on ties; behind them those of the tensor cores, the deep ones first, by decreasing K.
     unsigned short order[kStaticMaxProblems];
+    unsigned char chosen[kStaticMaxProblems];
     int used = 0;
     for (int i = 0; i < count; i++) {
         const dlspm_problem &q = problems[i];
@@ -825,10 +872,18 @@ extern "C" int dlspm_spmm_batched_f32_static(dlspm_ctx *ctx, int count, const dl
         if (q.M > 0 && q.N > 0) order[used++] = (unsigned short)i;
     }
     if (used == 0) return DLSPM_OK;
+    choose_one_shot(ctx, count, problems, chosen);
     std::sort(order, order + used, [&](unsigned short x, unsigned short y) {
+        if (!chosen[x] != !chosen[y]) return !chosen[x];
+        if (chosen[x]) {
+            const bool dx = dlspm_spmm_mma_deep(chosen[x]), dy = dlspm_spmm_mma_deep(chosen[y]);
+            return dx != dy ? dx : problems[x].K != problems[y].K ? problems[x].K > problems[y].K : x < y;
+        }
         const double wx = (double)problems[x].nnz * problems[x].N, wy = (double)problems[y].nnz * problems[y].N;
         return wx != wy ? wx > wy : x < y;
     });
+    int gather = 0;
+    while (gather < used && !chosen[order[gather]]) gather++;
 
     BatchProblem *d_tab = (BatchProblem *)base;
     long long *d_starts = (long long *)(base + kStaticStartsOff);
@@ -838,18 +893,54 @@ extern "C" int dlspm_spmm_batched_f32_static(dlspm_ctx *ctx, int count, const dl
     BatchProblem tab[kStaticChunk];
     long long starts[kStaticChunk + 1];
     long long run = 0;
-    for (int s0 = 0; s0 < used; s0 += kStaticChunk) {
-        const int n = std::min(kStaticChunk, used - s0);
+    for (int s0 = 0; s0 < gather; s0 += kStaticChunk) {
+        const int n = std::min(kStaticChunk, gather - s0);
         for (int s = 0; s < n; s++) {
             tab[s] = make_batch_problem(problems[order[s0 + s]], false);
             starts[s] = run;
             run += (long long)tab[s].row_groups * dlspm_ceil_div(tab[s].N, 32 * tab[s].vec * tab[s].chunks);
         }
-        const bool last = s0 + n == used;
+        const bool last = s0 + n == gather;
         if (last) starts[n] = run;
         DLSPM_CUDA_TRY(ctx, cudaMemcpyAsync(d_tab + s0, tab, sizeof(BatchProblem) * (size_t)n, cudaMemcpyHostToDevice, st));
         DLSPM_CUDA_TRY(ctx, cudaMemcpyAsync(d_starts + s0, starts, sizeof(long long) * (size_t)(n + (last ? 1 : 0)),
                                             cudaMemcpyHostToDevice, st));
     }
-    return batch_launch_tables(ctx, d_tab, d_starts, d_counter, GatherSplit{used, 0, run, 0}, st);
+    if (gather < used) {
+        rc = dlspm_mma_check(ctx);
+        if (rc) return rc;
+        unsigned char *d_mma = base + sizeof(BatchProblem) * (size_t)gather;
+        long long *d_index = d_starts + gather + 1;
+        dlspm_mma_parts parts = {0, 0, 0, 0};
+        unsigned char *entries = (unsigned char *)tab;
+        int sent = 0;  // tile index entries sent
+        for (int s0 = gather; s0 < used;) {
+            // a chunk of one part: its entries and first tiles, and the part's total with its last chunk
+            const bool deep = dlspm_spmm_mma_deep(chosen[order[s0]]);
+            long long &tiles = deep ? parts.deep_tiles : parts.rest_tiles;
+            int n = 0;
+            while (n < kStaticChunk && s0 + n < used && dlspm_spmm_mma_deep(chosen[order[s0 + n]]) == deep) {
+                starts[n] = tiles;
+                tiles += dlspm_spmm_mma_entry(problems[order[s0 + n]], entries + kMmaEntryBytes * (size_t)n);
+                n++;
+            }
+            (deep ? parts.deep : parts.rest) += n;
+            starts[n] = tiles;
+            const bool end = s0 + n == used || dlspm_spmm_mma_deep(chosen[order[s0 + n]]) != deep;
+            if (s0 == gather && !deep) {  // no deep part: its total, 0, in front
+                const long long none = 0;
+                DLSPM_CUDA_TRY(ctx, cudaMemcpyAsync(d_index, &none, sizeof(none), cudaMemcpyHostToDevice, st));
+                sent = 1;
+            }
+            DLSPM_CUDA_TRY(ctx, cudaMemcpyAsync(d_mma + kMmaEntryBytes * (size_t)(s0 - gather), entries, kMmaEntryBytes * (size_t)n,
+                                                cudaMemcpyHostToDevice, st));
+            DLSPM_CUDA_TRY(ctx, cudaMemcpyAsync(d_index + sent, starts, sizeof(long long) * (size_t)(n + (end ? 1 : 0)),
+                                                cudaMemcpyHostToDevice, st));
+            sent += n + (end ? 1 : 0);
+            s0 += n;
+        }
+        rc = dlspm_spmm_mma_launch_at(ctx, d_mma, d_index, parts, false, ctx->mma_error, st);
+        if (rc) return rc;
+    }
+    return batch_launch_tables(ctx, d_tab, d_starts, d_counter, GatherSplit{gather, 0, run, 0}, st);
 }

@@ -9,10 +9,10 @@ using namespace dlspm;
 
 namespace {
 
-template <bool TABLE, bool WIDE, bool DEEP>
+template <bool TABLE, bool WIDE, bool DEEP, bool CHECK>
 int mma_launch(dlspm_ctx *ctx, const MmaArgs &a, int clusters, cudaStream_t st)
 {
-    auto kernel = spmm_mma_kernel<TABLE, WIDE, DEEP>;
+    auto kernel = spmm_mma_kernel<TABLE, WIDE, DEEP, CHECK>;
     DLSPM_CUDA_TRY(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMmaSmemBytes));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(clusters * 2 * a.splits));
@@ -71,17 +71,31 @@ int mma_splits(const dlspm_ctx *ctx, long long tiles, int K)
 
 }  // namespace
 
-// One of many problems of a batch: a pair of blocks needs 1.5 us per chunk of 64 columns, more with more entries to
-// scatter, and 3 us per tile; the row-gather kernel 9 to 12 TFLOP/s.  Measured on batches of one shape with N = 3136,
-// row-gather / tensor cores in TFLOP/s: 1024 x 4096 at 50 % nonzeros 11 / 44, at 10 % 9.3 / 17, at 5 % equal;
-// 2048 x 512 at 50 % 13.5 / 45, at 10 % 11.4 / 13.1; 256 x 256 at 20 % 9.2 / 13.7, at 10 % equal.
-bool dlspm_spmm_mma_pays(int M, int K, int N, int nnz)
+// Which problems of a batch the tensor cores are faster for: chosen[i], not 0 on entry where problem i may go there, becomes
+// its depth or 0.  A pair of blocks needs 1.5 us per chunk of 64 columns, more with more entries to scatter, and 3 us per
+// tile; the row-gather kernel 9 to 12 TFLOP/s.  Measured on batches of one shape with N = 3136, row-gather / tensor cores
+// in TFLOP/s: 1024 x 4096 at 50 % nonzeros 11 / 54, at 10 % 9.3 / 17, at 5 % equal; 2048 x 512 at 50 % 13.5 / 48, at 10 %
+// 11.4 / 12.5; 256 x 256 at 20 % 10.8 / 16.7, at 10 % equal.  A batch whose tiles are too few for the 74 pairs of blocks
+// takes as long as its longest tile: then none is chosen.
+void dlspm_spmm_mma_choose(int count, const dlspm_problem *problems, unsigned char *chosen)
 {
-    if (!mma_fits(K, N, nnz)) return false;
-    const double density = (double)nnz / ((double)M * K);
-    const double tiles = (double)dlspm_ceil_div(M, 2 * kMmaRows) * dlspm_ceil_div(N, 2 * kMmaCols);
-    const double mma_us = tiles * (dlspm_ceil_div(K, kMmaChunk) * (1.5 + 3.2 * density) + 3.0) / 74.0;
-    return mma_us < 2.0 * nnz * N / 11e6;
+    double all = 0.0, longest = 0.0, gather = 0.0;
+    for (int i = 0; i < count; i++) {
+        if (!chosen[i]) continue;
+        chosen[i] = 0;
+        const dlspm_problem &q = problems[i];
+        if (q.nnz == 0 || q.M <= 0 || q.N <= 0 || q.K <= 0 || !mma_fits(q.K, q.N, q.nnz)) continue;
+        const double density = (double)q.nnz / ((double)q.M * q.K);
+        const double tiles = (double)dlspm_ceil_div(q.M, 2 * kMmaRows) * dlspm_ceil_div(q.N, 2 * kMmaCols);
+        const double tile_us = dlspm_ceil_div(q.K, kMmaChunk) * (1.5 + 2.4 * density) + 3.0;
+        const double gather_us = 2.0 * q.nnz * q.N / 11e6;
+        if (tiles * tile_us / 74.0 >= gather_us) continue;
+        chosen[i] = (unsigned char)mma_problem(q).depth;
+        all += tiles * tile_us / 74.0;
+        longest = std::max(longest, tile_us);
+        gather += gather_us;
+    }
+    if (count > kMmaCheckMost || std::max(all, longest) + 0.3 * longest + 8.0 >= 0.9 * gather) std::fill(chosen, chosen + count, (unsigned char)0);
 }
 
 // A matrix on its own: launch and first chunk 8.5 us, then 1.25 us per chunk and round of tiles; the row-gather
@@ -101,6 +115,17 @@ bool dlspm_spmm_mma_pays_alone(const dlspm_ctx *ctx, int M, int K, int N, int nn
 }
 
 size_t dlspm_spmm_mma_table_bytes(int count) { return mma_starts_offset(count) + sizeof(long long) * ((size_t)count + 2); }
+
+static_assert(sizeof(MmaProblem) == kMmaEntryBytes, "size of a table entry in common.cuh");
+
+long long dlspm_spmm_mma_entry(const dlspm_problem &q, void *at)
+{
+    const MmaProblem p = mma_problem(q);
+    memcpy(at, &p, sizeof(p));
+    return mma_tiles(p);
+}
+
+bool dlspm_spmm_mma_deep(int depth) { return depth > kMmaDepth; }
 
 dlspm_mma_parts dlspm_spmm_mma_tables(int count, const dlspm_problem *problems, void *image)
 {
@@ -128,10 +153,16 @@ dlspm_mma_parts dlspm_spmm_mma_tables(int count, const dlspm_problem *problems, 
     return parts;
 }
 
-int dlspm_spmm_mma_launch_tables(dlspm_ctx *ctx, const void *tables, const dlspm_mma_parts &parts, int *error, cudaStream_t st)
+int dlspm_spmm_mma_launch_tables(dlspm_ctx *ctx, const void *tables, const dlspm_mma_parts &parts, bool sorted, int *error,
+                                 cudaStream_t st)
 {
     const int count = parts.deep + parts.rest;
-    const long long *starts = (const long long *)((const char *)tables + mma_starts_offset(count));
+    return dlspm_spmm_mma_launch_at(ctx, tables, (const long long *)((const char *)tables + mma_starts_offset(count)), parts, sorted, error, st);
+}
+
+int dlspm_spmm_mma_launch_at(dlspm_ctx *ctx, const void *tables, const long long *starts, const dlspm_mma_parts &parts, bool sorted,
+                             int *error, cudaStream_t st)
+{
     MmaArgs a = {};
     a.splits = 1;
     a.error = error;
@@ -141,7 +172,8 @@ int dlspm_spmm_mma_launch_tables(dlspm_ctx *ctx, const void *tables, const dlspm
         a.count = parts.deep;
         a.tiles = parts.deep_tiles;
         a.before_next = parts.rest ? 1 : 0;
-        const int rc = mma_launch<true, true, true>(ctx, a, (int)std::min<long long>(a.tiles, ctx->sm_count / 2), st);
+        const int clusters = (int)std::min<long long>(a.tiles, ctx->sm_count / 2);
+        const int rc = sorted ? mma_launch<true, true, true, false>(ctx, a, clusters, st) : mma_launch<true, true, true, true>(ctx, a, clusters, st);
         if (rc) return rc;
     }
     if (parts.rest) {
@@ -151,7 +183,8 @@ int dlspm_spmm_mma_launch_tables(dlspm_ctx *ctx, const void *tables, const dlspm
         a.tiles = parts.rest_tiles;
         a.before_next = 0;
         a.beside = parts.deep ? 1 : 0;
-        return mma_launch<true, true, false>(ctx, a, (int)std::min<long long>(a.tiles, ctx->sm_count / 2), st);
+        const int clusters = (int)std::min<long long>(a.tiles, ctx->sm_count / 2);
+        return sorted ? mma_launch<true, true, false, false>(ctx, a, clusters, st) : mma_launch<true, true, false, true>(ctx, a, clusters, st);
     }
     return DLSPM_OK;
 }
@@ -159,10 +192,8 @@ int dlspm_spmm_mma_launch_tables(dlspm_ctx *ctx, const void *tables, const dlspm
 int dlspm_spmm_mma(dlspm_ctx *ctx, int M, int K, int N, int nnz, const float *values, const int *row_offsets, const int *cols,
                    const float *B, float *C, cudaStream_t st)
 {
-    if (*(volatile int *)ctx->mma_error) {  // of an earlier launch
-        *(volatile int *)ctx->mma_error = 0;
-        return DLSPM_ERR_TIMEOUT;
-    }
+    const int rc = dlspm_mma_check(ctx);
+    if (rc) return rc;
     MmaArgs a = {};
     a.one = mma_problem(dlspm_problem{M, K, N, nnz, values, row_offsets, cols, B, C});
     a.tiles = mma_tiles(a.one);
@@ -170,6 +201,6 @@ int dlspm_spmm_mma(dlspm_ctx *ctx, int M, int K, int N, int nnz, const float *va
     a.splits = mma_splits(ctx, a.tiles, K);
     const int clusters = a.splits > 1 ? (int)a.tiles : (int)std::min<long long>(a.tiles, ctx->sm_count / 2);
     const bool wide = dlspm_vec_width(N, B, B) == 4, deep = a.one.depth > kMmaDepth;
-    if (wide) return deep ? mma_launch<false, true, true>(ctx, a, clusters, st) : mma_launch<false, true, false>(ctx, a, clusters, st);
-    return deep ? mma_launch<false, false, true>(ctx, a, clusters, st) : mma_launch<false, false, false>(ctx, a, clusters, st);
+    if (wide) return deep ? mma_launch<false, true, true, true>(ctx, a, clusters, st) : mma_launch<false, true, false, true>(ctx, a, clusters, st);
+    return deep ? mma_launch<false, false, true, true>(ctx, a, clusters, st) : mma_launch<false, false, false, true>(ctx, a, clusters, st);
 }

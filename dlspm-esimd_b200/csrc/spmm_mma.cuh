@@ -45,6 +45,7 @@ constexpr int kMmaSumWarps = 8, kMmaOperandWarps = 16;
 constexpr int kMmaThreads = (kMmaSumWarps + kMmaOperandWarps + 4) * 32;
 constexpr int kMmaDensePlane = kMmaChunk * kMmaCols * 2;   // bytes of one part of one operand in a stage
 constexpr int kMmaSparsePlane = kMmaChunk * kMmaRows * 2;
+constexpr int kMmaCheckMost = 8192;  // problems of a launch whose columns may be out of order
 constexpr uint32_t kMmaSmallColumn = 256;  // tensor memory: two main accumulators, then two for the small products
 constexpr int kMmaRing = 16;    // tiles whose marks (rows to compute again) can be alive at once
 constexpr int kMmaRegsLaunch = 72, kMmaRegsSum = 88, kMmaRegsOperand = 72, kMmaRegsIssue = 40;
@@ -72,6 +73,7 @@ struct MmaSmem {
     unsigned long long sum_full[2], sum_empty[2];            // accumulators complete / added by all sum warps
     unsigned long long drain;                                // multiplies still running when a wait ran out
     unsigned again[kMmaRing][kMmaMarkWords];                  // rows of the tile to compute again
+    unsigned unsorted[kMmaCheckMost / 32];                   // problems whose columns do not ascend (see mma_looks_sorted)
     uint32_t tmem;
     int abort;
 };
@@ -141,6 +143,17 @@ __device__ __forceinline__ bool mma_tile_load(MmaTile &t, const MmaArgs &a, unsi
     t.chunk0 = (int)((long long)all * part / a.splits);
     t.chunks = (int)((long long)all * (part + 1) / a.splits) - t.chunk0;
     return true;
+}
+
+// The same, past tiles of problems that were computed at the start of the kernel.
+template <bool TABLE, bool CHECK>
+__device__ __forceinline__ bool mma_tile_next(MmaTile &t, const MmaArgs &a, const MmaSmem &sm, unsigned rank)
+{
+    while (mma_tile_load<TABLE>(t, a, rank)) {
+        if (!(TABLE && CHECK) || !((sm.unsorted[t.prob >> 5] >> (t.prob & 31)) & 1u)) return true;
+        t.tile += gridDim.x / (2u * (unsigned)a.splits);
+    }
+    return false;
 }
 
 // First entry of the row at or behind column `col`.
@@ -250,8 +263,8 @@ __device__ __forceinline__ void mma_mark_again(MmaSmem &sm, int ring, int bit, u
 }
 
 // One tile: every lane group of eight lanes owns one row of it, 4 * warp + group, and walks it once.  DEPTH: entries
-// of a row fetched ahead, in eights.  CHECK: columns may be out of order (with a table they were looked at when it
-// was made).
+// of a row fetched ahead, in eights.  CHECK: columns may be out of order (a prepared batch looked at them when it was
+// made).
 template <int DEPTH, bool CHECK, bool WIDE>
 __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, const MmaTile &t, unsigned rank, int warp, int lane,
                                                  int ring, MmaStage &st)
@@ -406,7 +419,7 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
     return true;
 }
 
-template <bool TABLE, bool WIDE, bool DEEP>
+template <bool TABLE, bool WIDE, bool DEEP, bool CHECK>
 __device__ __forceinline__ bool mma_operands(MmaSmem &sm, const MmaArgs &a, unsigned rank, int warp, int lane)
 {
     MmaTile t;
@@ -415,14 +428,14 @@ __device__ __forceinline__ bool mma_operands(MmaSmem &sm, const MmaArgs &a, unsi
     const unsigned stride = gridDim.x / (2u * (unsigned)a.splits);
     MmaStage st{0, 0u};
     int ring = 0;
-    while (mma_tile_load<TABLE>(t, a, rank)) {
+    while (mma_tile_next<TABLE, CHECK>(t, a, sm, rank)) {
         bool ok;
         if constexpr (DEEP) {
-            ok = mma_operand_tile<8, !TABLE, WIDE>(sm, a, t, rank, warp, lane, ring, st);
+            ok = mma_operand_tile<8, CHECK, WIDE>(sm, a, t, rank, warp, lane, ring, st);
         } else {
-            if (t.p->depth == 1) ok = mma_operand_tile<1, !TABLE, WIDE>(sm, a, t, rank, warp, lane, ring, st);
-            else if (t.p->depth == 2) ok = mma_operand_tile<2, !TABLE, WIDE>(sm, a, t, rank, warp, lane, ring, st);
-            else ok = mma_operand_tile<5, !TABLE, WIDE>(sm, a, t, rank, warp, lane, ring, st);
+            if (t.p->depth == 1) ok = mma_operand_tile<1, CHECK, WIDE>(sm, a, t, rank, warp, lane, ring, st);
+            else if (t.p->depth == 2) ok = mma_operand_tile<2, CHECK, WIDE>(sm, a, t, rank, warp, lane, ring, st);
+            else ok = mma_operand_tile<5, CHECK, WIDE>(sm, a, t, rank, warp, lane, ring, st);
         }
         if (!ok) return false;
         ring = (ring + 1) % kMmaRing;
@@ -435,7 +448,7 @@ __device__ __forceinline__ bool mma_operands(MmaSmem &sm, const MmaArgs &a, unsi
 
 // The whole warp walks the chunks, one lane issues (the instructions take their operands from uniform registers,
 // which the compiler can only use where control flow is uniform).
-template <bool TABLE>
+template <bool TABLE, bool CHECK>
 __device__ __forceinline__ bool mma_issue(MmaSmem &sm, const MmaArgs &a, unsigned rank, bool issuer)
 {
     volatile int *abort = &sm.abort;
@@ -451,7 +464,7 @@ __device__ __forceinline__ bool mma_issue(MmaSmem &sm, const MmaArgs &a, unsigne
     const uint64_t sparse0 = mma_descriptor(smem_u32(&sm.sparse[0][0][0]), 0, 1024, kSwizzle128);
     constexpr uint64_t kDense = kMmaDensePlane >> 4, kSparse = kMmaSparsePlane >> 4;
     unsigned g = 0, done = 0;  // chunks (one main accumulator each) and tiles so far
-    while (mma_tile_load<TABLE>(t, a, rank)) {
+    while (mma_tile_next<TABLE, CHECK>(t, a, sm, rank)) {
         const uint32_t instruction = mma_instruction(256, 2 * t.rows, true, false);
         const uint32_t small = tmem + kMmaSmallColumn + (done & 1u) * 128u;
         for (int c = 0; c < t.chunks; c++, g++) {
@@ -486,7 +499,7 @@ __device__ __forceinline__ bool mma_issue(MmaSmem &sm, const MmaArgs &a, unsigne
 
 // Passes the odd block's barriers on to the even block's, one arrival per phase: a remote arrival orders all
 // memory accesses of its thread first, which would hold up a warp with loads in flight.
-template <bool TABLE>
+template <bool TABLE, bool CHECK>
 __device__ __forceinline__ bool mma_relay(MmaSmem &sm, const MmaArgs &a, unsigned rank, bool sums)
 {
     volatile int *abort = &sm.abort;
@@ -498,7 +511,7 @@ __device__ __forceinline__ bool mma_relay(MmaSmem &sm, const MmaArgs &a, unsigne
     unsigned long long *own = sums ? sm.sum_empty : sm.full;
     const uint32_t other = cluster_map(smem_u32(own), rank ^ 1u);
     unsigned g = 0;
-    while (mma_tile_load<TABLE>(t, a, rank)) {
+    while (mma_tile_next<TABLE, CHECK>(t, a, sm, rank)) {
         for (int c = 0; c < t.chunks; c++, g++) {
             if (!mbar_wait_suspended(&own[g % slots], (g / slots) & 1u, abort)) return false;
             mbar_arrive_cluster(other + (g % slots) * 8u);
@@ -546,7 +559,7 @@ __device__ __forceinline__ void mma_mark_not_finite(MmaSmem &sm, int ring, const
 
 // Warp w: tensor-memory lanes 32 * (w % 4) .. + 31 (columns of C), accumulator columns 64 * (w / 4) .. + 63
 // (rows of the sparse matrix).
-template <bool TABLE>
+template <bool TABLE, bool CHECK>
 __device__ __forceinline__ bool mma_sums(MmaSmem &sm, const MmaArgs &a, unsigned rank, int warp, int lane)
 {
     volatile int *abort = &sm.abort;
@@ -558,7 +571,7 @@ __device__ __forceinline__ bool mma_sums(MmaSmem &sm, const MmaArgs &a, unsigned
     const uint32_t tmem = sm.tmem + ((uint32_t)quarter << 21) + (uint32_t)half;
     unsigned q = 0, done = 0;
     int ring = 0;
-    while (mma_tile_load<TABLE>(t, a, rank)) {
+    while (mma_tile_next<TABLE, CHECK>(t, a, sm, rank)) {
         const int tile_rows = 2 * t.rows;
         float acc[kMmaRows];
 #pragma unroll
@@ -645,12 +658,44 @@ __device__ __forceinline__ void mma_combine(MmaSmem &sm, const MmaArgs &a, unsig
     }
 }
 
+// ---- columns out of order ---------------------------------------------------------------------------------------
+
+// Looks at eight entries each of 32 rows.  Rows out of order that this does not find are computed again one by one; a
+// pattern whose rows are out of order as a rule (as some formats leave them) would take ten times as long that way as
+// with the row-gather loop, which the kernel then runs instead.
+__device__ __forceinline__ bool mma_looks_sorted(const MmaProblem &p, int lane)
+{
+    const int row = (int)((long long)p.M * lane / 32);
+    const int start = __ldg(p.row_offsets + row), end = __ldg(p.row_offsets + row + 1);
+    const int from = start + (end - start) / 2;
+    int c[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) c[i] = from + i < end ? __ldg(p.cols + from + i) : 0x7fffffff;
+    bool ok = true;
+#pragma unroll
+    for (int i = 1; i < 8; i++) ok = ok && (c[i] > c[i - 1] || from + i >= end);
+    return __all_sync(0xffffffffu, ok);
+}
+
+// A whole problem with the row-gather loop, by all warps of the launch.
+template <int VEC>
+__device__ __forceinline__ void mma_gather(const MmaProblem &p, int2 *stage, int warp, int lane)
+{
+    constexpr int kCols = 32 * VEC;
+    const long long items = (long long)p.M * ((p.N + kCols - 1) / kCols);
+    for (long long i = (long long)blockIdx.x * (kMmaThreads / 32) + warp; i < items; i += (long long)gridDim.x * (kMmaThreads / 32)) {
+        const int slab = (int)(i / p.M), row = (int)(i - (long long)slab * p.M);
+        spmm_warp_row_slab<VEC, 1, false, 4>(p.values, p.cols, __ldg(p.row_offsets + row), __ldg(p.row_offsets + row + 1), p.B,
+                                             p.C + (size_t)row * (size_t)p.N, p.N, slab * kCols, lane, stage);
+    }
+}
+
 // Grid: clusters of 2 * splits blocks; cluster i takes the tiles i, i + clusters, ...  error[0] is set to 1 if a
 // bounded wait ran out.
 // TABLE: the tiles of a table of problems; otherwise of the one problem among the arguments (whose fields then cost
 // no registers).  WIDE: rows of B are 16-byte aligned.  DEEP: the build for problems with more than 40 entries of a
-// row ahead (in one build with the others its registers cost those 10 to 20 %).
-template <bool TABLE, bool WIDE, bool DEEP>
+// row ahead (in one build with the others its registers cost those 10 to 20 %).  CHECK: columns may be out of order.
+template <bool TABLE, bool WIDE, bool DEEP, bool CHECK>
 __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_constant__ MmaArgs a)
 {
     extern __shared__ unsigned char smem_raw[];
@@ -682,31 +727,49 @@ __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_c
     if (a.before_next) grid_dependency_launch();
     cluster_wait();
     tmem_fence_after();
-    bool ok = true;
-    if (warp < kMmaSumWarps) {
+    bool ok = true, done = false;
+    if constexpr (CHECK) {
+        int2 *stage = reinterpret_cast<int2 *>(&sm.dense[0][0][0]) + warp * 32;
+        if constexpr (TABLE) {
+            for (int i = threadIdx.x; i < (a.count + 31) / 32; i += kMmaThreads) sm.unsorted[i] = 0u;
+            __syncthreads();
+            for (int i = warp; i < a.count; i += kMmaThreads / 32)
+                if (!mma_looks_sorted(a.problems[i], lane) && lane == 0) atomicOr(&sm.unsorted[i >> 5], 1u << (i & 31));
+            __syncthreads();
+            for (int w = 0; w < (a.count + 31) / 32; w++)
+                for (unsigned m = sm.unsorted[w]; m; m &= m - 1u) mma_gather<WIDE ? 4 : 1>(a.problems[32 * w + __ffs(m) - 1], stage, warp, lane);
+            __syncthreads();
+        } else {
+            done = !mma_looks_sorted(a.one, lane);
+            if (done) mma_gather<WIDE ? 4 : 1>(a.one, stage, warp, lane);
+        }
+    }
+    if (done) {
+        // nothing left to do
+    } else if (warp < kMmaSumWarps) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kMmaRegsSum));
-        ok = mma_sums<TABLE>(sm, a, rank, warp, lane);
+        ok = mma_sums<TABLE, CHECK>(sm, a, rank, warp, lane);
     } else if (warp < kIssueWarp) {
         if (kMmaRegsOperand != kMmaRegsLaunch) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kMmaRegsOperand));
-        ok = mma_operands<TABLE, WIDE, DEEP>(sm, a, rank, warp - kMmaSumWarps, lane);
+        ok = mma_operands<TABLE, WIDE, DEEP, CHECK>(sm, a, rank, warp - kMmaSumWarps, lane);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kMmaRegsIssue));
         if (warp == kIssueWarp && (rank & 1u) == 0u) {
             const bool issuer = elect_one();
-            ok = mma_issue<TABLE>(sm, a, rank, issuer);
+            ok = mma_issue<TABLE, CHECK>(sm, a, rank, issuer);
             if (!ok && issuer) {  // multiplies in flight get a bounded chance to end before the tensor memory is freed
                 mma_commit<true>(&sm.drain, 1u << rank);
                 (void)mbar_wait(&sm.drain, 0u);
             }
         }
-        if (warp <= kIssueWarp + 1 && (rank & 1u) && lane == 0) ok = mma_relay<TABLE>(sm, a, rank, warp != kIssueWarp);
+        if (warp <= kIssueWarp + 1 && (rank & 1u) && lane == 0) ok = mma_relay<TABLE, CHECK>(sm, a, rank, warp != kIssueWarp);
     }
     if (!ok) {
         *(volatile int *)&sm.abort = 1;
         *(volatile int *)a.error = 1;
     }
     __syncwarp();
-    if (a.splits > 1) {
+    if (a.splits > 1 && !done) {
         cluster_arrive();
         cluster_wait();
         if (warp < kMmaSumWarps && *(volatile int *)&sm.abort == 0) mma_combine<TABLE>(sm, a, rank, warp, lane);

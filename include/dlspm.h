@@ -200,7 +200,7 @@ int dlspm_spmm_batched_f32(dlspm_ctx *ctx, int count, const dlspm_problem *probl
  * counterpart in the reference.  It never calls cudaMalloc/cudaFree or any allocating routine: its
  * problem table, tile index and work counter live in a fixed __device__ array inside the library
  * (90 624 bytes = 88.5 KiB per GPU, held until the process exits).  Limit: count <= 1024 problems,
- * otherwise DLSPM_ERR_UNSUPPORTED.  Host side: no heap either, and about 5 KiB of stack (the table is
+ * otherwise DLSPM_ERR_UNSUPPORTED.  Host side: no heap either, and about 6 KiB of stack (the table is
  * built and sent in chunks of 32 problems), so it fits the small stacks of plug-in threads.  The
  * first call on a device looks up the array's device address; make that call before any stream
  * capture starts in the process.  Like the allocating one-shot call it copies its table from host
