@@ -85,8 +85,10 @@ int dlspm_stage_reserve(dlspm_ctx *ctx, size_t bytes);
 size_t dlspm_batched_table_bytes(int count);
 // `pinned` (optional, host memory of the same size): the tables are built there and copied
 // asynchronously; the caller must not reuse it before the launch has finished.
+// `given` (optional): which problems go to the tensor cores, from dlspm_spmm_choose_staged.
 int dlspm_spmm_batched_at(dlspm_ctx *ctx, int count, const dlspm_problem *problems, void *tables, cudaStream_t st,
-                          void *pinned = nullptr);
+                          void *pinned = nullptr, const unsigned char *given = nullptr);
+void dlspm_spmm_choose_staged(dlspm_ctx *ctx, int count, const dlspm_problem *problems, unsigned char *chosen);
 
 // Reports a bounded wait that ran out in an earlier tensor-core launch of the context.
 static inline int dlspm_mma_check(dlspm_ctx *ctx)
@@ -99,7 +101,7 @@ static inline int dlspm_mma_check(dlspm_ctx *ctx)
 // SpMM of one matrix on the tensor cores (spmm_mma.cu), and whether it is the faster way.
 bool dlspm_spmm_mma_pays_alone(const dlspm_ctx *ctx, int M, int K, int N, int nnz, int vec);
 int dlspm_spmm_mma(dlspm_ctx *ctx, int M, int K, int N, int nnz, const float *values, const int *row_offsets, const int *cols,
-                   const float *B, float *C, cudaStream_t st);
+                   const float *B, float *C, bool sorted, cudaStream_t st);  // sorted: columns are known to ascend
 
 // Which problems of a batch the tensor cores are the faster way for.
 void dlspm_spmm_mma_choose(int count, const dlspm_problem *problems, unsigned char *chosen);

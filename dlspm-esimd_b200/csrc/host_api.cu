@@ -281,6 +281,8 @@ static int dlspm_spmm_batched_f32_host_impl(dlspm_ctx *ctx, int count, const dls
         total += need(q);
     }
     if (count == 0) return DLSPM_OK;
+    std::vector<unsigned char> chosen((size_t)count);
+    dlspm_spmm_choose_staged(ctx, count, problems, chosen.data());
     rc = pipeline_init(ctx);
     if (rc) return rc;
     // Pieces: consecutive problems up to a budget (a single larger problem is its own piece).  Nothing
@@ -364,7 +366,7 @@ static int dlspm_spmm_batched_f32_host_impl(dlspm_ctx *ctx, int count, const dls
         DLSPM_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_h2d[b], h2d));
         DLSPM_CUDA_TRY(ctx, cudaStreamWaitEvent(run, ctx->ev_h2d[b], 0));
         rc = dlspm_spmm_batched_at(ctx, (int)dev[b].size(), dev[b].data(), base, run,
-                                   (char *)ctx->pinned + (size_t)b * padded(max_tables));
+                                   (char *)ctx->pinned + (size_t)b * padded(max_tables), chosen.data() + first);
         if (rc) return rc;
         DLSPM_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_kernel[b], run));
         DLSPM_CUDA_TRY(ctx, cudaStreamWaitEvent(d2h, ctx->ev_kernel[b], 0));

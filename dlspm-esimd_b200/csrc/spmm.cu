@@ -289,16 +289,16 @@ int spmm_row_split(const dlspm_ctx *ctx, int M, int N, int nnz, int vec, bool st
 }
 
 
-// max_row_len: longest row if known (from a plan), else 0.
+// Known from a plan: max_row_len, the longest row (else 0), and whether all rows are sorted (else -1).
 int spmm_launch(dlspm_ctx *ctx, int M, int K, int N, int nnz, const float *values, const int *row_offsets,
-                const int *cols, const float *B, float *C, const int *row_order, int max_row_len, cudaStream_t st)
+                const int *cols, const float *B, float *C, const int *row_order, int max_row_len, int sorted, cudaStream_t st)
 {
     if (M == 0 || N == 0) return DLSPM_OK;
     SpmmArgs a{values, row_offsets, cols, B, C, row_order, M, N, dlspm_ceil_div(M, kWarpsPerCta), 1, ctx->sm_count};
     const int vec = dlspm_vec_width(N, B, C);
     const bool strict = ctx->strict_fp32 != 0;
-    if (!strict && dlspm_spmm_mma_pays_alone(ctx, M, K, N, nnz, vec))
-        return dlspm_spmm_mma(ctx, M, K, N, nnz, values, row_offsets, cols, B, C, st);
+    if (!strict && sorted != 0 && dlspm_spmm_mma_pays_alone(ctx, M, K, N, nnz, vec))
+        return dlspm_spmm_mma(ctx, M, K, N, nnz, values, row_offsets, cols, B, C, sorted > 0, st);
     int split = spmm_row_split(ctx, M, N, nnz, vec, strict);
     // Long rows of uneven length (known only with a plan): eight warps per row make every thread
     // block finish its row together, which the binning by powers of two does not.  Measured on
@@ -355,7 +355,7 @@ extern "C" int dlspm_spmm_csr_f32(dlspm_ctx *ctx, int M, int K, int N, int nnz, 
     if (rc) return rc;
     rc = dlspm_check_input(ctx, M, K, nnz, row_offsets, column_indices, (cudaStream_t)stream);
     if (rc) return rc;
-    return spmm_launch(ctx, M, K, N, nnz, values, row_offsets, column_indices, B, C, nullptr, 0,
+    return spmm_launch(ctx, M, K, N, nnz, values, row_offsets, column_indices, B, C, nullptr, 0, -1,
                        (cudaStream_t)stream);
 }
 
@@ -372,7 +372,7 @@ extern "C" int dlspm_spmm_csr_f32_planned(dlspm_ctx *ctx, const dlspm_plan *plan
     rc = dlspm_check_input(ctx, plan->M, plan->K, plan->nnz, row_offsets, column_indices, (cudaStream_t)stream);
     if (rc) return rc;
     return spmm_launch(ctx, plan->M, plan->K, N, plan->nnz, values, row_offsets, column_indices, B, C, plan->row_order,
-                       plan->max_row_len, (cudaStream_t)stream);
+                       plan->max_row_len, plan->sorted_rows, (cudaStream_t)stream);
 }
 
 // ---- SpMM whose result rows go to several destinations (fused compute + gather) -----------------

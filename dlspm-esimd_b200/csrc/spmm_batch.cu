@@ -712,10 +712,22 @@ size_t dlspm_batched_table_bytes(int count)
     return tab + st + 256 + ((dlspm_spmm_mma_table_bytes(count) + 255) & ~(size_t)255);  // those of the tensor cores last
 }
 
+// The choice for a batch of host buffers, whose device copies are all aligned: made for the batch as a whole, so that the
+// results do not depend on how it is cut into pieces.
+void dlspm_spmm_choose_staged(dlspm_ctx *ctx, int count, const dlspm_problem *problems, unsigned char *chosen)
+{
+    std::vector<dlspm_problem> staged(problems, problems + count);
+    for (dlspm_problem &q : staged) {
+        q.B = nullptr;
+        q.C = nullptr;
+    }
+    choose_one_shot(ctx, count, staged.data(), chosen);
+}
+
 // One-shot grouped launch with its tables placed at `tables` (device memory of at least
 // dlspm_batched_table_bytes(count) bytes, owned by the caller until the launch has finished).
 int dlspm_spmm_batched_at(dlspm_ctx *ctx, int count, const dlspm_problem *problems, void *tables, cudaStream_t st,
-                          void *pinned)
+                          void *pinned, const unsigned char *given)
 {
     std::vector<BatchProblem> tab;
     std::vector<long long> starts;
@@ -726,7 +738,8 @@ int dlspm_spmm_batched_at(dlspm_ctx *ctx, int count, const dlspm_problem *proble
         if (bad) return bad;
     }
     std::vector<unsigned char> chosen((size_t)count);
-    choose_one_shot(ctx, count, problems, chosen.data());
+    if (given) std::copy(given, given + count, chosen.begin());
+    else choose_one_shot(ctx, count, problems, chosen.data());
     std::vector<dlspm_problem> dense, others;
     for (int i = 0; i < count; i++) (chosen[(size_t)i] ? dense : others).push_back(problems[i]);
     if (!dense.empty()) {

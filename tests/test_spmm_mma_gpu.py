@@ -33,11 +33,18 @@ def batch_run(pkg, ctx, dev, M, K, N, ro, ci, vals, B):
     return out[guard:guard + M * N].reshape(M, N)
 
 
-def lone_run(ctx, dev, M, K, N, ro, ci, vals, B):
+def lone_run(ctx, dev, M, K, N, ro, ci, vals, B, plan=False):
     import torch
 
     out = torch.full((M, N), float("nan"), device=dev)
-    ctx.spmm(M, K, N, int(ci.size), to_dev(vals, dev), to_dev(ro, dev), to_dev(ci, dev), to_dev(B, dev), out)
+    d = [to_dev(x, dev) for x in (vals, ro, ci, B)]
+    if plan:
+        p = ctx.plan_create(M, K, int(ci.size), d[1], d[2])
+        ctx.spmm_planned(p, N, *d, out)
+        torch.cuda.synchronize()
+        p.close()
+    else:
+        ctx.spmm(M, K, N, int(ci.size), *d, out)
     torch.cuda.synchronize()
     return out.cpu().numpy()
 
@@ -88,6 +95,7 @@ def test_lone_launches(pkg, oracle, ctx, dev, M, K, N, density, order):
     vals = pkg.gen_dense_host(int(ci.size), seed, 2)
     B = dense(pkg, K, N, seed, 10)
     check(oracle, ro, ci, vals, B, M, N, lone_run(ctx, dev, M, K, N, ro, ci, vals, B))
+    check(oracle, ro, ci, vals, B, M, N, lone_run(ctx, dev, M, K, N, ro, ci, vals, B, plan=True))
 
 
 @pytest.mark.parametrize("where", ["infinite", "tiny", "huge"])
