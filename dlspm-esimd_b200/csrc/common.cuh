@@ -103,6 +103,8 @@ bool dlspm_spmm_mma_pays_alone(const dlspm_ctx *ctx, int M, int K, int N, int nn
 int dlspm_spmm_mma(dlspm_ctx *ctx, int M, int K, int N, int nnz, const float *values, const int *row_offsets, const int *cols,
                    const float *B, float *C, bool sorted, cudaStream_t st);  // sorted: columns are known to ascend
 
+// Whether the kernel's 32-bit offsets reach all of a problem.
+bool dlspm_spmm_mma_fits(int K, int N, int nnz);
 // Which problems of a batch the tensor cores are the faster way for.
 void dlspm_spmm_mma_choose(int count, const dlspm_problem *problems, unsigned char *chosen);
 // Tables of a launch over `count` problems: their size, and their host image.

@@ -55,12 +55,6 @@ long long mma_tiles(const MmaProblem &p) { return (long long)p.row_blocks * dlsp
 
 size_t mma_starts_offset(int count) { return (sizeof(MmaProblem) * (size_t)count + 255) & ~(size_t)255; }
 
-// Byte offsets into B and into the CSR arrays are 32-bit in the kernel (and run up to two chunks past the end).
-bool mma_fits(int K, int N, int nnz)
-{
-    return ((double)K + 4 * kMmaChunk) * N < 1e9 && nnz < 1000000000;
-}
-
 // Parts of K for a launch of `tiles` tiles: as long as every part gets a pair of blocks of its own and eight chunks.
 int mma_splits(const dlspm_ctx *ctx, long long tiles, int K)
 {
@@ -70,6 +64,12 @@ int mma_splits(const dlspm_ctx *ctx, long long tiles, int K)
 }
 
 }  // namespace
+
+// Byte offsets into B and into the CSR arrays are 32-bit in the kernel (and run up to two chunks past the end).
+bool dlspm_spmm_mma_fits(int K, int N, int nnz)
+{
+    return ((double)K + 4 * kMmaChunk) * N < 1e9 && nnz < 1000000000;
+}
 
 // Which problems of a batch the tensor cores are faster for: chosen[i], not 0 on entry where problem i may go there, becomes
 // its depth or 0.  A pair of blocks needs 1.5 us per chunk of 64 columns, more with more entries to scatter, and 3 us per
@@ -84,7 +84,7 @@ void dlspm_spmm_mma_choose(int count, const dlspm_problem *problems, unsigned ch
         if (!chosen[i]) continue;
         chosen[i] = 0;
         const dlspm_problem &q = problems[i];
-        if (q.nnz == 0 || q.M <= 0 || q.N <= 0 || q.K <= 0 || !mma_fits(q.K, q.N, q.nnz)) continue;
+        if (q.nnz == 0 || q.M <= 0 || q.N <= 0 || q.K <= 0 || !dlspm_spmm_mma_fits(q.K, q.N, q.nnz)) continue;
         const double density = (double)q.nnz / ((double)q.M * q.K);
         const double tiles = (double)dlspm_ceil_div(q.M, 2 * kMmaRows) * dlspm_ceil_div(q.N, 2 * kMmaCols);
         const double tile_us = dlspm_ceil_div(q.K, kMmaChunk) * (1.5 + 2.4 * density) + 3.0;
@@ -104,7 +104,7 @@ void dlspm_spmm_mma_choose(int count, const dlspm_problem *problems, unsigned ch
 // 50 %, N = 3136 1012 / 243; 512 x 2048 at 30 %, N = 256 equal; 256 x 512, N = 256 7.3 / 18.
 bool dlspm_spmm_mma_pays_alone(const dlspm_ctx *ctx, int M, int K, int N, int nnz, int vec)
 {
-    if (nnz == 0 || N < 32 || !mma_fits(K, N, nnz)) return false;
+    if (nnz == 0 || N < 32 || !dlspm_spmm_mma_fits(K, N, nnz)) return false;
     const double density = (double)nnz / ((double)M * K);
     const long long tiles = (long long)dlspm_ceil_div(M, 2 * kMmaRows) * dlspm_ceil_div(N, 2 * kMmaCols);
     const int splits = mma_splits(ctx, tiles, K);

@@ -127,3 +127,34 @@ def test_numbers_that_cannot_be_split(pkg, oracle, ctx, dev, where):
         B[7, 3] = np.float32(3.4e38)  # rounds to infinity as bf16
         vals *= np.float32(1e-3)
     check(oracle, ro, ci, vals, B, M, N, batch_run(pkg, ctx, dev, M, K, N, ro, ci, vals, B))
+
+
+def test_problems_beyond_32_bit_offsets_stay_on_other_kernels(pkg, ctx, dev):
+    """B of 2^30 elements and more, with a density threshold of the caller's (which takes the place of the estimate):
+    the byte offsets of such a B do not fit the tensor-core kernel."""
+    import torch
+
+    M, K, N, per_row = 64, (1 << 21) + 64, 512, 60
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(5)
+    ci = torch.randint(0, K // per_row, (M, per_row), generator=gen, device=dev, dtype=torch.int32)
+    ci += torch.arange(per_row, device=dev, dtype=torch.int32) * (K // per_row)  # ascending, over the whole range
+    ci[:, -1] = K - 1 - torch.arange(M, device=dev, dtype=torch.int32)           # the last rows of B among them
+    ro = torch.arange(0, M * per_row + 1, per_row, dtype=torch.int32, device=dev)
+    vals = torch.rand(M * per_row, generator=gen, device=dev) - 0.5
+    B = torch.rand(K, N, generator=gen, device=dev) - 0.5
+    C = torch.full((M, N), float("nan"), device=dev)
+    arr = pkg.ProblemArray(1)
+    arr.set(0, M, K, N, M * per_row, vals, ro, ci.reshape(-1), B, C)
+    ctx.set_option(pkg.OPT_TILE_MIN_DENSITY, 0)
+    try:
+        batch = ctx.batch_create(arr)
+        batch.launch()
+        torch.cuda.synchronize()
+        assert batch.info(check_device=True)[2] == 0
+        batch.close()
+    finally:
+        ctx.set_option(pkg.OPT_TILE_MIN_DENSITY, -1)
+    v, rows = vals.reshape(M, per_row, 1).double(), B[ci.long()].double()
+    want, scale = (v * rows).sum(1), (v * rows).abs().sum(1)
+    assert ((C.double() - want).abs() <= TOL * scale).all()
