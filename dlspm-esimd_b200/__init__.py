@@ -142,6 +142,7 @@ _SIGNATURES = {
     "dlspm_measure_fp32_peaks": (_I, [_P, C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "dlspm_host_copy_count": (_I, [_P, C.POINTER(C.c_longlong)]),
     "dlspm_sanity_check_csr": (_I, [_P, _I, _I, _I, _P, _P, C.c_char_p, C.c_size_t, _P]),
+    "dlspm_device_error": (_I, [_P, C.POINTER(_I)]),
     "dlspm_selftest_bounded_wait": (_I, [_P, C.c_uint, C.POINTER(_I)]),
     "dlspm_spmm_csr_f32_scatter": (_I, [_P, _I, _I, _I, _I, _P, _P, _P, _P, _I, C.POINTER(_P), C.c_longlong, _P]),
     "dlspm_enable_peer_access": (_I, [_P, _I]),
@@ -485,6 +486,12 @@ class Context:
 
     def peer_free(self, ptr: int) -> None:
         _check(self.lib.dlspm_peer_free(self.handle, ptr), "dlspm_peer_free", self)
+
+    def device_error(self) -> int:
+        """1 if a kernel of this context (prepared batches aside) gave up a bounded wait since the last look."""
+        e = _I()
+        _check(self.lib.dlspm_device_error(self.handle, C.byref(e)), "dlspm_device_error", self)
+        return e.value
 
     def selftest_bounded_wait(self, polls: int = 1000):
         """(status, timed_out) of the bounded-wait self-test; the context stays usable afterwards."""

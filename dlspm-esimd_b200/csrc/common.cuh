@@ -90,7 +90,8 @@ int dlspm_spmm_batched_at(dlspm_ctx *ctx, int count, const dlspm_problem *proble
                           void *pinned = nullptr, const unsigned char *given = nullptr);
 void dlspm_spmm_choose_staged(dlspm_ctx *ctx, int count, const dlspm_problem *problems, unsigned char *chosen);
 
-// Reports a bounded wait that ran out in an earlier tensor-core launch of the context.
+// Reports, once, a bounded wait that ran out in a tensor-core launch of the context that was not a prepared batch's: before
+// the next such launch, before and after a host-buffer call (host_api.cu), or through dlspm_device_error.
 static inline int dlspm_mma_check(dlspm_ctx *ctx)
 {
     if (*(volatile int *)ctx->mma_error == 0) return DLSPM_OK;

@@ -352,6 +352,16 @@ extern "C" int dlspm_peer_free(dlspm_ctx *ctx, void *ptr)
     return DLSPM_OK;
 }
 
+extern "C" int dlspm_device_error(dlspm_ctx *ctx, int *device_error)
+{
+    if (!ctx || !device_error) return DLSPM_ERR_INVALID_ARGUMENT;
+    int rc = dlspm_use(ctx);
+    if (rc) return rc;
+    DLSPM_CUDA_TRY(ctx, cudaDeviceSynchronize());
+    *device_error = dlspm_mma_check(ctx) != DLSPM_OK;
+    return DLSPM_OK;
+}
+
 // ---- bounded-wait self-test --------------------------------------------------------------------
 // Every wait inside a kernel of this library is a bounded poll that ends in a status, never a trap
 // or an endless loop.  This entry point shows that path without any fault: one thread polls an

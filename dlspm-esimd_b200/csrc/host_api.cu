@@ -25,13 +25,21 @@ struct Carver {
 
 inline size_t padded(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
 
-// A host-buffer call that fails half-way may still have copies and kernels in flight that read the
-// staging memory or write the caller's buffers.  Every such call therefore leaves through here: on
-// an error the streams it used are drained before the error is reported, so that when the call
+// Every host-buffer call runs through here.
+// A call that fails half-way may still have copies and kernels in flight that read the staging memory or write the
+// caller's buffers: on an error the streams it used are drained before the error is reported, so that when the call
 // returns nothing of it is running any more.
-int drain_on_error(dlspm_ctx *ctx, int rc)
+// A kernel whose bounded wait ran out has left its result incomplete; the body has synchronised by the time it returns,
+// so the word says whether one of its own kernels did.  A word that is set on entry belongs to an earlier call, and is
+// reported before anything runs.
+template <typename Body>
+int host_call(dlspm_ctx *ctx, Body body)
 {
-    if (rc == DLSPM_OK || !ctx) return rc;
+    if (!ctx) return body();
+    int rc = dlspm_mma_check(ctx);
+    if (rc) return rc;
+    rc = body();
+    if (rc == DLSPM_OK) return dlspm_mma_check(ctx);
     if (cudaSetDevice(ctx->device) == cudaSuccess) {
         if (ctx->stream) (void)cudaStreamSynchronize(ctx->stream);
         if (ctx->pipeline_ready) {
@@ -40,6 +48,7 @@ int drain_on_error(dlspm_ctx *ctx, int rc)
         }
     }
     (void)cudaGetLastError();
+    (void)dlspm_mma_check(ctx);  // the call fails as it is: nothing is left for the next one to report
     return rc;
 }
 
@@ -531,12 +540,12 @@ int rows_batched_host(dlspm_ctx *ctx, int count, const typename T::Problem *prob
 
 extern "C" int dlspm_sddmm_batched_f32_host(dlspm_ctx *ctx, int count, const dlspm_sddmm_problem *problems)
 {
-    return drain_on_error(ctx, rows_batched_host<SddmmTraits>(ctx, count, problems));
+    return host_call(ctx, [&] { return rows_batched_host<SddmmTraits>(ctx, count, problems); });
 }
 
 extern "C" int dlspm_fused_batched_f32_host(dlspm_ctx *ctx, int count, const dlspm_fused_problem *problems)
 {
-    return drain_on_error(ctx, rows_batched_host<FusedTraits>(ctx, count, problems));
+    return host_call(ctx, [&] { return rows_batched_host<FusedTraits>(ctx, count, problems); });
 }
 
 // ---- exported entry points: the implementations above plus the drain on failure ---------------------
@@ -544,26 +553,26 @@ extern "C" int dlspm_spmm_csr_f32_host(dlspm_ctx *ctx, int M, int K, int N, int 
                                        const int *row_offsets, const int *column_indices, const float *B,
                                        float *C)
 {
-    return drain_on_error(ctx, dlspm_spmm_csr_f32_host_impl(ctx, M, K, N, nnz, values, row_offsets, column_indices, B, C));
+    return host_call(ctx, [&] { return dlspm_spmm_csr_f32_host_impl(ctx, M, K, N, nnz, values, row_offsets, column_indices, B, C); });
 }
 
 extern "C" int dlspm_sddmm_csr_f32_host(dlspm_ctx *ctx, int M, int K, int N, int nnz, const int *row_offsets,
                                         const int *column_indices, const float *lhs, const float *rhs,
                                         float *out_values)
 {
-    return drain_on_error(ctx, dlspm_sddmm_csr_f32_host_impl(ctx, M, K, N, nnz, row_offsets, column_indices, lhs, rhs, out_values));
+    return host_call(ctx, [&] { return dlspm_sddmm_csr_f32_host_impl(ctx, M, K, N, nnz, row_offsets, column_indices, lhs, rhs, out_values); });
 }
 
 extern "C" int dlspm_fused_sddmm_spmm_f32_host(dlspm_ctx *ctx, int M, int K, int N, int nnz,
                                                const int *row_offsets, const int *column_indices,
                                                const float *C, const float *B, const float *D, float *E)
 {
-    return drain_on_error(ctx, dlspm_fused_sddmm_spmm_f32_host_impl(ctx, M, K, N, nnz, row_offsets, column_indices, C, B, D, E));
+    return host_call(ctx, [&] { return dlspm_fused_sddmm_spmm_f32_host_impl(ctx, M, K, N, nnz, row_offsets, column_indices, C, B, D, E); });
 }
 
 extern "C" int dlspm_spmm_batched_f32_host(dlspm_ctx *ctx, int count, const dlspm_problem *problems)
 {
-    return drain_on_error(ctx, dlspm_spmm_batched_f32_host_impl(ctx, count, problems));
+    return host_call(ctx, [&] { return dlspm_spmm_batched_f32_host_impl(ctx, count, problems); });
 }
 
 extern "C" int dlspm_host_copy_count(const dlspm_ctx *ctx, long long *copies)

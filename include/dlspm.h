@@ -431,9 +431,19 @@ int dlspm_peer_free(dlspm_ctx *ctx, void *ptr);
 
 /* ---- failure reporting ---------------------------------------------------------------------------- */
 
-/* No kernel of the library waits without a limit: a wait that runs out sets a status word and the
- * kernel returns (DLSPM_ERR_TIMEOUT through dlspm_batch_info).  This self-test exercises exactly that
- * path with no fault involved: one thread polls, at most `polls` (<= 2^20) times, an mbarrier that
+/* No kernel of the library waits without a limit: a wait that runs out sets a status word and the kernel returns
+ * with an incomplete result.  Who reports it:
+ *   - prepared batches: dlspm_batch_info (device_error).
+ *   - host-buffer calls (*_host, dlspm_mg_*): the call itself, with DLSPM_ERR_TIMEOUT.
+ *   - every other call returns before its kernels have run.  The word stays set until it is read: by dlspm_device_error,
+ *     or by the next call on the context that takes host buffers or would launch a kernel of that kind, which then
+ *     returns DLSPM_ERR_TIMEOUT without having run and may be repeated.  Launches replayed from a CUDA graph are
+ *     reported in the same way. */
+
+/* Synchronises the device; *device_error = 1 if a kernel of this context gave up a bounded wait since the word was
+ * last read (0 = no), and clears the word.  Prepared batches have a word of their own (dlspm_batch_info). */
+int dlspm_device_error(dlspm_ctx *ctx, int *device_error);
+/* Self-test of such a wait with no fault involved: one thread polls, at most `polls` (<= 2^20) times, an mbarrier that
  * nothing completes.  Returns DLSPM_ERR_TIMEOUT with *timed_out = 1, and the context stays usable. */
 int dlspm_selftest_bounded_wait(dlspm_ctx *ctx, unsigned polls, int *timed_out);
 

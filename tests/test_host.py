@@ -336,3 +336,29 @@ def test_row_partition_by_nnz(pkg, parts):
     assert b[0] == 0 and b[-1] == 100 and (np.diff(b) >= 0).all() and b[1] >= 90
     # no nonzeros: rows split evenly
     assert pkg.partition_rows_by_nnz(np.zeros(9, dtype=np.int32), 4).tolist() == [0, 2, 4, 6, 8]
+
+
+# ---- kernels that gave up a bounded wait -----------------------------------------------------------------
+
+def test_host_calls_report_a_kernel_that_gave_up(pkg, tmp_path):
+    """A host-buffer call whose own kernel gave up returns the status itself, and the call after it is not blamed; a
+    word that an earlier call left set is reported before anything runs.  (The entry points are compiled for the CPU
+    over a stand-in for the CUDA runtime.)"""
+    import shutil
+    import subprocess
+
+    nvcc = shutil.which("nvcc")
+    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include") if nvcc else ""
+    if not os.path.exists(os.path.join(include, "cuda_runtime.h")) or not shutil.which("g++"):
+        pytest.skip("no CUDA headers or no g++")
+    here = os.path.dirname(os.path.abspath(__file__))
+    exe = str(tmp_path / "host_calls")
+    api = os.path.join(pkg.PKG_DIR, "csrc", "host_api.cu")
+    subprocess.run(["g++", "-std=c++17", "-O1", f'-DHOST_API="{api}"', "-I", include, "-o", exe,
+                    os.path.join(here, "fake_host_calls.cpp")], check=True)
+    lines = subprocess.run([exe], check=True, capture_output=True, text=True).stdout.split("\n")
+    seen = {line.split()[0]: [int(x) for x in line.split()[1:]] for line in lines if line}
+    assert sorted(seen) == ["fused", "fused_batched", "sddmm", "sddmm_batched", "spmm", "spmm_batched"]
+    for name, (own, after, pending, calls, then) in seen.items():
+        assert (own, after) == (pkg.ERR_TIMEOUT, pkg.OK), name
+        assert (pending, calls, then) == (pkg.ERR_TIMEOUT, 0, pkg.OK), name
