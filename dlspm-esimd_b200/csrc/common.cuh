@@ -128,9 +128,9 @@ int dlspm_spmm_mma_launch_at(dlspm_ctx *ctx, const void *tables, const long long
                              int *error, cudaStream_t st);
 
 // SDDMM of one pattern on the tensor cores (sddmm_mma.cu), and whether it is the faster way: alone, or as one of many
-// problems of a grouped call.
-bool dlspm_sddmm_mma_pays_alone(const dlspm_ctx *ctx, int M, int K, int N, int nnz, int vec);
-void dlspm_sddmm_mma_choose(int count, const dlspm_sddmm_problem *problems, unsigned char *chosen);
+// problems of a grouped call (estimates of sddmm_route.h).
+bool dlspm_sddmm_mma_pays_alone(const dlspm_ctx *ctx, int M, int K, int N, int nnz, bool masked, int vec);
+void dlspm_sddmm_mma_choose(const dlspm_ctx *ctx, int count, const dlspm_sddmm_problem *problems, unsigned char *chosen);
 int dlspm_sddmm_mma(dlspm_ctx *ctx, int M, int K, int N, int nnz, const int *row_offsets, const int *cols, const float *mask,
                     const float *lhs, const float *rhs, float *out, cudaStream_t st);
 // Tables of a launch over `count` problems: their size, and their host image (returns the number of strips).

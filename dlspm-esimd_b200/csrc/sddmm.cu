@@ -349,7 +349,7 @@ int sddmm_launch(dlspm_ctx *ctx, int M, int K, int N, int nnz, const int *row_of
         return DLSPM_OK;
     }
     const int vec = dlspm_vec_width(N, lhs, rhs);
-    if (dlspm_sddmm_mma_pays_alone(ctx, M, K, N, nnz, vec))
+    if (dlspm_sddmm_mma_pays_alone(ctx, M, K, N, nnz, mask != nullptr, vec))
         return dlspm_sddmm_mma(ctx, M, K, N, nnz, row_offsets, column_indices, mask, lhs, rhs, out_values, st);
     int G = 0, R = 0;
     const int blocks = dlspm_ceil_div(M, kWarps);

@@ -17,6 +17,7 @@
 #include "common.cuh"
 #include "fused_device.cuh"
 #include "sddmm_device.cuh"
+#include "sddmm_route.h"
 
 using namespace dlspm;
 
@@ -283,24 +284,14 @@ struct HostEntry {
 // extra test.
 void choose_sharing(const dlspm_ctx *ctx, std::vector<HostEntry> (&by_class)[kClasses])
 {
-    const long long want = (long long)ctx->sm_count * 32;
     for (int c = 0; c < kClasses; c++) {
         if (c == 8 || c == 9) continue;  // filled below from 6 and 7
         std::vector<HostEntry> &v = by_class[c];
         long long rows = 0;
         for (const HostEntry &e : v) rows += e.p.M;
-        if (v.empty() || rows * 4 >= want * 3) continue;
-        int cls_shift = 0;
-        while (cls_shift < 3 && (rows << cls_shift) < want) cls_shift++;
-        for (HostEntry &e : v) {
-            int s = 0;
-            if (c < 6 || c >= 10) {
-                while (s < cls_shift && e.avg_row > 32.0 * (1 << s)) s++;
-            } else {
-                s = cls_shift;
-            }
-            e.p.shift = s;
-        }
+        const int most = sharing_most(ctx->sm_count, rows);
+        if (v.empty() || most == 0) continue;
+        for (HostEntry &e : v) e.p.shift = c < 6 || c >= 10 ? sharing_shift(most, e.avg_row) : most;
         if (c == 6 || c == 7) {  // shared long rows run on the kernels with the extra test
             for (HostEntry &e : v)
                 if (e.p.shift > 0) by_class[c + 2].push_back(e);
@@ -437,11 +428,10 @@ int dlspm_sddmm_batched_at(dlspm_ctx *ctx, int count, const dlspm_sddmm_problem 
             return DLSPM_ERR_INVALID_ARGUMENT;
     }
     std::vector<unsigned char> chosen((size_t)count);
-    dlspm_sddmm_mma_choose(count, problems, chosen.data());
+    dlspm_sddmm_mma_choose(ctx, count, problems, chosen.data());
     for (int i = 0; i < count; i++) {
         const dlspm_sddmm_problem &q = problems[i];
         if (q.M == 0 || q.nnz == 0) continue;
-        int G = 0, R = 0;
         const bool wide = q.N > 0 && dlspm_vec_width(q.N, q.lhs, q.rhs) == 4;
         if (chosen[(size_t)i]) {
             dense.push_back(q);
@@ -451,11 +441,7 @@ int dlspm_sddmm_batched_at(dlspm_ctx *ctx, int count, const dlspm_sddmm_problem 
             e.avg_row = (double)q.nnz / (double)q.M;
             e.work = (double)q.nnz * q.N;
             e.index = i;
-            // beyond the register-resident layouts: segments of 1024 floats, of 512 from N = 2052 on
-            // (the choice of the single-matrix launcher)
-            // rows of up to 32 floats: groups of four lanes, as in the single-matrix launcher
-            const int cls = q.N <= 16 ? 10 : q.N <= 32 ? 11 : sddmm_layout(q.N / 4, &G, &R) ? layout_class(G, R) : (q.N > 2048 ? 7 : 6);
-            by_class[cls].push_back(e);
+            by_class[sddmm_class(q.N)].push_back(e);
         } else {
             int rc = dlspm_sddmm_csr_masked_f32(ctx, q.M, q.K, q.N, q.nnz, q.row_offsets, q.column_indices, q.mask_values,
                                                 q.lhs, q.rhs, q.out_values, st);

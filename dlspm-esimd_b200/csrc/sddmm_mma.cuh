@@ -22,13 +22,11 @@
 // computed one by one with fp32 multiply-adds.
 #pragma once
 #include "mma_split.cuh"
+#include "sddmm_route.h"
 
 namespace dlspm {
 
-constexpr int kPickInner = 64;   // of the inner dimension per stage, and per main accumulator
 constexpr int kPickStages = 2;
-constexpr int kPickCols = 128;   // columns of the pattern per block, 256 per pair
-constexpr int kPickRows = 64;    // rows of the pattern converted per block at most, 128 per pair
 constexpr int kPickSumWarps = 8, kPickOperandWarps = 8, kPickWarps = 8;
 constexpr int kPickThreads = (kPickSumWarps + kPickOperandWarps + kPickWarps + 4) * 32;
 constexpr int kPickRhsPlane = kPickInner * kPickCols * 2, kPickLhsPlane = kPickInner * kPickRows * 2;
@@ -37,7 +35,6 @@ static_assert(kPickThreads * kPickRegsLaunch <= 65536 &&
                   32 * (kPickSumWarps * kPickRegsSum + kPickOperandWarps * kPickRegsOperand + kPickWarps * kPickRegsPick + 4 * kPickRegsIssue) <=
                       kPickThreads * kPickRegsLaunch,
               "register budgets exceed what the block is launched with");
-constexpr int kPickCheckMost = 8192;         // problems of a launch at most
 constexpr uint32_t kPickSmallColumn = 256;  // tensor memory: two main accumulators, then two for the small products
 constexpr int kPickRing = 16;               // tiles whose mark (numbers that cannot be split) can be alive at once
 

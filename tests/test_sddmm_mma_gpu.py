@@ -34,7 +34,10 @@ def lone_run(ctx, dev, M, K, N, ro, ci, lhs, rhs, mask=None):
 
 @pytest.mark.parametrize("M,K,N,density,kind", [(1024, 4096, 256, 0.5, "plain"), (1000, 4000, 300, 0.6, "masked"),
                                                 (900, 3001, 255, 0.4, "masked"), (1024, 4096, 256, 0.5, "reversed"),
-                                                (1024, 4096, 256, 0.5, "infinite"), (1024, 4096, 256, 0.5, "tiny")])
+                                                (1024, 4096, 256, 0.5, "infinite"), (1024, 4096, 256, 0.5, "tiny"),
+                                                (1024, 2048, 512, 0.5, "reversed"), (1024, 2048, 512, 0.5, "infinite"),
+                                                (1024, 2048, 512, 0.5, "tiny"), (2048, 512, 512, 0.5, "masked"),
+                                                (1500, 1000, 516, 0.4, "masked")])
 def test_lone_launches(pkg, oracle, ctx, dev, M, K, N, density, kind):
     seed = M + N
     ro, ci = csr_rowlen_normal(pkg, M, K, 1.0 - density, seed)
