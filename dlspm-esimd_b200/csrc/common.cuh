@@ -102,7 +102,7 @@ static inline int dlspm_mma_check(dlspm_ctx *ctx)
 // SpMM of one matrix on the tensor cores (spmm_mma.cu), and whether it is the faster way.
 bool dlspm_spmm_mma_pays_alone(const dlspm_ctx *ctx, int M, int K, int N, int nnz, int vec);
 int dlspm_spmm_mma(dlspm_ctx *ctx, int M, int K, int N, int nnz, const float *values, const int *row_offsets, const int *cols,
-                   const float *B, float *C, bool sorted, cudaStream_t st);  // sorted: columns are known to ascend
+                   const float *B, float *C, cudaStream_t st);
 
 // Whether the kernel's 32-bit offsets reach all of a problem.
 bool dlspm_spmm_mma_fits(int K, int N, int nnz);

@@ -289,7 +289,9 @@ int spmm_row_split(const dlspm_ctx *ctx, int M, int N, int nnz, int vec, bool st
 }
 
 
-// Known from a plan: max_row_len, the longest row (else 0), and whether all rows are sorted (else -1).
+// Known from a plan: max_row_len, the longest row (else 0), and whether all rows were sorted when it was made (else -1).
+// The kernels do not rely on the order (a plan may be used with its entries permuted inside rows since): rows that were not
+// sorted then only speak against the tensor cores, which would compute them a second time or gather them all.
 int spmm_launch(dlspm_ctx *ctx, int M, int K, int N, int nnz, const float *values, const int *row_offsets,
                 const int *cols, const float *B, float *C, const int *row_order, int max_row_len, int sorted, cudaStream_t st)
 {
@@ -298,7 +300,7 @@ int spmm_launch(dlspm_ctx *ctx, int M, int K, int N, int nnz, const float *value
     const int vec = dlspm_vec_width(N, B, C);
     const bool strict = ctx->strict_fp32 != 0;
     if (!strict && sorted != 0 && dlspm_spmm_mma_pays_alone(ctx, M, K, N, nnz, vec))
-        return dlspm_spmm_mma(ctx, M, K, N, nnz, values, row_offsets, cols, B, C, sorted > 0, st);
+        return dlspm_spmm_mma(ctx, M, K, N, nnz, values, row_offsets, cols, B, C, st);
     int split = spmm_row_split(ctx, M, N, nnz, vec, strict);
     // Long rows of uneven length (known only with a plan): eight warps per row make every thread
     // block finish its row together, which the binning by powers of two does not.  Measured on

@@ -190,7 +190,7 @@ int dlspm_spmm_mma_launch_at(dlspm_ctx *ctx, const void *tables, const long long
 }
 
 int dlspm_spmm_mma(dlspm_ctx *ctx, int M, int K, int N, int nnz, const float *values, const int *row_offsets, const int *cols,
-                   const float *B, float *C, bool sorted, cudaStream_t st)
+                   const float *B, float *C, cudaStream_t st)
 {
     const int rc = dlspm_mma_check(ctx);
     if (rc) return rc;
@@ -201,8 +201,6 @@ int dlspm_spmm_mma(dlspm_ctx *ctx, int M, int K, int N, int nnz, const float *va
     a.splits = mma_splits(ctx, a.tiles, K);
     const int clusters = a.splits > 1 ? (int)a.tiles : (int)std::min<long long>(a.tiles, ctx->sm_count / 2);
     const bool wide = dlspm_vec_width(N, B, B) == 4, deep = a.one.depth > kMmaDepth;
-    if (sorted && wide)
-        return deep ? mma_launch<false, true, true, false>(ctx, a, clusters, st) : mma_launch<false, true, false, false>(ctx, a, clusters, st);
     if (wide) return deep ? mma_launch<false, true, true, true>(ctx, a, clusters, st) : mma_launch<false, true, false, true>(ctx, a, clusters, st);
     return deep ? mma_launch<false, false, true, true>(ctx, a, clusters, st) : mma_launch<false, false, false, true>(ctx, a, clusters, st);
 }

@@ -110,7 +110,8 @@ int dlspm_spmm_csr_f32(dlspm_ctx *ctx, int M, int K, int N, int nnz, const float
                        const int *row_offsets, const int *column_indices, const float *B,
                        float *C, void *stream);
 
-/* Same with a plan (row-length binning computed once per sparsity pattern). */
+/* Same with a plan (row-length binning computed once per sparsity pattern).  A plan is a matter of speed only: row
+ * offsets, columns, their order inside rows and values are read anew by every call. */
 int dlspm_spmm_csr_f32_planned(dlspm_ctx *ctx, const dlspm_plan *plan, int N,
                                const float *values, const int *row_offsets,
                                const int *column_indices, const float *B, float *C,
@@ -252,7 +253,9 @@ int dlspm_fused_batched_f32_host(dlspm_ctx *ctx, int count, const dlspm_fused_pr
 /* A prepared batch: the problem table and its tile index live on the device, so repeated
  * launches cost no host work.  Creating it also analyses the patterns on the device: rows are
  * ordered by length inside every problem (so that the warps of a tile finish together), and
- * problems that are dense enough and have ascending columns are routed to the tiled kernel. */
+ * problems that are dense enough and have ascending columns are routed to the tiled kernels, which rely on
+ * that order.  So row_offsets and column_indices must hold what they held at creation whenever the batch is
+ * launched; values and B are read anew by every launch. */
 typedef struct dlspm_batch dlspm_batch;
 int dlspm_batch_create(dlspm_ctx *ctx, int count, const dlspm_problem *problems,
                        dlspm_batch **batch);

@@ -158,3 +158,32 @@ def test_problems_beyond_32_bit_offsets_stay_on_other_kernels(pkg, ctx, dev):
     v, rows = vals.reshape(M, per_row, 1).double(), B[ci.long()].double()
     want, scale = (v * rows).sum(1), (v * rows).abs().sum(1)
     assert ((C.double() - want).abs() <= TOL * scale).all()
+
+
+@pytest.mark.parametrize("what", ["permuted", "permuted everywhere", "doubled", "other columns"])
+def test_a_plan_does_not_keep_the_order_of_columns(pkg, oracle, ctx, dev, what):
+    """A plan made of a sorted pattern, used after the columns inside rows have changed."""
+    import torch
+
+    M, K, N = 1024, 2048, 512
+    ro, ci = csr_rowlen_normal(pkg, M, K, 0.7, 11)
+    vals = pkg.gen_dense_host(int(ci.size), 11, 2)
+    B = dense(pkg, K, N, 11, 10)
+    d_ro = to_dev(ro, dev)
+    p = ctx.plan_create(M, K, int(ci.size), d_ro, to_dev(ci, dev))
+    if what.startswith("permuted"):
+        other = shuffle_rows_columns(ro, ci, 3)
+        for i in range(M):  # every 32nd row is one that the kernel looks at first
+            if i % 32 or what == "permuted everywhere":
+                ci[ro[i]:ro[i + 1]] = other[ro[i]:ro[i + 1]]
+    elif what == "doubled":
+        for i in range(0, M, 7):
+            if ro[i + 1] - ro[i] > 3:
+                ci[ro[i] + 1] = ci[ro[i]]
+    else:
+        ci = pkg.gen_sample_columns_host(M, K, ro, 12)
+    out = torch.full((M, N), float("nan"), device=dev)
+    ctx.spmm_planned(p, N, to_dev(vals, dev), d_ro, to_dev(ci, dev), to_dev(B, dev), out)
+    torch.cuda.synchronize()
+    p.close()
+    check(oracle, ro, ci, vals, B, M, N, out.cpu().numpy())
