@@ -203,14 +203,6 @@ __device__ __forceinline__ void pick_store(uint32_t plane, const float4 (&d)[PAI
     }
 }
 
-__device__ __forceinline__ void pick_mark_slow(PickSmem &sm, int ring, unsigned rank)
-{
-    // in both blocks of the pair: rows of lhs are shared
-    atomicOr(&sm.slow[ring], 1u);
-    const uint32_t other = cluster_map(smem_u32(&sm.slow[ring]), rank ^ 1u);
-    asm volatile("red.relaxed.cluster.shared::cluster.or.b32 [%0], %1;" ::"r"(other), "r"(1u) : "memory");
-}
-
 template <bool TABLE, bool WIDE>
 __device__ __forceinline__ bool pick_operands(PickSmem &sm, const PickArgs &a, unsigned rank, int warp, int lane)
 {
@@ -252,7 +244,7 @@ __device__ __forceinline__ bool pick_operands(PickSmem &sm, const PickArgs &a, u
             }
         }
         if (have) load();
-        if (__any_sync(0xffffffffu, least < kSplitLeast) && lane == 0) pick_mark_slow(sm, now, rank);
+        if (__any_sync(0xffffffffu, least < kSplitLeast) && lane == 0) mark_in_pair(&sm.slow[now], 1u, rank);  // rows of lhs are shared
         if (chunk == 0) least = 0xffffffffu;
         fence_async_smem();
         __syncwarp();

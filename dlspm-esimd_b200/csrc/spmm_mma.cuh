@@ -256,10 +256,7 @@ __device__ __forceinline__ void mma_store_entry(uint32_t row, int col, float v, 
 
 __device__ __forceinline__ void mma_mark_again(MmaSmem &sm, int ring, int bit, unsigned rank)
 {
-    // the marks of a tile are kept in both blocks of the pair
-    atomicOr(&sm.again[ring][bit >> 5], 1u << (bit & 31));
-    const uint32_t other = cluster_map(smem_u32(&sm.again[ring][bit >> 5]), rank ^ 1u);
-    asm volatile("red.relaxed.cluster.shared::cluster.or.b32 [%0], %1;" ::"r"(other), "r"(1u << (bit & 31)) : "memory");
+    mark_in_pair(&sm.again[ring][bit >> 5], 1u << (bit & 31), rank);
 }
 
 // One tile: every lane group of eight lanes owns one row of it, 4 * warp + group, and walks it once.  DEPTH: entries

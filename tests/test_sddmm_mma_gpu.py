@@ -37,7 +37,7 @@ def lone_run(ctx, dev, M, K, N, ro, ci, lhs, rhs, mask=None):
                                                 (1024, 4096, 256, 0.5, "infinite"), (1024, 4096, 256, 0.5, "tiny"),
                                                 (1024, 2048, 512, 0.5, "reversed"), (1024, 2048, 512, 0.5, "infinite"),
                                                 (1024, 2048, 512, 0.5, "tiny"), (2048, 512, 512, 0.5, "masked"),
-                                                (1500, 1000, 516, 0.4, "masked")])
+                                                (1500, 1000, 516, 0.4, "masked"), (1024, 2048, 512, 0.5, "tiny rows")])
 def test_lone_launches(pkg, oracle, ctx, dev, M, K, N, density, kind):
     seed = M + N
     ro, ci = csr_rowlen_normal(pkg, M, K, 1.0 - density, seed)
@@ -47,6 +47,9 @@ def test_lone_launches(pkg, oracle, ctx, dev, M, K, N, density, kind):
     lhs = dense(pkg, M, N, seed, 11, kind=pkg.KIND_NORMAL)
     rhs = dense(pkg, K, N, seed, 12, kind=pkg.KIND_NORMAL)
     mask = pkg.gen_dense_host(int(ci.size), seed, 2) if kind == "masked" else None
+    if kind == "tiny rows":  # each converted by one block of a pair, and looked up by both
+        lhs, rhs = lhs.copy(), (rhs * np.float32(1e20)).astype(np.float32)
+        lhs[[0, 9, 20, 31, 500, 1023]] *= np.float32(1e-36)
     if kind == "tiny":
         lhs, rhs = (lhs * np.float32(1e-36)).astype(np.float32), (rhs * np.float32(1e20)).astype(np.float32)
     if kind == "infinite":

@@ -98,7 +98,7 @@ def test_lone_launches(pkg, oracle, ctx, dev, M, K, N, density, order):
     check(oracle, ro, ci, vals, B, M, N, lone_run(ctx, dev, M, K, N, ro, ci, vals, B, plan=True))
 
 
-@pytest.mark.parametrize("where", ["infinite", "tiny", "huge"])
+@pytest.mark.parametrize("where", ["infinite", "tiny", "huge", "tiny rows", "tiny columns"])
 def test_numbers_that_cannot_be_split(pkg, oracle, ctx, dev, where):
     """Infinities and NaN reach the rows that refer to them and no others; magnitudes at the ends of the range keep
     their precision."""
@@ -120,7 +120,15 @@ def test_numbers_that_cannot_be_split(pkg, oracle, ctx, dev, where):
         keep[[5, 300]] = False
         assert np.allclose(out[:, keep], want[:, keep], rtol=1e-4, atol=1e-4)
         return
-    if where == "tiny":
+    if where.startswith("tiny "):  # seen by one block of a pair only: a row of its half, columns of its half
+        B *= np.float32(1e20)
+        if where == "tiny rows":
+            for i in (3, 77, 140, 260, 299):
+                vals[ro[i]:ro[i + 1]] *= np.float32(1e-36)
+        else:
+            for _ in range(2):
+                B[:, [3, 140, 141, 400]] *= np.float32(1e-28)
+    elif where == "tiny":
         vals = (vals * np.float32(1e-36)).astype(np.float32)
         B *= np.float32(1e20)
     else:
