@@ -13,6 +13,7 @@ The directory name contains a hyphen, so it is imported through `importlib` unde
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import importlib.machinery
 import importlib.util
 import os
@@ -159,8 +160,8 @@ def exported_names() -> Sequence[str]:
 
 
 def build(verbose: bool = False) -> None:
-    """Compiles libdlspm.so and the drivers in-tree with nvcc for sm_100a (no GPU needed)."""
-    cmd = ["make", "-C", PKG_DIR, "-j", str(os.cpu_count() or 4), "PYTHON=" + sys.executable, "all"]
+    """Compiles libdlspm.so, the drivers and the binding's native module in-tree, for sm_100a (no GPU needed)."""
+    cmd = ["make", "-C", PKG_DIR, "-j", str(os.cpu_count() or 4), "PYTHON=" + sys.executable, "all", "python"]
     proc = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if verbose or proc.returncode != 0:
         print(proc.stdout)
@@ -193,7 +194,7 @@ def _load_call():
     if _call is None:
         load_library()
         if not os.path.exists(CALL_PATH):
-            raise RuntimeError(f"{CALL_PATH} is missing: build it with `make -C {PKG_DIR}` (no fallback exists)")
+            raise RuntimeError(f"{CALL_PATH} is missing: build it with `make -C {PKG_DIR} python` (no fallback exists)")
         import torch  # noqa: F401  (the module links against torch's libraries)
 
         loader = importlib.machinery.ExtensionFileLoader("_dlspm_call", CALL_PATH)
@@ -269,8 +270,12 @@ class Context:
         self.handle = _P()
         self.device = device
         _check(self.lib.dlspm_create(C.byref(self.handle), device), "dlspm_create")
-        self._call = _load_call()
         self._address = self.handle.value
+
+    @functools.cached_property
+    def _call(self):
+        """The native module of the tensor-taking calls, loaded (and torch with it) by the first of them."""
+        return _load_call()
 
     def close(self) -> None:
         if self.handle:

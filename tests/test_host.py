@@ -54,6 +54,29 @@ def test_strerror_and_no_device_failure(pkg):
         assert e.value.status == pkg.ERR_NO_DEVICE
 
 
+def test_library_and_host_calls_need_no_torch(pkg, monkeypatch):
+    """The library and the drivers build without torch or the Python headers, and a context that is used for host
+    buffers only does not load the binding's native module."""
+    import subprocess
+
+    plan = subprocess.run(["make", "-n", "-B", "-C", pkg.PKG_DIR, "PYTHON=/nonexistent/python"], capture_output=True, text=True)
+    assert plan.returncode == 0 and "libdlspm.so" in plan.stdout and "bin/spmm-fromfile" in plan.stdout
+    assert "torch" not in plan.stdout and "_dlspm_call" not in plan.stdout and "nonexistent" not in plan.stdout + plan.stderr
+
+    class Library:
+        def __getattr__(self, name):
+            return lambda *args: pkg.OK
+
+    monkeypatch.setattr(pkg, "load_library", lambda: Library())
+    monkeypatch.setattr(pkg, "CALL_PATH", "/nonexistent/_dlspm_call.so")
+    monkeypatch.setattr(pkg, "_call", None)
+    ctx = pkg.Context(0)
+    one = np.ones(1, dtype=np.float32)
+    ctx.spmm_host(1, 1, 1, 1, one, np.array([0, 1], np.int32), np.zeros(1, np.int32), one, one.copy())
+    with pytest.raises(RuntimeError, match="make .* python"):
+        ctx.spmm(1, 1, 1, 1, None, None, None, None, None)
+
+
 # ---- .smtx reader ------------------------------------------------------------------------------------
 
 def test_smtx_round_trip(pkg, oracle, tmp_path):
