@@ -383,10 +383,12 @@ void launch_fast(const int *ro, const int *ci, const float *c, const float *b, c
         launch_overlapped(fused_rows_split_kernel<G, R, MODE>, (unsigned)((warps + kWarps - 1) / kWarps), kWarps * 32, smem, st, ro, ci, c, b, d, e, M, chunks, scale, split_shift);
         return;
     }
-    // Launches of a few waves in blocks of four rows: the SMs then differ by less (4096 rows are 3.5 blocks of eight per
-    // SM: 40.9 -> 39.3 us at d = 64; 5353 rows, d = 224: 123 -> 102 us).  Longer launches keep eight, whose rows meet
-    // in L1 (16384 rows, d = 128, with four: 217 -> 222 us).
-    const int warps = (long long)M <= 40LL * kWarps * sm_count / 10 ? 4 : kWarps;
+    // Launches of two to five blocks per SM in blocks of four rows where a row is up to 128 floats: the SMs then differ by
+    // less.  Measured (band masks with 1 and 5 % more entries, and uniform ones), time with four against eight rows per
+    // block: d = 32, 3700 rows 0.89 to 0.93, 5000 0.93; d = 64, 4096 0.95 to 0.99; d = 128, 2600 0.88 to 0.92, 3000 0.95
+    // to 0.97, 5353 0.95 to 1.0; in between 0.98 to 1.02.  Outside, eight rows meet in L1: d = 128, 2200 rows 0.97 to
+    // 1.06; d = 192 and 256, 2048 rows 1.0 to 1.06; d = 32, 10000 rows 1.07 to 1.11.
+    const int warps = G <= 8 && (long long)M > 2LL * kWarps * sm_count && (long long)M <= 5LL * kWarps * sm_count ? kWarps / 2 : kWarps;
     if constexpr (G == 32 && R == 4) {
         if ((long long)M > 2LL * kWarps * sm_count) {  // more rows than two resident blocks per SM hold
             launch_overlapped(fused_rows_kernel<G, R, MODE, true>, dlspm_ceil_div(M, warps), warps * 32, 0, st, ro, ci, c, b, d, e, M, chunks, scale);

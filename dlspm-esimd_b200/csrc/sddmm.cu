@@ -268,8 +268,8 @@ void launch_fast(const int *ro, const int *ci, const float *lhs, const float *rh
             per_sm = n > 0 ? n : 4;
         }
         // (Patterns that fit one wave of the two-chunk layout's build for eight resident blocks are shared as well: left
-        // alone they are 5 to 20 % faster with even rows, 8192 x 8192 at 10 %, N = 64 96 -> 90 us, but last as long as
-        // their longest row with uneven ones, with a spread of 40 % 1.1 to 1.8 times as long.)
+        // alone they are 5 to 20 % faster with even rows (8192 x 8192 at 10 %, N = 64 96 -> 90 us, with factors 105 -> 90),
+        // but last as long as their longest row with uneven ones, with a spread of 40 % 1.1 to 1.8 times as long.)
         split_shift = sddmm_wave_shift(((long long)M + kWarps - 1) / kWarps, (long long)per_sm * sm_count, avg_row);
     }
     const long long warps = (long long)M << (split_shift + k_shift);

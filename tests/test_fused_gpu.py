@@ -2,7 +2,7 @@
 import numpy as np
 import pytest
 
-from cases import csr_bernoulli, csr_from_lengths, dense, shuffle_rows_columns
+from cases import csr_bernoulli, csr_from_lengths, csr_rowlen_normal, dense, shuffle_rows_columns
 from conftest import TOL, to_dev
 
 pytestmark = pytest.mark.gpu
@@ -130,3 +130,11 @@ def test_rows_of_32_floats_in_a_long_launch(pkg, oracle, ctx, dev, offset_floats
     ctx.fused(M, K, N, int(ci.size), to_dev(ro, dev), to_dev(ci, dev), d_q, d_k, d_v, out)
     torch.cuda.synchronize()
     check(oracle, ro, ci, q, k, v, M, N, out.cpu().numpy().reshape(M, N))
+
+
+@pytest.mark.parametrize("M,N", [(2368, 128), (2369, 128), (2371, 32), (4099, 64), (5920, 16), (5921, 128), (3002, 132)])
+def test_blocks_of_four_and_eight_rows(pkg, oracle, ctx, dev, M, N):
+    """Either side of the launch sizes that run in blocks of four rows, with a last block that is not full."""
+    ro, ci = csr_rowlen_normal(pkg, M, 300, 0.9, M + N)
+    q, k, v = dense(pkg, M, N, 1, 11), dense(pkg, 300, N, 1, 12), dense(pkg, 300, N, 1, 13)
+    check(oracle, ro, ci, q, k, v, M, N, run_fused(ctx, dev, M, 300, N, ro, ci, q, k, v))
