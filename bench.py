@@ -11,11 +11,13 @@ a seed.  A step is one pass over the whole batch: one grouped launch per GPU.  W
 problems are dealt out by nnz*N (longest-processing-time), so total work is fixed ("strong").
 The metric is GFLOP/s = sum(2*nnz*N) / time.
 
-One JSON line is printed by rank 0.  Besides the contract keys it carries `roofline` (algorithmic
-bytes of rank 0's launch over its event-timed duration, against the measured HBM copy bandwidth),
-`e2e` (the same metric through the host-buffer C-ABI call, copies included, on a stated sample of
-the batch), `cpu_baseline` (the CPU oracle on the host cores, N=1 only) and `extras` (the other
-configurations: single SpMM, SDDMM, fused, the 90 % sparsity sweep, the row-sharded large SpMM).
+One JSON line is printed by rank 0, short enough to be read back from the end of a log.  Besides the
+contract keys it carries `roofline` (algorithmic bytes of rank 0's launch over its event-timed duration,
+against the measured HBM copy bandwidth), `e2e` (the same metric through the host-buffer C-ABI call,
+copies included, on a stated sample of the batch) and `cpu_baseline` (the CPU oracle on the host cores,
+N=1 only).  What is longer (the kernels of the step one by one, variants of the CPU baseline, the other
+configurations: single SpMM, SDDMM, fused, the 90 % sparsity sweep, the row-sharded large SpMM) goes to
+standard error as one JSON line per item, and with --details FILE, unrounded, to a file.
 """
 from __future__ import annotations
 
@@ -39,12 +41,12 @@ WIDTHS = [256, 1024, 3136]
 COV = 0.4
 STREAM_PICK = 50
 FALLBACK_HBM_GBS = 6650.0
-# DRAM bytes per algorithmic byte of the two kernels of a step, from one ncu capture each on the
-# first 256 problems of the batch (dram__bytes_read.sum + dram__bytes_write.sum over the algorithmic
-# bytes of the problems the kernel served: 2.18 + 0.61 GB for 3.06 GB on the row-gather kernel, whose
-# last results are still in L2 when it ends; 0.72 + 0.16 GB for 0.82 GB on the tiled kernel).  Traffic
-# grows with the bytes of the problems processed, so the ratios are applied to the full launch.
-NCU_TRAFFIC_PER_ALGORITHMIC_BYTE = {"spmm_batched_kernel": 0.913, "spmm_tile_kernel": 1.077}
+# DRAM bytes per algorithmic byte of the two parts of a step, from one ncu capture each on the first 256 problems of the
+# batch (dram__bytes_read.sum + dram__bytes_write.sum over the algorithmic bytes of the problems the part served: 2.18 +
+# 0.61 GB for 3.06 GB on the row-gather kernel, whose last results are still in L2 when it ends; 5.62 + 0.53 GB for 2.52 GB
+# in the two builds of the tensor-core kernel, which read a B that L2 does not hold once per 128 rows).  Traffic grows with
+# the bytes of the problems processed, so the ratios are applied to the full launch.
+NCU_TRAFFIC_PER_ALGORITHMIC_BYTE = {"spmm_batched_kernel": 0.913, "spmm_mma_kernel": 2.44}
 
 
 def log(*a):
@@ -453,7 +455,66 @@ def run_reference_arm(args, rank, world):
         "e2e": {"value": gflops, "unit": "GFLOP/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
         "gpu_launches": 0,
     }
-    print(json.dumps(line), flush=True)
+    print_result(line, args.details)
+
+
+LINE_LIMIT = 2500  # characters of the result line
+
+
+def rounded(x, digits=6):
+    """The same JSON value with its floats cut to `digits` significant digits."""
+    if isinstance(x, float):
+        return float(f"{x:.{digits}g}")
+    if isinstance(x, dict):
+        return {k: rounded(v, digits) for k, v in x.items()}
+    return [rounded(v, digits) for v in x] if isinstance(x, (list, tuple)) else x
+
+
+def result_line(line):
+    """(the line to print, the parts left out of it): the result without the long parts."""
+    short, rest = dict(line), {}
+    for path in (("extras",), ("roofline", "kernels"), ("cpu_baseline", "single_thread"), ("cpu_baseline", "o3_march_native"),
+                 ("cpu_baseline", "loops_interchanged"), ("cpu_baseline", "onemkl")):
+        inner = short.get(path[0])
+        if len(path) == 1:
+            if inner is not None:
+                rest[path[0]] = short.pop(path[0])
+        elif isinstance(inner, dict) and path[1] in inner:
+            short[path[0]] = {k: v for k, v in inner.items() if k != path[1]}
+            rest[".".join(path)] = inner[path[1]]
+    text = json.dumps(rounded(short))
+    if len(text) > LINE_LIMIT:  # (not seen: what is left is bounded)
+        log(f"the result line has {len(text)} characters")
+    return text, rest
+
+
+def count_launches(run, at_least):
+    """Kernels of this library that one call of `run` launches, counted by the profiler outside the timed region (the
+    call's own count of parts where the profiler is not to be had)."""
+    import torch
+
+    try:
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            run()
+            torch.cuda.synchronize()
+        names = [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+        ours = [n for n in names if "spmm_" in n and "kernel" in n]
+        return max(len(ours), at_least)
+    except Exception as e:
+        log(f"launches not counted: {str(e)[:100]}")
+        return at_least
+
+
+def print_result(line, details):
+    text, rest = result_line(line)
+    for name, part in rest.items():
+        items = part.items() if name == "extras" and isinstance(part, dict) else [(None, part)]
+        for key, value in items:
+            log(json.dumps({name if key is None else f"{name}.{key}": rounded(value)}))
+    if details:
+        with open(details, "w") as f:
+            json.dump(line, f, indent=1)
+    print(text, flush=True)
 
 
 def workload_config(args, world):
@@ -980,6 +1041,7 @@ def main():
     ap.add_argument("--spmm-kernel", type=int, default=0, help="0 auto, 1 row-gather only, 2 tiled where possible, 3 tiled with zeros")
     ap.add_argument("--e2e-bytes", type=float, default=None,
                     help="host bytes of the e2e sample per rank (default: 16e9 on one GPU, 4e9 per rank on several)")
+    ap.add_argument("--details", default=None, metavar="FILE", help="write the whole result, unrounded, to FILE (rank 0)")
     args = ap.parse_args()
 
     rank = int(os.environ.get("RANK", "0"))
@@ -1063,10 +1125,11 @@ def main():
     ms_per_step = total_ms / args.steps
     value = float(tot[0]) / (ms_per_step * 1e-3) * 1e-9
 
-    # each kernel of the step on its own (rank 0's share), for the roofline of the dominant one
+    # each part of the step on its own (rank 0's share), for the roofline of the dominant one: the row-gather launches, and
+    # the launches over 128-row tiles (tensor cores; the FMA tile kernel for half-full problems that do not suit them)
     parts = {}
     for part, name, nprob, fl, by in ((1, "spmm_batched_kernel", n_gather, part_stats[0], part_stats[1]),
-                                      (2, "spmm_tile_kernel", n_tiled, part_stats[2], part_stats[3])):
+                                      (2, "spmm_mma_kernel", n_tiled, part_stats[2], part_stats[3])):
         if not nprob:
             continue
         batch.batch.launch_part(part)
@@ -1081,6 +1144,10 @@ def main():
         parts[name] = {"problems": nprob, "launch_ms": ms, "gflops": fl / ms * 1e-6,
                        "algorithmic_bytes_per_launch": by, "achieved_gbs": by / ms * 1e-6,
                        "fp32_frac": fl / (ms * 1e-3) * 1e-12 / fp32_tflops}
+    barrier()
+
+    if rank == 0:
+        launches_per_step = count_launches(lambda: batch.batch.launch(), launches_per_step)
     barrier()
 
     # what the timed launches computed, against the CPU oracle (rank 0's share; after the timed
@@ -1184,7 +1251,7 @@ def main():
                                               f"({flops / 1e9:.2f} GFLOP, {dt:.1f} s)",
                                     "build": "-O2 -ffp-contract=off (the build the parity tests pin)"}
             line["cpu_baseline"].update(cpu_variants(oracle, data, flops, dt, threads))
-        print(json.dumps(line), flush=True)
+        print_result(line, args.details)
     if world > 1:
         dist.destroy_process_group()
     ctx.close()

@@ -70,3 +70,33 @@ def test_profile_summaries_keep_the_profiler_rules():
             if re.match(r"\s+ncu\s", line):
                 assert "--clock-control none" in line, f"{os.path.basename(path)}: {line.strip()}"
                 assert "--set full" not in line or " -k " in line, f"{os.path.basename(path)}: a full capture of every kernel"
+
+
+def test_result_line_is_short_and_keeps_the_contract(bench, tmp_path, capsys):
+    """The line that is read back from the end of a log: one JSON object below the limit, however much was measured."""
+    import json
+
+    kernels = {f"kernel_{i}": {"problems": 4643, "launch_ms": 214.123456789012, "gflops": 27800.123456789} for i in range(5)}
+    line = {"metric": "spmm_batch_gflops", "value": 27812.3456789012, "unit": "GFLOP/s", "n_gpus": 1, "steps": 20, "warmup": 5,
+            "ms_per_step": 213.98765432101, "higher_is_better": True, "scaling": "strong", "vs_baseline": None, "dtype": "f32",
+            "data": "synthetic", "config": {"workload": "w" * 300, "problems": 8192, "partition": "lpt by nnz*N"},
+            "clocks": {"sm_mhz": 1965.0, "sm_max_mhz": 1965.0, "reasons": ["sw_power_cap"]},
+            "e2e": {"value": 3070.123456789, "unit": "GFLOP/s", "h2d_bytes_per_step": 1.1e10, "d2h_bytes_per_step": 4.8e9, "sample": "s" * 200},
+            "gpu_launches": 100, "parity": {"checked": 90, "violations": 0, "worst_ratio_of_tol": 0.00412345678901},
+            "roofline": {"bound": "hbm", "achieved": 373.123456789, "peak": 6552.3, "kernel": "kernel_0", "kernels": kernels},
+            "extras": {f"case_{i}": dict(kernels) for i in range(40)},
+            "cpu_baseline": {"value": 25.0123456789, "unit": "GFLOP/s", "cores": 16, "kind": "port", "sample": "s" * 100,
+                             "single_thread": kernels, "o3_march_native": kernels, "loops_interchanged": kernels, "onemkl": kernels}}
+    whole = str(tmp_path / "details.json")
+    bench.print_result(line, whole)
+    captured = capsys.readouterr()
+    assert captured.out.count("\n") == 1 and len(captured.out) <= bench.LINE_LIMIT
+    got = json.loads(captured.out)
+    for key in line:
+        if key != "extras":
+            assert key in got
+    assert got["value"] == pytest.approx(line["value"], rel=1e-5) and got["e2e"]["h2d_bytes_per_step"] == 1.1e10
+    assert "kernels" not in got["roofline"] and "onemkl" not in got["cpu_baseline"]
+    said = [json.loads(x) for x in captured.err.splitlines()]
+    assert {k for x in said for k in x} >= {"extras.case_0", "extras.case_39", "roofline.kernels", "cpu_baseline.onemkl"}
+    assert json.load(open(whole)) == line
