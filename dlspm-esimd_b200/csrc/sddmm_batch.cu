@@ -7,10 +7,14 @@
 // inner dimension, see sddmm_device.cuh) run in ONE persistent launch: warps pull rows from a device
 // counter (thread blocks pull tiles of eight where the fused chain shares rows between warps), one
 // warp per row, and every row is processed exactly as in the
-// single-matrix kernels (same passes, same butterfly, same order of additions), so results have the
-// same bits (one exception: rows of exactly 32 floats in single-matrix launches of 8192 rows or more use
-// 256-bit loads there and can differ in the last place).  A batch with one inner dimension is one
-// launch; a mixed batch is at most twelve.
+// single-matrix gather kernels (same passes, same butterfly, same order of additions), so results have
+// the same bits as theirs (one exception: rows of exactly 32 floats in single-matrix launches of 8192 rows
+// or more use 256-bit loads there and can differ in the last place).  A batch with one inner dimension is
+// one launch; a mixed batch is at most twelve.
+//
+// Denser SDDMMs with long inner dimensions go to the tensor cores instead (sddmm_mma.cuh), one launch in
+// front of these.  The choice is made for the call as a whole (sddmm_route.h), and lone calls make one of
+// their own, so the last bits of a problem's result depend on which problems it is grouped with.
 #include <algorithm>
 #include <vector>
 

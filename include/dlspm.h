@@ -74,10 +74,11 @@ typedef enum dlspm_option {
      * multiplied as zeros, except in chunks of B that hold an infinity or a NaN, which run under the presence
      * masks, so that a non-finite value of B reaches exactly the rows that reference it, as in the reference loop.
      * 2 runs every chunk under the masks (slower; kept for tests).  1, 2 and 3 give the same bits on the same input
-     * (apart from the sign of a zero sum, see the kernel).  The automatic choice takes, problem by problem, the
+     * (apart from the sign of a zero sum, see the kernel).  The automatic choice takes for every problem the
      * row-gather kernel or the tensor cores (from about 5 % nonzeros where the matrix is large; every fp32 product
      * from six bf16 products of its operands' exact three-part splits, sums in fp32, errors below those of the other
-     * kernels; the tiled kernel above for problems from 45 % nonzeros that do not suit them).  In strict mode
+     * kernels; the tiled kernel above for problems from 45 % nonzeros that do not suit them).  It estimates the batch
+     * as a whole: in another batch a problem may run on another kernel and differ in its last bits.  In strict mode
      * (DLSPM_OPT_STRICT_FP32) it stays on the kernels whose order of additions is the reference's. */
     DLSPM_OPT_SPMM_KERNEL = 1,
     /* Threshold of the automatic choice, in thousandths: the tiled kernels (tensor cores, fp32 tile kernel) are taken
@@ -192,7 +193,8 @@ typedef struct dlspm_problem {
  * on one stream (two calls whose work overlaps on the GPU would share that scratch).  The table
  * copies read host memory that dies with the call, so the call cannot be recorded into a CUDA
  * graph: on a capturing stream it returns DLSPM_ERR_UNSUPPORTED before anything is enqueued (use
- * dlspm_batch_create + dlspm_batch_launch there). */
+ * dlspm_batch_create + dlspm_batch_launch there).  Problems are dealt to the row-gather kernel and the tensor
+ * cores as in the automatic choice of prepared batches (DLSPM_OPT_SPMM_KERNEL). */
 int dlspm_spmm_batched_f32(dlspm_ctx *ctx, int count, const dlspm_problem *problems,
                            void *stream);
 
@@ -233,9 +235,12 @@ typedef struct dlspm_fused_problem {
     float *E;                  /* device, M x N */
 } dlspm_fused_problem;
 
-/* Runs `count` independent SDDMMs (each as dlspm_sddmm_csr_masked_f32 would) in one persistent
- * launch per register layout present in the batch (the layout follows from N: at most twelve, one for
- * a batch with a single inner dimension); denser problems with long inner dimensions share one launch on the tensor cores.  Replaces the per-matrix process launches of
+/* Runs `count` independent SDDMMs (each as dlspm_sddmm_csr_masked_f32 would, up to the order of additions) in
+ * one persistent launch per register layout present in the batch (the layout follows from N: at most twelve,
+ * one for a batch with a single inner dimension); denser problems with long inner dimensions share one launch on
+ * the tensor cores in front of these, where an estimate from the sizes of all problems says that the call is then
+ * faster.  So which kernel a problem runs on, and with it the last bits of its result, depends on the other
+ * problems of the call; the same call gives the same bits every time.  Replaces the per-matrix process launches of
  * SDDMM/batch-run-sddmm_fromfile:31-47, where every layer-sized pattern is launch-bound on its own.
  * `problems` is a HOST array; the tables go to the context's scratch, so the same rules as for
  * dlspm_spmm_batched_f32 hold: calls on one context ordered on one stream, not on a capturing
