@@ -24,6 +24,7 @@
 //   16 operand warps  convert 64 rows of B and scatter the matching 64 columns of the sparse rows, eight lanes a
 //                     row, into one of three stages; both come from registers loaded one chunk ahead.
 //   1 issuing warp    (of the even block) issues 24 multiplies a chunk; in the odd block it relays barriers.
+//   1 planning warp   lays the next tiles out (problem, place, the rows' entries) for all others.
 // (registers are handed out in groups of four warps; the rest of the last group is idle)
 //
 // Rows whose columns are not strictly ascending, tiles with magnitudes that cannot be split, and sums that are
@@ -47,6 +48,7 @@ constexpr int kMmaDensePlane = kMmaChunk * kMmaCols * 2;   // bytes of one part 
 constexpr int kMmaSparsePlane = kMmaChunk * kMmaRows * 2;
 constexpr int kMmaCheckMost = 8192;  // problems of a launch whose columns may be out of order
 constexpr uint32_t kMmaSmallColumn = 256;  // tensor memory: two main accumulators, then two for the small products
+constexpr int kMmaAhead = 4;    // tiles planned ahead
 constexpr int kMmaRing = 16;    // tiles whose marks (rows to compute again) can be alive at once
 constexpr int kMmaRegsLaunch = 72, kMmaRegsSum = 88, kMmaRegsOperand = 72, kMmaRegsIssue = 40;
 static_assert(kMmaThreads * kMmaRegsLaunch <= 65536 &&
@@ -66,12 +68,24 @@ struct MmaProblem {
     int depth;       // entries of a row fetched ahead, in eights: 1 to 8
 };
 
+// A tile as the planning warp hands it to the other roles.
+struct MmaTile {
+    MmaProblem p;                        // (launches over a table)
+    int row0, n0;                        // first row and column of this block's part
+    int rows;                            // rows per block of the pair
+    int chunk0, chunks;                  // its part of K; no chunks: there are no more tiles
+    int ring;                            // its marks
+    int start[kMmaRows], end[kMmaRows];  // entries of this block's rows
+};
+
 struct MmaSmem {
     unsigned char dense[kMmaStages][3][kMmaDensePlane];    // B: rows of 64 of its columns, 128-byte swizzle
     unsigned char sparse[kMmaStages][3][kMmaSparsePlane];  // A: rows of 64 columns, 128-byte swizzle
     unsigned long long full[kMmaStages], empty[kMmaStages];  // operands written (both blocks) / multiplies done
     unsigned long long sum_full[2], sum_empty[2];            // accumulators complete / added by all sum warps
+    unsigned long long tile_full[kMmaAhead], tile_empty[kMmaAhead];  // tile planned / no longer read
     unsigned long long drain;                                // multiplies still running when a wait ran out
+    MmaTile tile[kMmaAhead];
     unsigned again[kMmaRing][kMmaMarkWords];                  // rows of the tile to compute again
     unsigned unsorted[kMmaCheckMost / 32];                   // problems whose columns do not ascend (see mma_looks_sorted)
     uint32_t tmem;
@@ -93,15 +107,6 @@ struct MmaArgs {
     int *error;
 };
 
-struct MmaTile {
-    long long tile;
-    int prob;
-    const MmaProblem *p;
-    int row0, n0;       // first row and column of this block's part
-    int rows;           // rows per block of the pair
-    int chunk0, chunks; // its part of K
-};
-
 // A position in the ring of stages and the parity of its barriers' current phase.
 struct MmaStage {
     int stage;
@@ -115,8 +120,18 @@ struct MmaStage {
     }
 };
 
+// ---- planning warp ------------------------------------------------------------------------------------
+
+// Where the walk over the tiles of a cluster is.
+struct MmaPlan {
+    long long tile;
+    int prob;
+    const MmaProblem *p;
+    int cb, rb;  // 256 columns, block_rows rows
+};
+
 template <bool TABLE>
-__device__ __forceinline__ bool mma_tile_load(MmaTile &t, const MmaArgs &a, unsigned rank)
+__device__ __forceinline__ bool mma_plan_load(MmaPlan &t, const MmaArgs &a)
 {
     if (t.tile >= a.tiles) return false;
     long long first = 0;
@@ -134,35 +149,120 @@ __device__ __forceinline__ bool mma_tile_load(MmaTile &t, const MmaArgs &a, unsi
         t.p = &a.one;
     }
     const int i = (int)(t.tile - first);
-    const int cb = i / t.p->row_blocks, rb = i - cb * t.p->row_blocks;
-    t.rows = t.p->block_rows >> 1;
-    t.row0 = rb * t.p->block_rows;
-    t.n0 = cb * 2 * kMmaCols + (int)(rank & 1u) * kMmaCols;
-    const int all = (t.p->K + kMmaChunk - 1) / kMmaChunk;
-    const int part = (int)(rank >> 1);
-    t.chunk0 = (int)((long long)all * part / a.splits);
-    t.chunks = (int)((long long)all * (part + 1) / a.splits) - t.chunk0;
+    t.cb = i / t.p->row_blocks;
+    t.rb = i - t.cb * t.p->row_blocks;
     return true;
 }
 
 // The same, past tiles of problems that were computed at the start of the kernel.
 template <bool TABLE, bool CHECK>
-__device__ __forceinline__ bool mma_tile_next(MmaTile &t, const MmaArgs &a, const MmaSmem &sm, unsigned rank)
+__device__ __forceinline__ bool mma_plan_next(MmaPlan &t, const MmaArgs &a, const MmaSmem &sm)
 {
-    while (mma_tile_load<TABLE>(t, a, rank)) {
+    while (mma_plan_load<TABLE>(t, a)) {
         if (!(TABLE && CHECK) || !((sm.unsorted[t.prob >> 5] >> (t.prob & 31)) & 1u)) return true;
         t.tile += gridDim.x / (2u * (unsigned)a.splits);
     }
     return false;
 }
 
-// First entry of the row at or behind column `col`.
-__device__ __forceinline__ int mma_lower_bound(const int *__restrict__ cols, int lo, int hi, int col)
+// Lays tile n of this cluster out; false behind the last one.
+template <bool TABLE, bool CHECK>
+__device__ __forceinline__ bool mma_plan_tile(MmaSmem &sm, const MmaArgs &a, unsigned rank, int lane, MmaPlan &t, unsigned n)
 {
-    while (lo < hi) {
-        const int mid = lo + ((hi - lo) >> 1);
-        if (__ldg(cols + mid) < col) lo = mid + 1;
-        else hi = mid;
+    const bool more = mma_plan_next<TABLE, CHECK>(t, a, sm);
+    MmaTile &out = sm.tile[n % kMmaAhead];
+    if (more) {
+        const int rows = t.p->block_rows >> 1, row0 = t.rb * t.p->block_rows;
+        int start[kMmaRows / 32], end[kMmaRows / 32];
+#pragma unroll
+        for (int i = 0; i < kMmaRows / 32; i++) {  // (all of them in flight)
+            const int r = lane + 32 * i, row = row0 + (int)(rank & 1u) * rows + r;
+            start[i] = end[i] = 0;
+            if (r < rows && row < t.p->M) {
+                start[i] = __ldg(t.p->row_offsets + row);
+                end[i] = __ldg(t.p->row_offsets + row + 1);
+            }
+        }
+        if constexpr (TABLE) {
+            static_assert(sizeof(MmaProblem) == 64, "copied by sixteen lanes");
+            if (lane < 16) reinterpret_cast<int *>(&out.p)[lane] = __ldg(reinterpret_cast<const int *>(t.p) + lane);
+        }
+        if (lane == 0) {
+            const int all = (t.p->K + kMmaChunk - 1) / kMmaChunk, part = (int)(rank >> 1), shift = __ffs(a.splits) - 1;  // splits: 1, 2 or 4
+            out.rows = rows;
+            out.row0 = row0;
+            out.n0 = t.cb * 2 * kMmaCols + (int)(rank & 1u) * kMmaCols;
+            out.chunk0 = (all * part) >> shift;
+            out.chunks = ((all * (part + 1)) >> shift) - out.chunk0;
+            out.ring = (int)(n % kMmaRing);
+        }
+#pragma unroll
+        for (int i = 0; i < kMmaRows / 32; i++) {
+            out.start[lane + 32 * i] = start[i];
+            out.end[lane + 32 * i] = end[i];
+        }
+        t.tile += gridDim.x / (2u * (unsigned)a.splits);
+    } else if (lane == 0) {
+        out.chunks = 0;
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sm.tile_full[n % kMmaAhead]);
+    return more;
+}
+
+// Tiles n, n + 1, .. up to kMmaAhead ahead of the other roles, so that none of them meets the chain of dependent loads
+// (which problem, its sizes and addresses, the rows' offsets) between two tiles: with every role looking its tiles up by
+// itself a tile cost 2 to 3 us more (37 problems of 2048 x 512 at 10 %, N = 3136, eight chunks a tile: 2.06 -> 1.65 us per
+// chunk of 64 columns; of 1024 x 4096, N = 1024, 64 chunks a tile: 1.75 -> 1.62; a batch of 256 problems 6040 -> 5640 us).
+template <bool TABLE, bool CHECK>
+__device__ __forceinline__ bool mma_plan(MmaSmem &sm, const MmaArgs &a, unsigned rank, int lane, MmaPlan &t, unsigned n)
+{
+    for (;; n++) {
+        if (!mbar_wait_suspended(&sm.tile_empty[n % kMmaAhead], ((n / kMmaAhead) & 1u) ^ 1u, &sm.abort)) return false;
+        if (!mma_plan_tile<TABLE, CHECK>(sm, a, rank, lane, t, n)) return true;
+    }
+}
+
+// A role's walk over the planned tiles.
+struct MmaWalk {
+    unsigned n = 0;
+    // Waits for the tile; false if a wait ran out.
+    __device__ __forceinline__ bool wait(MmaSmem &sm) const
+    {
+        return mbar_wait_suspended(&sm.tile_full[n % kMmaAhead], (n / kMmaAhead) & 1u, &sm.abort);
+    }
+    __device__ __forceinline__ const MmaTile &tile(const MmaSmem &sm) const { return sm.tile[n % kMmaAhead]; }
+    // By one thread per warp (or relay), when the tile is no longer read.
+    __device__ __forceinline__ void done(MmaSmem &sm) { mbar_arrive(&sm.tile_empty[n % kMmaAhead]); }
+};
+// The problem of a tile: of a lone launch among the kernel's arguments, where its fields cost no registers.
+template <bool TABLE>
+__device__ __forceinline__ const MmaProblem &mma_problem_of(const MmaTile &t, const MmaArgs &a)
+{
+    if constexpr (TABLE) return t.p;
+    else return a.one;
+}
+
+// First entries at or behind column `col` of the rows of a warp, eight lanes a row, 32 probes a round: two or three
+// rounds of dependent loads for a row, where halving took twelve (with the planning, 1024 x 4096 at 10 %, N = 1024 in two
+// parts: 59.2 -> 57.2 us).
+__device__ __forceinline__ int mma_lower_bound(const int *__restrict__ cols, int lo, int hi, int col, int l8)
+{
+    while (__any_sync(0xffffffffu, lo < hi)) {
+        const int step = max(1, (hi - lo + 31) / 32);
+        int below = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int at = lo + (4 * l8 + i) * step;
+            if (at < hi && __ldg(cols + at) < col) below++;
+        }
+#pragma unroll
+        for (int d = 1; d < 8; d <<= 1) below += __shfl_xor_sync(0xffffffffu, below, d);
+        if (lo < hi) {
+            const int l = lo;
+            if (below > 0) lo = l + (below - 1) * step + 1;
+            hi = min(hi, l + below * step);
+        }
     }
     return lo;
 }
@@ -262,28 +362,20 @@ __device__ __forceinline__ void mma_mark_again(MmaSmem &sm, int ring, int bit, u
 // One tile: every lane group of eight lanes owns one row of it, 4 * warp + group, and walks it once.  DEPTH: entries
 // of a row fetched ahead, in eights.  CHECK: columns may be out of order (a prepared batch looked at them when it was
 // made).
-template <int DEPTH, bool CHECK, bool WIDE>
-__device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, const MmaTile &t, unsigned rank, int warp, int lane,
-                                                 int ring, MmaStage &st)
+template <int DEPTH, bool TABLE, bool CHECK, bool WIDE>
+__device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, const MmaTile &t, unsigned rank, int warp, int lane, MmaStage &st)
 {
     volatile int *abort = &sm.abort;
-    const MmaProblem &p = *t.p;
+    const MmaProblem &p = mma_problem_of<TABLE>(t, a);
     const int l8 = lane & 7, group = lane & 24, own = warp * 4 + (lane >> 3);
     const int swizzle = (own & 7) << 4;
+    const int chunks = t.chunks;
     const bool row_warp = warp * 4 < t.rows;  // this warp has rows in the tile
-    int cursor = 0, end = 0;
-    {
-        const int row = t.row0 + (int)(rank & 1u) * t.rows + own;
-        if (own < t.rows && row < p.M) {
-            const int start = __ldg(p.row_offsets + row), stop = __ldg(p.row_offsets + row + 1);
-            cursor = start;
-            end = stop;
-            if (a.splits > 1) {
-                const int part = (int)(rank >> 1);
-                if (part > 0) cursor = mma_lower_bound(p.cols, start, stop, t.chunk0 * kMmaChunk);
-                if (part + 1 < a.splits) end = mma_lower_bound(p.cols, start, stop, (t.chunk0 + t.chunks) * kMmaChunk);
-            }
-        }
+    int cursor = t.start[own], end = t.end[own];
+    if (a.splits > 1) {
+        const int part = (int)(rank >> 1), first = cursor, stop = end;
+        if (part > 0) cursor = mma_lower_bound(p.cols, first, stop, t.chunk0 * kMmaChunk, l8);
+        if (part + 1 < a.splits) end = mma_lower_bound(p.cols, first, stop, (t.chunk0 + t.chunks) * kMmaChunk, l8);
     }
     int k0 = t.chunk0 * kMmaChunk;
     MmaDense b;
@@ -377,9 +469,9 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
             if (CHECK && cursor != end) bad = true;  // entries out of order were never reached
             const bool all = __any_sync(0xffffffffu, least < kSplitLeast);
             if (__any_sync(0xffffffffu, bad) || all) {
-                if (bad && own < t.rows) mma_mark_again(sm, ring, (int)(rank & 1u) * t.rows + own, rank);
+                if (bad && own < t.rows) mma_mark_again(sm, t.ring, (int)(rank & 1u) * t.rows + own, rank);
                 if (all)
-                    for (int r = lane; r < 2 * t.rows; r += 32) mma_mark_again(sm, ring, r, rank);
+                    for (int r = lane; r < 2 * t.rows; r += 32) mma_mark_again(sm, t.ring, r, rank);
             }
         }
         fence_async_smem();
@@ -395,22 +487,22 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
         // two chunks a turn with the register sets exchanged: copying one to the other would wait for its loads
         int c1[DEPTH];
         float v1[DEPTH];
-        for (int i = 0; i < t.chunks; i += 2) {
+        for (int i = 0; i < chunks; i += 2) {
             step(c0, v0, c1, v1);
             if (!ok) return false;
-            hand_over(i + 1 == t.chunks);
-            if (i + 1 < t.chunks) {
+            hand_over(i + 1 == chunks);
+            if (i + 1 < chunks) {
                 step(c1, v1, c0, v0);
                 if (!ok) return false;
-                hand_over(i + 2 == t.chunks);
+                hand_over(i + 2 == chunks);
             }
         }
     } else {
         // (no registers for a second set; the entries of a dense chunk are fetched behind the last one's)
-        for (int i = 0; i < t.chunks; i++) {
+        for (int i = 0; i < chunks; i++) {
             step(c0, v0, c0, v0);
             if (!ok) return false;
-            hand_over(i + 1 == t.chunks);
+            hand_over(i + 1 == chunks);
         }
     }
     return true;
@@ -419,40 +511,33 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
 template <bool TABLE, bool WIDE, bool DEEP, bool CHECK>
 __device__ __forceinline__ bool mma_operands(MmaSmem &sm, const MmaArgs &a, unsigned rank, int warp, int lane)
 {
-    MmaTile t;
-    t.tile = blockIdx.x / (2u * (unsigned)a.splits);
-    t.prob = 0;
-    const unsigned stride = gridDim.x / (2u * (unsigned)a.splits);
     MmaStage st{0, 0u};
-    int ring = 0;
-    while (mma_tile_next<TABLE, CHECK>(t, a, sm, rank)) {
+    for (MmaWalk walk;; walk.n++) {
+        if (!walk.wait(sm)) return false;
+        const MmaTile &t = walk.tile(sm);
+        if (t.chunks == 0) return true;
         bool ok;
         if constexpr (DEEP) {
-            ok = mma_operand_tile<8, CHECK, WIDE>(sm, a, t, rank, warp, lane, ring, st);
+            ok = mma_operand_tile<8, TABLE, CHECK, WIDE>(sm, a, t, rank, warp, lane, st);
         } else {
-            if (t.p->depth == 1) ok = mma_operand_tile<1, CHECK, WIDE>(sm, a, t, rank, warp, lane, ring, st);
-            else if (t.p->depth == 2) ok = mma_operand_tile<2, CHECK, WIDE>(sm, a, t, rank, warp, lane, ring, st);
-            else ok = mma_operand_tile<5, CHECK, WIDE>(sm, a, t, rank, warp, lane, ring, st);
+            const int depth = mma_problem_of<TABLE>(t, a).depth;
+            if (depth == 1) ok = mma_operand_tile<1, TABLE, CHECK, WIDE>(sm, a, t, rank, warp, lane, st);
+            else if (depth == 2) ok = mma_operand_tile<2, TABLE, CHECK, WIDE>(sm, a, t, rank, warp, lane, st);
+            else ok = mma_operand_tile<5, TABLE, CHECK, WIDE>(sm, a, t, rank, warp, lane, st);
         }
         if (!ok) return false;
-        ring = (ring + 1) % kMmaRing;
-        t.tile += stride;
+        __syncwarp();
+        if (lane == 0) walk.done(sm);
     }
-    return true;
 }
 
 // ---- issuing warp (of the even block) ----------------------------------------------------------
 
 // The whole warp walks the chunks, one lane issues (the instructions take their operands from uniform registers,
 // which the compiler can only use where control flow is uniform).
-template <bool TABLE, bool CHECK>
-__device__ __forceinline__ bool mma_issue(MmaSmem &sm, const MmaArgs &a, unsigned rank, bool issuer)
+__device__ __forceinline__ bool mma_issue(MmaSmem &sm, unsigned rank, bool issuer, int lane)
 {
     volatile int *abort = &sm.abort;
-    MmaTile t;
-    t.tile = blockIdx.x / (2u * (unsigned)a.splits);
-    t.prob = 0;
-    const unsigned stride = gridDim.x / (2u * (unsigned)a.splits);
     const unsigned pair_mask = 3u << rank;
     const uint32_t tmem = sm.tmem;
     // parts (of B, of A) of the five small products
@@ -460,11 +545,16 @@ __device__ __forceinline__ bool mma_issue(MmaSmem &sm, const MmaArgs &a, unsigne
     const uint64_t dense0 = mma_descriptor(smem_u32(&sm.dense[0][0][0]), 8192, 1024, kSwizzle128);
     const uint64_t sparse0 = mma_descriptor(smem_u32(&sm.sparse[0][0][0]), 0, 1024, kSwizzle128);
     constexpr uint64_t kDense = kMmaDensePlane >> 4, kSparse = kMmaSparsePlane >> 4;
-    unsigned g = 0, done = 0;  // chunks (one main accumulator each) and tiles so far
-    while (mma_tile_next<TABLE, CHECK>(t, a, sm, rank)) {
-        const uint32_t instruction = mma_instruction(256, 2 * t.rows, true, false);
-        const uint32_t small = tmem + kMmaSmallColumn + (done & 1u) * 128u;
-        for (int c = 0; c < t.chunks; c++, g++) {
+    unsigned g = 0;  // chunks (one main accumulator each) so far
+    for (MmaWalk walk;; walk.n++) {
+        if (!walk.wait(sm)) return false;
+        const int chunks = walk.tile(sm).chunks, rows = walk.tile(sm).rows;
+        __syncwarp();
+        if (lane == 0) walk.done(sm);
+        if (chunks == 0) return true;
+        const uint32_t instruction = mma_instruction(256, 2 * rows, true, false);
+        const uint32_t small = tmem + kMmaSmallColumn + (walk.n & 1u) * 128u;
+        for (int c = 0; c < chunks; c++, g++) {
             const int s = (int)(g % kMmaStages);
             // (the accumulator of the small products was read together with the tile's last main one)
             if (g >= 2u && !mbar_wait_suspended(&sm.sum_empty[g & 1u], ((g >> 1) - 1u) & 1u, abort)) return false;
@@ -486,36 +576,30 @@ __device__ __forceinline__ bool mma_issue(MmaSmem &sm, const MmaArgs &a, unsigne
             }
             __syncwarp();
         }
-        done++;
-        t.tile += stride;
     }
-    return true;
 }
 
 // ---- relay (odd block) ------------------------------------------------------------------------------------
 
 // Passes the odd block's barriers on to the even block's, one arrival per phase: a remote arrival orders all
-// memory accesses of its thread first, which would hold up a warp with loads in flight.
-template <bool TABLE, bool CHECK>
-__device__ __forceinline__ bool mma_relay(MmaSmem &sm, const MmaArgs &a, unsigned rank, bool sums)
+// memory accesses of its thread first, which would hold up a warp with loads in flight.  (One thread.)
+__device__ __forceinline__ bool mma_relay(MmaSmem &sm, unsigned rank, bool sums)
 {
     volatile int *abort = &sm.abort;
-    MmaTile t;
-    t.tile = blockIdx.x / (2u * (unsigned)a.splits);
-    t.prob = 0;
-    const unsigned stride = gridDim.x / (2u * (unsigned)a.splits);
     const unsigned slots = sums ? 2u : (unsigned)kMmaStages;
     unsigned long long *own = sums ? sm.sum_empty : sm.full;
     const uint32_t other = cluster_map(smem_u32(own), rank ^ 1u);
     unsigned g = 0;
-    while (mma_tile_next<TABLE, CHECK>(t, a, sm, rank)) {
-        for (int c = 0; c < t.chunks; c++, g++) {
+    for (MmaWalk walk;; walk.n++) {
+        if (!walk.wait(sm)) return false;
+        const int chunks = walk.tile(sm).chunks;
+        walk.done(sm);
+        if (chunks == 0) return true;
+        for (int c = 0; c < chunks; c++, g++) {
             if (!mbar_wait_suspended(&own[g % slots], (g / slots) & 1u, abort)) return false;
             mbar_arrive_cluster(other + (g % slots) * 8u);
         }
-        t.tile += stride;
     }
-    return true;
 }
 
 // ---- sum warps --------------------------------------------------------------------------------------------
@@ -556,34 +640,31 @@ __device__ __forceinline__ void mma_mark_not_finite(MmaSmem &sm, int ring, const
 
 // Warp w: tensor-memory lanes 32 * (w % 4) .. + 31 (columns of C), accumulator columns 64 * (w / 4) .. + 63
 // (rows of the sparse matrix).
-template <bool TABLE, bool CHECK>
+template <bool TABLE>
 __device__ __forceinline__ bool mma_sums(MmaSmem &sm, const MmaArgs &a, unsigned rank, int warp, int lane)
 {
     volatile int *abort = &sm.abort;
-    MmaTile t;
-    t.tile = blockIdx.x / (2u * (unsigned)a.splits);
-    t.prob = 0;
-    const unsigned stride = gridDim.x / (2u * (unsigned)a.splits);
     const int half = (warp >> 2) * kMmaRows, quarter = warp & 3;
     const uint32_t tmem = sm.tmem + ((uint32_t)quarter << 21) + (uint32_t)half;
-    unsigned q = 0, done = 0;
-    int ring = 0;
-    while (mma_tile_next<TABLE, CHECK>(t, a, sm, rank)) {
+    unsigned q = 0;
+    for (MmaWalk walk;; walk.n++) {
+        if (!walk.wait(sm)) return false;
+        const MmaTile &t = walk.tile(sm);
+        const int chunks = t.chunks;
+        if (chunks == 0) return true;
         const int tile_rows = 2 * t.rows;
         float acc[kMmaRows];
 #pragma unroll
         for (int j = 0; j < kMmaRows; j++) acc[j] = 0.f;
-        for (int i = 0; i < t.chunks; i++, q++) {
+        for (int i = 0; i < chunks; i++, q++) {
             if (!mbar_wait_suspended(&sm.sum_full[q & 1u], (q >> 1) & 1u, abort)) return false;
             tmem_fence_after();
             tmem_add(acc, tmem + (q & 1u) * 128u, tile_rows - half);
-            if (i + 1 == t.chunks) tmem_add(acc, tmem + kMmaSmallColumn + (done & 1u) * 128u, tile_rows - half);
+            if (i + 1 == chunks) tmem_add(acc, tmem + kMmaSmallColumn + (walk.n & 1u) * 128u, tile_rows - half);
             tmem_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.sum_empty[q & 1u]);
         }
-        done++;
-        const int n = t.n0 + 32 * quarter + lane;
         if (a.splits > 1) {
             // partial sums to shared memory (the stages are free: this was the last tile); the blocks of the
             // cluster that hold the same columns add them up behind a cluster barrier, in mma_combine
@@ -592,28 +673,30 @@ __device__ __forceinline__ bool mma_sums(MmaSmem &sm, const MmaArgs &a, unsigned
             for (int j = 0; j < kMmaRows; j++) part[(half + j) * kMmaCols + 32 * quarter + lane] = acc[j];
             return true;
         }
+        const int ring = t.ring;
         mma_mark_not_finite(sm, ring, acc, half, lane);
-        if (n < t.p->N) {
-            float *c = t.p->C + (size_t)(t.row0 + half) * (size_t)t.p->N + n;
-            const int rows = min(tile_rows, t.p->M - t.row0) - half;
+        const MmaProblem &p = mma_problem_of<TABLE>(t, a);
+        const int n = t.n0 + 32 * quarter + lane;
+        if (n < p.N) {
+            const int N = p.N, rows = min(tile_rows, p.M - t.row0) - half;
+            float *c = p.C + (size_t)(t.row0 + half) * (size_t)N + n;
 #pragma unroll
             for (int j = 0; j < kMmaRows; j++)
-                if (j < rows) __stcs(c + (size_t)j * (size_t)t.p->N, acc[j]);
+                if (j < rows) __stcs(c + (size_t)j * (size_t)N, acc[j]);
         }
         sum_warps_barrier();
         unsigned any = 0;
         for (int w = 0; w < kMmaMarkWords; w++) any |= *(volatile unsigned *)&sm.again[ring][w];
         if (any) {
             for (int j = warp; j < tile_rows; j += kMmaSumWarps)
-                if (((*(volatile unsigned *)&sm.again[ring][j >> 5] >> (j & 31)) & 1u) && t.row0 + j < t.p->M)
-                    mma_row_again(*t.p, t.row0 + j, t.n0, lane);
+                if (((*(volatile unsigned *)&sm.again[ring][j >> 5] >> (j & 31)) & 1u) && t.row0 + j < p.M)
+                    mma_row_again(p, t.row0 + j, t.n0, lane);
             sum_warps_barrier();
             if (warp == 0 && lane < kMmaMarkWords) sm.again[ring][lane] = 0u;
         }
-        ring = (ring + 1) % kMmaRing;
-        t.tile += stride;
+        __syncwarp();
+        if (lane == 0) walk.done(sm);
     }
-    return true;
 }
 
 // splits > 1: adds the partial sums of the tile over the parts of K, in order.  Block part p takes the rows of
@@ -621,13 +704,11 @@ __device__ __forceinline__ bool mma_sums(MmaSmem &sm, const MmaArgs &a, unsigned
 template <bool TABLE>
 __device__ __forceinline__ void mma_combine(MmaSmem &sm, const MmaArgs &a, unsigned rank, int warp, int lane)
 {
-    MmaTile t;
-    t.tile = blockIdx.x / (2u * (unsigned)a.splits);
-    t.prob = 0;
-    mma_tile_load<TABLE>(t, a, rank);
+    const MmaTile &t = sm.tile[0];  // the only one
+    const MmaProblem &p = mma_problem_of<TABLE>(t, a);
     const int tile_rows = 2 * t.rows, part = (int)(rank >> 1);
     const int per = (tile_rows + a.splits - 1) / a.splits;
-    const int first = part * per, last = min(min(first + per, tile_rows), t.p->M - t.row0);
+    const int first = part * per, last = min(min(first + per, tile_rows), p.M - t.row0);
     const uint32_t sums = smem_u32(&sm.dense[0][0][0]);
     uint32_t again = 0;  // lane w < 4: word w of the marks of all parts
     if (lane < kMmaMarkWords)
@@ -645,12 +726,12 @@ __device__ __forceinline__ void mma_combine(MmaSmem &sm, const MmaArgs &a, unsig
         for (int i = 0; i < 4; i++) probe = fmaf(v[i], 0.f, probe);
         const unsigned word = __shfl_sync(0xffffffffu, again, j >> 5);
         if (__any_sync(0xffffffffu, probe != 0.f) || ((word >> (j & 31)) & 1u)) {
-            mma_row_again(*t.p, t.row0 + j, t.n0, lane);
+            mma_row_again(p, t.row0 + j, t.n0, lane);
         } else {
-            float *c = t.p->C + (size_t)(t.row0 + j) * (size_t)t.p->N + t.n0 + lane;
+            float *c = p.C + (size_t)(t.row0 + j) * (size_t)p.N + t.n0 + lane;
 #pragma unroll
             for (int i = 0; i < 4; i++)
-                if (t.n0 + lane + 32 * i < t.p->N) c[32 * i] = v[i];
+                if (t.n0 + lane + 32 * i < p.N) c[32 * i] = v[i];
         }
     }
 }
@@ -699,7 +780,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_c
     MmaSmem &sm = *reinterpret_cast<MmaSmem *>(smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned rank = cluster_rank();
-    constexpr int kIssueWarp = kMmaSumWarps + kMmaOperandWarps;
+    constexpr int kIssueWarp = kMmaSumWarps + kMmaOperandWarps, kPlanWarp = kIssueWarp + 2;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kMmaStages; s++) {
             mbar_init(&sm.full[s], kMmaOperandWarps + (rank & 1u ? 0u : 1u));  // even block: plus the odd one's relay
@@ -708,6 +789,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_c
         for (int b = 0; b < 2; b++) {
             mbar_init(&sm.sum_full[b], 1);
             mbar_init(&sm.sum_empty[b], kMmaSumWarps + (rank & 1u ? 0u : 1u));
+        }
+        for (int n = 0; n < kMmaAhead; n++) {
+            mbar_init(&sm.tile_full[n], 1);
+            mbar_init(&sm.tile_empty[n], kMmaSumWarps + kMmaOperandWarps + (rank & 1u ? 2u : 1u));  // and the issuing warp or both relays
         }
         mbar_init(&sm.drain, 1);
         sm.abort = 0;
@@ -722,6 +807,12 @@ __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_c
     else cluster_arrive_relaxed();
     if (!a.beside) grid_dependency_wait();
     if (a.before_next) grid_dependency_launch();
+    MmaPlan plan;
+    plan.tile = blockIdx.x / (2u * (unsigned)a.splits);
+    plan.prob = 0;
+    // (a lone launch has few tiles: its first one is planned before the other warps look at the order of the columns)
+    bool more = true;
+    if (!TABLE && warp == kPlanWarp) more = mma_plan_tile<TABLE, CHECK>(sm, a, rank, lane, plan, 0u);
     cluster_wait();
     tmem_fence_after();
     bool ok = true, done = false;
@@ -745,21 +836,22 @@ __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_c
         // nothing left to do
     } else if (warp < kMmaSumWarps) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kMmaRegsSum));
-        ok = mma_sums<TABLE, CHECK>(sm, a, rank, warp, lane);
+        ok = mma_sums<TABLE>(sm, a, rank, warp, lane);
     } else if (warp < kIssueWarp) {
         if (kMmaRegsOperand != kMmaRegsLaunch) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kMmaRegsOperand));
         ok = mma_operands<TABLE, WIDE, DEEP, CHECK>(sm, a, rank, warp - kMmaSumWarps, lane);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kMmaRegsIssue));
+        if (warp == kPlanWarp && more) ok = mma_plan<TABLE, CHECK>(sm, a, rank, lane, plan, TABLE ? 0u : 1u);
         if (warp == kIssueWarp && (rank & 1u) == 0u) {
             const bool issuer = elect_one();
-            ok = mma_issue<TABLE, CHECK>(sm, a, rank, issuer);
+            ok = mma_issue(sm, rank, issuer, lane);
             if (!ok && issuer) {  // multiplies in flight get a bounded chance to end before the tensor memory is freed
                 mma_commit<true>(&sm.drain, 1u << rank);
                 (void)mbar_wait(&sm.drain, 0u);
             }
         }
-        if (warp <= kIssueWarp + 1 && (rank & 1u) && lane == 0) ok = mma_relay<TABLE, CHECK>(sm, a, rank, warp != kIssueWarp);
+        if (warp <= kIssueWarp + 1 && (rank & 1u) && lane == 0) ok = mma_relay(sm, rank, warp != kIssueWarp);
     }
     if (!ok) {
         *(volatile int *)&sm.abort = 1;

@@ -98,6 +98,35 @@ def test_lone_launches(pkg, oracle, ctx, dev, M, K, N, density, order):
     check(oracle, ro, ci, vals, B, M, N, lone_run(ctx, dev, M, K, N, ro, ci, vals, B, plan=True))
 
 
+def test_many_tiles_per_cluster(pkg, oracle, ctx, dev):
+    """More tiles for every pair of blocks than are planned ahead, of problems of different sizes, as a prepared batch
+    (columns known to ascend) and as a one-shot call (columns checked)."""
+    import torch
+
+    shapes = [(17 + 53 * i % 290, 40 + 31 * i % 90, 260 + 4 * (i % 3)) for i in range(120)]
+    assert sum(-(-M // 128) * -(-N // 256) for M, K, N in shapes) > 5 * 74
+    ctx.set_option(pkg.OPT_TILE_MIN_DENSITY, 0)
+    try:
+        arr, keep = pkg.ProblemArray(len(shapes)), []
+        for i, (M, K, N) in enumerate(shapes):
+            ro, ci = csr_bernoulli(pkg, M, K, 0.3, i)
+            vals, B = pkg.gen_dense_host(int(ci.size), i, 2), dense(pkg, K, N, i, 10)
+            out = torch.full((M * N,), float("nan"), device=dev)
+            arr.set(i, M, K, N, int(ci.size), to_dev(vals, dev), to_dev(ro, dev), to_dev(ci, dev), to_dev(B, dev), out)
+            keep.append((ro, ci, vals, B, out))
+        batch = ctx.batch_create(arr)
+        assert batch.info()[1] == len(shapes)
+        for launch in (batch.launch, lambda: ctx.spmm_batched(arr)):
+            launch()
+            torch.cuda.synchronize()
+            for (M, K, N), (ro, ci, vals, B, out) in zip(shapes, keep):
+                check(oracle, ro, ci, vals, B, M, N, out.cpu().numpy().reshape(M, N))
+                out.fill_(float("nan"))
+        batch.close()
+    finally:
+        ctx.set_option(pkg.OPT_TILE_MIN_DENSITY, -1)
+
+
 @pytest.mark.parametrize("where", ["infinite", "tiny", "huge", "tiny rows", "tiny columns"])
 def test_numbers_that_cannot_be_split(pkg, oracle, ctx, dev, where):
     """Infinities and NaN reach the rows that refer to them and no others; magnitudes at the ends of the range keep
