@@ -43,25 +43,40 @@ __device__ __forceinline__ uint32_t bf16x2_bits(float lo, float hi)
     return *reinterpret_cast<const uint32_t *>(&t);
 }
 
-// (x, y) -> the packed first, second and third parts.  The remainders are formed two at a time (both subtractions
-// are exact).
+// x minus the low (high) half of a packed pair, exact where the half is x rounded to bf16.  One instruction that takes the
+// half as it is: 7 instructions for a pair instead of 9 (with the halves widened first, two subtractions packed into one
+// instruction); a batch of 256 SpMMs 5690 -> 5540 us, whose operand warps are bound by instruction issue.
+__device__ __forceinline__ float minus_low(uint32_t pair, float x)
+{
+    float r;
+    asm("{\n .reg .b16 lo, hi, m;\n mov.b32 {lo, hi}, %1;\n mov.b16 m, 0xbf80;\n fma.rn.f32.bf16 %0, lo, m, %2;\n}\n" : "=f"(r) : "r"(pair), "f"(x));
+    return r;
+}
+__device__ __forceinline__ float minus_high(uint32_t pair, float x)
+{
+    float r;
+    asm("{\n .reg .b16 lo, hi, m;\n mov.b32 {lo, hi}, %1;\n mov.b16 m, 0xbf80;\n fma.rn.f32.bf16 %0, hi, m, %2;\n}\n" : "=f"(r) : "r"(pair), "f"(x));
+    return r;
+}
+
+// (x, y) -> the packed first, second and third parts.
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t &p1, uint32_t &p2, uint32_t &p3)
 {
-    float2 r = make_float2(x, y);
-    const float2 minus = make_float2(-1.f, -1.f);
-    p1 = bf16x2_bits(r.x, r.y);
-    r = __ffma2_rn(make_float2(__uint_as_float(p1 << 16), __uint_as_float(p1 & 0xffff0000u)), minus, r);
-    p2 = bf16x2_bits(r.x, r.y);
-    r = __ffma2_rn(make_float2(__uint_as_float(p2 << 16), __uint_as_float(p2 & 0xffff0000u)), minus, r);
-    p3 = bf16x2_bits(r.x, r.y);
+    p1 = bf16x2_bits(x, y);
+    x = minus_low(p1, x);
+    y = minus_high(p1, y);
+    p2 = bf16x2_bits(x, y);
+    x = minus_low(p2, x);
+    y = minus_high(p2, y);
+    p3 = bf16x2_bits(x, y);
 }
 // One number alone, parts in the low halves.
 __device__ __forceinline__ void split_one(float x, uint32_t &p1, uint32_t &p2, uint32_t &p3)
 {
     p1 = bf16x2_bits(x, 0.f);
-    x -= __uint_as_float(p1 << 16);
+    x = minus_low(p1, x);
     p2 = bf16x2_bits(x, 0.f);
-    x -= __uint_as_float(p2 << 16);
+    x = minus_low(p2, x);
     p3 = bf16x2_bits(x, 0.f);
 }
 
