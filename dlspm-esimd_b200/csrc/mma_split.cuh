@@ -219,6 +219,14 @@ __device__ __forceinline__ void tmem_load_wait(float (&v)[16])
                  : "memory");
 }
 
+// Four columns of this warp's 32 tensor-memory lanes; tmem_store_wait before another thread is told.
+__device__ __forceinline__ void tmem_store4(uint32_t addr, const uint32_t (&v)[4])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
 // Adds 64 columns of an accumulator to the warp's registers (those of them below `columns`).
 __device__ __forceinline__ void tmem_add(float (&acc)[64], uint32_t addr, int columns)
 {
@@ -264,6 +272,13 @@ __device__ __forceinline__ void mma_bf16(uint32_t acc, uint64_t a, uint64_t b, u
         asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(acc),
                      "l"(a), "l"(b), "r"(instruction), "r"(add ? 1u : 0u)
                      : "memory");
+}
+// The first operand from tensor memory (a lane a row, two neighbouring elements of K a word), by a pair of blocks.
+__device__ __forceinline__ void mma_bf16_tmem(uint32_t acc, uint32_t a, uint64_t b, uint32_t instruction, bool add)
+{
+    asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(acc),
+                 "r"(a), "l"(b), "r"(instruction), "r"(add ? 1u : 0u)
+                 : "memory");
 }
 // The barrier (of both blocks of the pair) receives one arrival when all multiplies issued so far are done.
 template <bool PAIR>

@@ -1,6 +1,6 @@
 // SpMM on the tensor cores, for patterns from a few percent nonzeros upwards: the sparse matrix is written
-// out densely, 64 columns at a time, in shared memory and multiplied with B by tcgen05.mma with both operands
-// split into three bf16 parts (mma_split.cuh), six products per fp32 product.
+// out densely, 64 columns at a time, in shared memory and multiplied with B, in tensor memory, by tcgen05.mma with
+// both operands split into three bf16 parts (mma_split.cuh), six products per fp32 product.
 //
 // Why: the row-gather kernel pays one L1 wavefront per FMA instruction and ends at 13 to 17 TFLOP/s of stored
 // entries, the FMA tile kernel at 45 TFLOP/s of dense arithmetic.  Six bf16 products per fp32 product leave
@@ -17,12 +17,25 @@
 // Sums: the product of the two first parts goes to one accumulator, the five small products to another.  The
 // tensor core does not round its sums to nearest, so an accumulator drifts with the number of additions: the
 // main one is added to fp32 registers every 64 columns of the sparse matrix, the small one once per tile (its
-// drift is relative to sums 2^-8 as large).
+// drift is relative to sums 2^-8 as large).  A chunk's main product is multiplied first, so that its sums are fetched
+// while the five small ones are multiplied: one accumulator of each kind is enough, and the other half of the tensor
+// memory holds two stages of B's parts.
+//
+// B comes by cp.async two chunks ahead, as it is, every warp its own part (also across tiles, so that a tile finds its
+// first chunks there), and goes from there split to tensor memory, the first operand of the multiplies.  What bounds the
+// kernel are the operand warps: some 360 instructions each per chunk, 63 % of the issue slots (ncu), most of the rest
+// their dependences; the tensor pipe needs 1500 of the 2300 cycles of a chunk at 10 % nonzeros.  With B's parts in shared memory
+// instead (written once and read by six multiplies, three stages of 72 KiB, 28 KiB left for L1): 2048 x 4096 at 50 %,
+// N = 2048 327 -> 297 us, at 10 % 182 -> 180 us, a batch of 256 problems 5540 -> 5060 us, where the entries of the sparse rows
+// now find their lines in L1.  Measured and left: B's third part in shared memory and three stages (batch 5460 us; with
+// two chunks of raw B 5150 us); rows of B by bulk copies of 512 bytes from one warp (6680 us: it cannot issue them fast
+// enough); the entries by cp.async through rings of 128 per row (6560 us: more instructions); 37 to 70 KiB more for L1
+// (no change).
 //
 // Roles of the 28 warps of a block:
 //   8 sum warps       add finished accumulators to their registers and write C.
 //   16 operand warps  convert 64 rows of B and scatter the matching 64 columns of the sparse rows, eight lanes a
-//                     row, into one of three stages; both come from registers loaded one chunk ahead.
+//                     row, into one of two stages; the entries come from registers loaded one chunk ahead.
 //   1 issuing warp    (of the even block) issues 24 multiplies a chunk; in the odd block it relays barriers.
 //   1 planning warp   lays the next tiles out (problem, place, the rows' entries) for all others.
 // (registers are handed out in groups of four warps; the rest of the last group is idle)
@@ -37,17 +50,20 @@
 namespace dlspm {
 
 constexpr int kMmaChunk = 64;   // columns of the sparse matrix per stage, and per main accumulator
-constexpr int kMmaStages = 3;
+constexpr int kMmaStages = 2;
+constexpr int kMmaRawSlots = 3; // chunks of B fetched at once
 constexpr int kMmaDepth = 5;    // entries of a row fetched ahead, in eights, of the usual build at most (the deep one: 8)
 constexpr int kMmaCols = 128;   // columns of C per block, 256 per pair
 constexpr int kMmaRows = 64;    // rows of the sparse matrix per block at most, 128 per pair
 constexpr int kMmaMarkWords = 2 * kMmaRows / 32;
 constexpr int kMmaSumWarps = 8, kMmaOperandWarps = 16;
 constexpr int kMmaThreads = (kMmaSumWarps + kMmaOperandWarps + 4) * 32;
-constexpr int kMmaDensePlane = kMmaChunk * kMmaCols * 2;   // bytes of one part of one operand in a stage
-constexpr int kMmaSparsePlane = kMmaChunk * kMmaRows * 2;
+constexpr int kMmaSparsePlane = kMmaChunk * kMmaRows * 2;  // bytes of one part of the sparse operand in a stage
+constexpr int kMmaDensePart = kMmaChunk / 2;               // columns of tensor memory of one part of the dense operand
 constexpr int kMmaCheckMost = 8192;  // problems of a launch whose columns may be out of order
-constexpr uint32_t kMmaSmallColumn = 256;  // tensor memory: two main accumulators, then two for the small products
+// Columns of tensor memory: the main accumulator, the one of the small products, two stages of the dense operand.
+constexpr uint32_t kMmaSmallColumn = 128, kMmaDenseColumn = 256, kMmaDenseStage = 128;
+static_assert(3 * kMmaDensePart <= (int)kMmaDenseStage && kMmaDenseColumn + kMmaStages * kMmaDenseStage <= 512, "tensor memory");
 constexpr int kMmaAhead = 4;    // tiles planned ahead
 constexpr int kMmaRing = 16;    // tiles whose marks (rows to compute again) can be alive at once
 constexpr int kMmaRegsLaunch = 72, kMmaRegsSum = 88, kMmaRegsOperand = 72, kMmaRegsIssue = 40;
@@ -79,10 +95,15 @@ struct MmaTile {
 };
 
 struct MmaSmem {
-    unsigned char dense[kMmaStages][3][kMmaDensePlane];    // B: rows of 64 of its columns, 128-byte swizzle
-    unsigned char sparse[kMmaStages][3][kMmaSparsePlane];  // A: rows of 64 columns, 128-byte swizzle
+    union {
+        unsigned char sparse[kMmaStages][3][kMmaSparsePlane];  // A: rows of 64 columns, 128-byte swizzle
+        float part[2 * kMmaRows][kMmaCols];                    // partial sums of a part of K, when the stages are free
+        int2 gather[kMmaThreads];                              // pairs of the row-gather loop
+    };
+    float raw[kMmaRawSlots][kMmaOperandWarps][16 * 32];      // B as it is: 16 rows of 32 columns per warp
     unsigned long long full[kMmaStages], empty[kMmaStages];  // operands written (both blocks) / multiplies done
-    unsigned long long sum_full[2], sum_empty[2];            // accumulators complete / added by all sum warps
+    unsigned long long sum_full, sum_empty;                  // main accumulator complete / added by all sum warps
+    unsigned long long small_full, small_empty;              // the same for the small products, once a tile
     unsigned long long tile_full[kMmaAhead], tile_empty[kMmaAhead];  // tile planned / no longer read
     unsigned long long drain;                                // multiplies still running when a wait ran out
     MmaTile tile[kMmaAhead];
@@ -269,59 +290,104 @@ __device__ __forceinline__ int mma_lower_bound(const int *__restrict__ cols, int
 
 // ---- operand warps ------------------------------------------------------------------------------------
 
-// What a lane needs to read B: byte offsets of its four columns in the chunk row that comes next, 16 rows further
-// and in the last row of B.  (Offsets instead of pointers: the base addresses stay in uniform registers.)
-struct MmaDense {
-    unsigned next, step, last;
-    unsigned d1, d2, d3;  // of the second to fourth column against the first (not WIDE)
+// The fetches of an operand warp's part of B, rows 16 * (warp / 4) .. + 15 of a chunk and columns 32 * (warp % 4) .. + 31 of
+// this block's, two chunks ahead of the conversion and across tiles.  Rows and columns past the end of B repeat its last
+// ones: no entry refers to such a row, and such a column is not stored.
+struct MmaFetch {
+    unsigned n;        // tile
+    int left;          // its chunks to come; < 0: behind the last tile
+    int rows;          // rows of B from this warp's first one of the next chunk on
+    const char *next;  // this lane's first element of the next chunk
+    unsigned row;      // bytes from row to row
 };
 
-// Half a chunk of B, rows k and k + 16 of 32 (k = warp), lane l columns 4l .. 4l + 3 of this block's 128.  Rows and
-// columns past the end of B repeat its last ones: no entry refers to such a row, and such a column is not stored.
-template <bool WIDE>
-__device__ __forceinline__ void mma_load_dense(float4 (&d)[2], MmaDense &b, const float *__restrict__ B)
+__device__ __forceinline__ void copy_async16(uint32_t dst, const void *src)
 {
-    const char *base = reinterpret_cast<const char *>(B);
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-        const unsigned at = min(b.next, b.last);
-        b.next += b.step;
-        if constexpr (WIDE) {
-            d[i] = load_once(reinterpret_cast<const float *>(base + at));
-        } else {
-            d[i].x = __ldg(reinterpret_cast<const float *>(base + at));
-            d[i].y = __ldg(reinterpret_cast<const float *>(base + (at + b.d1)));
-            d[i].z = __ldg(reinterpret_cast<const float *>(base + (at + b.d2)));
-            d[i].w = __ldg(reinterpret_cast<const float *>(base + (at + b.d3)));
-        }
-    }
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async4(uint32_t dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void copy_async_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
 }
 
-// Writes a half split to shared memory at `dst`: 64 columns are one 128-byte row of an 8-row block, the 16-byte
-// units of row r permuted by XOR with r.  Eight-row blocks along K are 1024 bytes apart, the two halves of 64
-// columns 8192.
-__device__ __forceinline__ void mma_store_dense(uint32_t dst, const float4 (&d)[2], unsigned &least)
+// The tile's place in B; false if a wait ran out.
+template <bool TABLE, bool WIDE>
+__device__ __forceinline__ bool mma_fetch_tile(MmaFetch &f, MmaSmem &sm, const MmaArgs &a, int warp, int lane)
 {
+    if (!mbar_wait_suspended(&sm.tile_full[f.n % kMmaAhead], (f.n / kMmaAhead) & 1u, &sm.abort)) return false;
+    const MmaTile &t = sm.tile[f.n % kMmaAhead];
+    const MmaProblem &p = mma_problem_of<TABLE>(t, a);
+    f.left = t.chunks == 0 ? -1 : t.chunks;
+    if (f.left < 0) return true;
+    const int n = min(t.n0 + 32 * (warp & 3) + (WIDE ? 4 * (lane & 7) : lane), p.N - (WIDE ? 4 : 1));
+    const int k = t.chunk0 * kMmaChunk + 16 * (warp >> 2);
+    f.rows = p.K - k;
+    f.row = 4u * (unsigned)p.N;
+    f.next = reinterpret_cast<const char *>(p.B) + 4 * ((size_t)(k + (WIDE ? lane >> 3 : 0)) * (size_t)p.N + (size_t)n);
+    return true;
+}
+
+// Requests the next chunk into `dst`, the warp's part of a slot.
+template <bool TABLE, bool WIDE>
+__device__ __forceinline__ bool mma_fetch(MmaFetch &f, MmaSmem &sm, const MmaArgs &a, int warp, int lane, uint32_t dst)
+{
+    if (f.left == 0) {
+        f.n++;
+        if (!mma_fetch_tile<TABLE, WIDE>(f, sm, a, warp, lane)) return false;
+    }
+    if (f.left > 0) {
+        f.left--;
+        constexpr int kStep = WIDE ? 4 : 1;  // rows a request of the warp covers
+        dst += (WIDE ? 16u : 4u) * (unsigned)lane;
+        const char *src = f.next;
+        if (f.rows >= 16) {
+#pragma unroll
+            for (int i = 0; i < 16 / kStep; i++) {
+                if constexpr (WIDE) copy_async16(dst + 128 * kStep * i, src);
+                else copy_async4(dst + 128 * i, src);
+                src += kStep * f.row;
+            }
+        } else {  // (the last chunk of a problem)
+            const int first = WIDE ? lane >> 3 : 0;
+            for (int i = 0; i < 16; i += kStep) {
+                const char *at = src + (long long)(min(first + i, f.rows - 1) - first) * (long long)f.row;
+                if constexpr (WIDE) copy_async16(dst + 128 * i, at);
+                else copy_async4(dst + 128 * i, at);
+            }
+        }
+        f.next += 64ull * f.row;
+        f.rows -= 64;
+    }
+    copy_async_commit();
+    return true;
+}
+
+// Writes eight rows split to tensor memory: a lane is a column of B, a 32-bit word two neighbouring rows.
+__device__ __forceinline__ void mma_store_dense(uint32_t dst, const float *raw, unsigned &least)
+{
+    float d[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) d[i] = raw[32 * i];
+    uint32_t x1[4], x2[4], x3[4];
     float small = 1.f;
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
-        small = min3_magnitude(small, d[i].x, d[i].y);
-        small = min3_magnitude(small, d[i].z, d[i].w);
-        uint32_t x1, x2, x3, y1, y2, y3;
-        split_pair(d[i].x, d[i].y, x1, x2, x3);
-        split_pair(d[i].z, d[i].w, y1, y2, y3);
-        store_shared(dst + i * 2048, x1, y1);
-        store_shared(dst + i * 2048 + kMmaDensePlane, x2, y2);
-        store_shared(dst + i * 2048 + 2 * kMmaDensePlane, x3, y3);
+    for (int i = 0; i < 4; i++) {
+        small = min3_magnitude(small, d[2 * i], d[2 * i + 1]);
+        split_pair(d[2 * i], d[2 * i + 1], x1[i], x2[i], x3[i]);
     }
+    __syncwarp();
+    tmem_store4(dst, x1);
+    tmem_store4(dst + kMmaDensePart, x2);
+    tmem_store4(dst + 2 * kMmaDensePart, x3);
     if (small < kSplitSmall) {  // a zero, or a number that cannot be split
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
-            least = split_magnitude(d[i].x, least);
-            least = split_magnitude(d[i].y, least);
-            least = split_magnitude(d[i].z, least);
-            least = split_magnitude(d[i].w, least);
-        }
+        for (int i = 0; i < 8; i++) least = split_magnitude(d[i], least);
     }
 }
 
@@ -362,8 +428,9 @@ __device__ __forceinline__ void mma_mark_again(MmaSmem &sm, int ring, int bit, u
 // One tile: every lane group of eight lanes owns one row of it, 4 * warp + group, and walks it once.  DEPTH: entries
 // of a row fetched ahead, in eights.  CHECK: columns may be out of order (a prepared batch looked at them when it was
 // made).
-template <int DEPTH, bool TABLE, bool CHECK, bool WIDE>
-__device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, const MmaTile &t, unsigned rank, int warp, int lane, MmaStage &st)
+template <int DEPTH, bool TABLE, bool WIDE, bool CHECK>
+__device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, const MmaTile &t, unsigned rank, int warp, int lane, MmaStage &st,
+                                                 MmaFetch &f, unsigned &slot)
 {
     volatile int *abort = &sm.abort;
     const MmaProblem &p = mma_problem_of<TABLE>(t, a);
@@ -378,30 +445,23 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
         if (part + 1 < a.splits) end = mma_lower_bound(p.cols, first, stop, (t.chunk0 + t.chunks) * kMmaChunk, l8);
     }
     int k0 = t.chunk0 * kMmaChunk;
-    MmaDense b;
-    {
-        const int n = min(t.n0 + 4 * lane, WIDE ? p.N - 4 : p.N - 1);
-        b.next = 4u * ((unsigned)(k0 + warp) * (unsigned)p.N + (unsigned)n);
-        b.step = 64u * (unsigned)p.N;
-        b.last = 4u * ((unsigned)(p.K - 1) * (unsigned)p.N + (unsigned)n);
-        if constexpr (!WIDE) {
-            b.d1 = 4u * (unsigned)min(1, p.N - 1 - n);
-            b.d2 = 4u * (unsigned)min(2, p.N - 1 - n);
-            b.d3 = 4u * (unsigned)min(3, p.N - 1 - n);
-        }
-    }
-    const uint32_t dense_at = smem_u32(&sm.dense[0][0][0]) + (lane >> 4) * 8192 + (warp >> 3) * 1024 + (warp & 7) * 128 +
-                              ((((lane & 15) >> 1) ^ (warp & 7)) << 4) + (lane & 1) * 8;
+    const uint32_t dense_at = sm.tmem + ((uint32_t)(warp & 3) << 21) + kMmaDenseColumn + 8u * (unsigned)(warp >> 2);
     const uint32_t sparse_at = smem_u32(&sm.sparse[0][0][0]) + own * 128;
-    float4 dense[2];
     unsigned least = 0xffffffffu;
     bool bad = false, ok = true;  // bad: the lane group's row has columns out of order
     // One chunk: its entries are in (c, v), the next chunk's are fetched into (cn, vn).
     auto step = [&](int (&c)[DEPTH], float (&v)[DEPTH], int (&cn)[DEPTH], float (&vn)[DEPTH]) {
-        ok = mbar_wait_suspended(&sm.empty[st.stage], st.parity ^ 1u, abort);  // passes at once in the first round
+        copy_async_wait<1>();
+        __syncwarp();  // this chunk has landed, and the one before it has been read
+        const float *raw = sm.raw[slot][warp] + lane;
+        const unsigned behind = slot == 0u ? kMmaRawSlots - 1u : slot - 1u;
+        ok = mma_fetch<TABLE, WIDE>(f, sm, a, warp, lane, smem_u32(sm.raw[behind][warp])) &&
+             mbar_wait_suspended(&sm.empty[st.stage], st.parity ^ 1u, abort);  // passes at once in the first round
+        slot = slot == kMmaRawSlots - 1u ? 0u : slot + 1u;
         if (!ok) return;
+        tmem_fence_after();
         const uint32_t row = sparse_at + st.stage * (3 * kMmaSparsePlane);
-        const uint32_t dst = dense_at + st.stage * (3 * kMmaDensePlane);
+        const uint32_t dst = dense_at + st.stage * kMmaDenseStage;
         int turns = 0;  // eights of entries at hand of which some row uses one
         if (row_warp) {
             // this warp's four rows: zeros in all three parts
@@ -439,8 +499,7 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
             }
             if constexpr (DEPTH <= 2) mma_load_pairs(cn, vn, cursor + l8, end, p);
         }
-        mma_store_dense(dst, dense, least);
-        mma_load_dense<WIDE>(dense, b, p.B);
+        mma_store_dense(dst, raw, least);
         if (row_warp) {
             int last = -1;  // column in front of the first entry at hand (entries of earlier chunks are in order)
 #pragma unroll
@@ -459,8 +518,7 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
             }
             if constexpr (DEPTH > 2) mma_load_pairs(c, v, cursor + l8, end, p);
         }
-        mma_store_dense(dst + 4096, dense, least);
-        mma_load_dense<WIDE>(dense, b, p.B);
+        mma_store_dense(dst + 4, raw + 8 * 32, least);
         k0 += kMmaChunk;
     };
     // Hands a stage over; `marks`: the tile's last one.
@@ -474,6 +532,8 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
                     for (int r = lane; r < 2 * t.rows; r += 32) mma_mark_again(sm, t.ring, r, rank);
             }
         }
+        tmem_store_wait();
+        tmem_fence_before();
         fence_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.full[st.stage]);
@@ -482,7 +542,6 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
     int c0[DEPTH];
     float v0[DEPTH];
     mma_load_pairs(c0, v0, cursor + l8, end, p);
-    mma_load_dense<WIDE>(dense, b, p.B);
     if constexpr (DEPTH <= 2) {
         // two chunks a turn with the register sets exchanged: copying one to the other would wait for its loads
         int c1[DEPTH];
@@ -512,23 +571,30 @@ template <bool TABLE, bool WIDE, bool DEEP, bool CHECK>
 __device__ __forceinline__ bool mma_operands(MmaSmem &sm, const MmaArgs &a, unsigned rank, int warp, int lane)
 {
     MmaStage st{0, 0u};
-    for (MmaWalk walk;; walk.n++) {
-        if (!walk.wait(sm)) return false;
+    MmaFetch f;
+    f.n = 0u;
+    unsigned slot = 0u;
+    bool ok = mma_fetch_tile<TABLE, WIDE>(f, sm, a, warp, lane);
+#pragma unroll
+    for (int i = 0; i + 1 < kMmaRawSlots; i++) ok = ok && mma_fetch<TABLE, WIDE>(f, sm, a, warp, lane, smem_u32(sm.raw[i][warp]));
+    for (MmaWalk walk; ok; walk.n++) {
+        ok = walk.wait(sm);
+        if (!ok) break;
         const MmaTile &t = walk.tile(sm);
-        if (t.chunks == 0) return true;
-        bool ok;
+        if (t.chunks == 0) break;
         if constexpr (DEEP) {
-            ok = mma_operand_tile<8, TABLE, CHECK, WIDE>(sm, a, t, rank, warp, lane, st);
+            ok = mma_operand_tile<8, TABLE, WIDE, CHECK>(sm, a, t, rank, warp, lane, st, f, slot);
         } else {
             const int depth = mma_problem_of<TABLE>(t, a).depth;
-            if (depth == 1) ok = mma_operand_tile<1, TABLE, CHECK, WIDE>(sm, a, t, rank, warp, lane, st);
-            else if (depth == 2) ok = mma_operand_tile<2, TABLE, CHECK, WIDE>(sm, a, t, rank, warp, lane, st);
-            else ok = mma_operand_tile<5, TABLE, CHECK, WIDE>(sm, a, t, rank, warp, lane, st);
+            if (depth == 1) ok = mma_operand_tile<1, TABLE, WIDE, CHECK>(sm, a, t, rank, warp, lane, st, f, slot);
+            else if (depth == 2) ok = mma_operand_tile<2, TABLE, WIDE, CHECK>(sm, a, t, rank, warp, lane, st, f, slot);
+            else ok = mma_operand_tile<5, TABLE, WIDE, CHECK>(sm, a, t, rank, warp, lane, st, f, slot);
         }
-        if (!ok) return false;
         __syncwarp();
-        if (lane == 0) walk.done(sm);
+        if (ok && lane == 0) walk.done(sm);
     }
+    copy_async_wait<0>();
+    return ok;
 }
 
 // ---- issuing warp (of the even block) ----------------------------------------------------------
@@ -542,37 +608,44 @@ __device__ __forceinline__ bool mma_issue(MmaSmem &sm, unsigned rank, bool issue
     const uint32_t tmem = sm.tmem;
     // parts (of B, of A) of the five small products
     const int part_b[5] = {2, 1, 1, 0, 0}, part_a[5] = {0, 1, 0, 2, 1};
-    const uint64_t dense0 = mma_descriptor(smem_u32(&sm.dense[0][0][0]), 8192, 1024, kSwizzle128);
     const uint64_t sparse0 = mma_descriptor(smem_u32(&sm.sparse[0][0][0]), 0, 1024, kSwizzle128);
-    constexpr uint64_t kDense = kMmaDensePlane >> 4, kSparse = kMmaSparsePlane >> 4;
-    unsigned g = 0;  // chunks (one main accumulator each) so far
+    constexpr uint64_t kSparse = kMmaSparsePlane >> 4;
+    const uint32_t main = tmem, small = tmem + kMmaSmallColumn;
+    unsigned g = 0;  // chunks so far
     for (MmaWalk walk;; walk.n++) {
         if (!walk.wait(sm)) return false;
         const int chunks = walk.tile(sm).chunks, rows = walk.tile(sm).rows;
         __syncwarp();
         if (lane == 0) walk.done(sm);
         if (chunks == 0) return true;
-        const uint32_t instruction = mma_instruction(256, 2 * rows, true, false);
-        const uint32_t small = tmem + kMmaSmallColumn + (walk.n & 1u) * 128u;
+        const uint32_t instruction = mma_instruction(256, 2 * rows, false, false);
         for (int c = 0; c < chunks; c++, g++) {
             const int s = (int)(g % kMmaStages);
-            // (the accumulator of the small products was read together with the tile's last main one)
-            if (g >= 2u && !mbar_wait_suspended(&sm.sum_empty[g & 1u], ((g >> 1) - 1u) & 1u, abort)) return false;
             if (!mbar_wait_suspended(&sm.full[s], (g / kMmaStages) & 1u, abort)) return false;
+            if (!mbar_wait_suspended(&sm.sum_empty, (g & 1u) ^ 1u, abort)) return false;  // passes at once the first time
             tmem_fence_after();
-            const uint32_t main = tmem + (g & 1u) * 128u;
-            const uint64_t dense = dense0 + s * (3 * kDense), sparse = sparse0 + s * (3 * kSparse);
+            const uint32_t dense = tmem + kMmaDenseColumn + s * kMmaDenseStage;
+            const uint64_t sparse = sparse0 + s * (3 * kSparse);
             if (issuer) {
 #pragma unroll
-                for (int ks = 0; ks < kMmaChunk / 16; ks++) {
-                    const uint64_t d = dense + ks * (2048 >> 4), x = sparse + ks * (32 >> 4);
+                for (int ks = 0; ks < kMmaChunk / 16; ks++)
+                    mma_bf16_tmem(main, dense + ks * 8, sparse + ks * (32 >> 4), instruction, ks > 0);
+                mma_commit<true>(&sm.sum_full, pair_mask);
+            }
+            __syncwarp();
+            if (c == 0) {  // the small sums of the tile before have been read
+                if (!mbar_wait_suspended(&sm.small_empty, (walk.n & 1u) ^ 1u, abort)) return false;
+                tmem_fence_after();
+            }
+            if (issuer) {
+#pragma unroll
+                for (int ks = 0; ks < kMmaChunk / 16; ks++)
 #pragma unroll
                     for (int j = 0; j < 5; j++)
-                        mma_bf16<true>(small, d + part_b[j] * kDense, x + part_a[j] * kSparse, instruction, c + j + ks > 0);
-                    mma_bf16<true>(main, d, x, instruction, ks > 0);
-                }
+                        mma_bf16_tmem(small, dense + part_b[j] * kMmaDensePart + ks * 8, sparse + part_a[j] * kSparse + ks * (32 >> 4),
+                                      instruction, c + j + ks > 0);
                 mma_commit<true>(&sm.empty[s], pair_mask);
-                mma_commit<true>(&sm.sum_full[g & 1u], pair_mask);
+                if (c + 1 == chunks) mma_commit<true>(&sm.small_full, pair_mask);
             }
             __syncwarp();
         }
@@ -586,9 +659,9 @@ __device__ __forceinline__ bool mma_issue(MmaSmem &sm, unsigned rank, bool issue
 __device__ __forceinline__ bool mma_relay(MmaSmem &sm, unsigned rank, bool sums)
 {
     volatile int *abort = &sm.abort;
-    const unsigned slots = sums ? 2u : (unsigned)kMmaStages;
-    unsigned long long *own = sums ? sm.sum_empty : sm.full;
-    const uint32_t other = cluster_map(smem_u32(own), rank ^ 1u);
+    const unsigned slots = sums ? 1u : (unsigned)kMmaStages;
+    unsigned long long *own = sums ? &sm.sum_empty : sm.full;
+    const uint32_t other = cluster_map(smem_u32(own), rank ^ 1u), other_small = cluster_map(smem_u32(&sm.small_empty), rank ^ 1u);
     unsigned g = 0;
     for (MmaWalk walk;; walk.n++) {
         if (!walk.wait(sm)) return false;
@@ -597,7 +670,15 @@ __device__ __forceinline__ bool mma_relay(MmaSmem &sm, unsigned rank, bool sums)
         if (chunks == 0) return true;
         for (int c = 0; c < chunks; c++, g++) {
             if (!mbar_wait_suspended(&own[g % slots], (g / slots) & 1u, abort)) return false;
+            tmem_fence_after();
+            tmem_fence_before();
             mbar_arrive_cluster(other + (g % slots) * 8u);
+        }
+        if (sums) {
+            if (!mbar_wait_suspended(&sm.small_empty, walk.n & 1u, abort)) return false;
+            tmem_fence_after();
+            tmem_fence_before();
+            mbar_arrive_cluster(other_small);
         }
     }
 }
@@ -657,20 +738,24 @@ __device__ __forceinline__ bool mma_sums(MmaSmem &sm, const MmaArgs &a, unsigned
 #pragma unroll
         for (int j = 0; j < kMmaRows; j++) acc[j] = 0.f;
         for (int i = 0; i < chunks; i++, q++) {
-            if (!mbar_wait_suspended(&sm.sum_full[q & 1u], (q >> 1) & 1u, abort)) return false;
+            if (!mbar_wait_suspended(&sm.sum_full, q & 1u, abort)) return false;
             tmem_fence_after();
-            tmem_add(acc, tmem + (q & 1u) * 128u, tile_rows - half);
-            if (i + 1 == chunks) tmem_add(acc, tmem + kMmaSmallColumn + (walk.n & 1u) * 128u, tile_rows - half);
+            tmem_add(acc, tmem, tile_rows - half);
             tmem_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.sum_empty[q & 1u]);
+            if (lane == 0) mbar_arrive(&sm.sum_empty);
         }
+        if (!mbar_wait_suspended(&sm.small_full, walk.n & 1u, abort)) return false;
+        tmem_fence_after();
+        tmem_add(acc, tmem + kMmaSmallColumn, tile_rows - half);
+        tmem_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.small_empty);
         if (a.splits > 1) {
             // partial sums to shared memory (the stages are free: this was the last tile); the blocks of the
             // cluster that hold the same columns add them up behind a cluster barrier, in mma_combine
-            float *part = reinterpret_cast<float *>(&sm.dense[0][0][0]);
 #pragma unroll
-            for (int j = 0; j < kMmaRows; j++) part[(half + j) * kMmaCols + 32 * quarter + lane] = acc[j];
+            for (int j = 0; j < kMmaRows; j++) sm.part[half + j][32 * quarter + lane] = acc[j];
             return true;
         }
         const int ring = t.ring;
@@ -709,7 +794,7 @@ __device__ __forceinline__ void mma_combine(MmaSmem &sm, const MmaArgs &a, unsig
     const int tile_rows = 2 * t.rows, part = (int)(rank >> 1);
     const int per = (tile_rows + a.splits - 1) / a.splits;
     const int first = part * per, last = min(min(first + per, tile_rows), p.M - t.row0);
-    const uint32_t sums = smem_u32(&sm.dense[0][0][0]);
+    const uint32_t sums = smem_u32(&sm.part[0][0]);
     uint32_t again = 0;  // lane w < 4: word w of the marks of all parts
     if (lane < kMmaMarkWords)
         for (int s = 0; s < a.splits; s++)
@@ -786,10 +871,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_c
             mbar_init(&sm.full[s], kMmaOperandWarps + (rank & 1u ? 0u : 1u));  // even block: plus the odd one's relay
             mbar_init(&sm.empty[s], 1);
         }
-        for (int b = 0; b < 2; b++) {
-            mbar_init(&sm.sum_full[b], 1);
-            mbar_init(&sm.sum_empty[b], kMmaSumWarps + (rank & 1u ? 0u : 1u));
-        }
+        mbar_init(&sm.sum_full, 1);
+        mbar_init(&sm.sum_empty, kMmaSumWarps + (rank & 1u ? 0u : 1u));
+        mbar_init(&sm.small_full, 1);
+        mbar_init(&sm.small_empty, kMmaSumWarps + (rank & 1u ? 0u : 1u));
         for (int n = 0; n < kMmaAhead; n++) {
             mbar_init(&sm.tile_full[n], 1);
             mbar_init(&sm.tile_empty[n], kMmaSumWarps + kMmaOperandWarps + (rank & 1u ? 2u : 1u));  // and the issuing warp or both relays
@@ -817,7 +902,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_c
     tmem_fence_after();
     bool ok = true, done = false;
     if constexpr (CHECK) {
-        int2 *stage = reinterpret_cast<int2 *>(&sm.dense[0][0][0]) + warp * 32;
+        int2 *stage = sm.gather + warp * 32;
         if constexpr (TABLE) {
             for (int i = threadIdx.x; i < (a.count + 31) / 32; i += kMmaThreads) sm.unsorted[i] = 0u;
             __syncthreads();
