@@ -98,6 +98,30 @@ def test_lone_launches(pkg, oracle, ctx, dev, M, K, N, density, order):
     check(oracle, ro, ci, vals, B, M, N, lone_run(ctx, dev, M, K, N, ro, ci, vals, B, plan=True))
 
 
+@pytest.mark.parametrize("M,K,N", [(12900, 200, 1028), (130, 4097, 260)])
+def test_order_of_columns_is_seen_in_every_tile_of_a_lone_launch(pkg, oracle, ctx, dev, M, K, N):
+    """More tiles for every pair of blocks than are planned ahead, and one tile in parts of K; empty rows among them.
+    Columns repeated at the start, in the middle and at the end of rows, and rows that run backwards."""
+    seed = M
+    rng = np.random.default_rng(seed)
+    lengths = rng.integers(K // 4, K // 2, M)
+    lengths[rng.integers(0, M, M // 8)] = 0
+    lengths[:3] = 0
+    lengths[-1] = 0
+    ro, ci = csr_from_lengths(pkg, K, [int(x) for x in lengths], seed=seed)
+    for n, i in enumerate(i for i in range(M) if lengths[i]):
+        at = {0: 0, 1: int(lengths[i]) // 2, 2: int(lengths[i]) - 2}.get(n % 11)
+        if at is not None:
+            ci[ro[i] + at + 1] = ci[ro[i] + at]
+        elif n % 11 == 3:
+            ci[ro[i]:ro[i + 1]] = ci[ro[i]:ro[i + 1]][::-1].copy()
+    vals = pkg.gen_dense_host(int(ci.size), seed, 2)
+    B = dense(pkg, K, N, seed, 10)
+    out = lone_run(ctx, dev, M, K, N, ro, ci, vals, B)
+    check(oracle, ro, ci, vals, B, M, N, out)
+    assert (out[lengths == 0] == 0).all()
+
+
 def test_many_tiles_per_cluster(pkg, oracle, ctx, dev):
     """More tiles for every pair of blocks than are planned ahead, of problems of different sizes, as a prepared batch
     (columns known to ascend) and as a one-shot call (columns checked)."""
