@@ -27,6 +27,7 @@ namespace {
 
 constexpr int kWarps = 8;
 
+// EXACT: a row is exactly G * R chunks (see launch_fast).
 // CAP: second builds with a register cap, chosen per launch.
 //  - one chunk per lane (d <= 32): 32 registers for eight resident blocks instead of six.  It pays
 //    when it saves a wave of thread blocks: 8192 rows are 1.15 waves of six blocks per SM but fit
@@ -35,7 +36,7 @@ constexpr int kWarps = 8;
 //  - 32 lanes x four chunks (d = 260..512): 64 registers for four resident blocks instead of two:
 //    1.3 to 1.5x faster once the pattern has more rows than the uncapped build keeps resident
 //    (8192 x 2048, d = 512: 637 -> 479 us), 12 % slower below that.
-template <int G, int R, int MODE, bool CAP = false, bool WIDE = false>
+template <int G, int R, int MODE, bool CAP = false, bool WIDE = false, bool EXACT = false>
 __global__ void __launch_bounds__(kWarps * 32, CAP ? (G == 8 ? 8 : 4) : 0)
 fused_rows_kernel(const int *__restrict__ row_offsets, const int *__restrict__ cols,
                   const float *__restrict__ c, const float *__restrict__ b, const float *__restrict__ d,
@@ -54,7 +55,7 @@ fused_rows_kernel(const int *__restrict__ row_offsets, const int *__restrict__ c
 #pragma unroll
     for (int r = 0; r < R; r++) acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
     float run_max = -INFINITY, run_sum = 0.f;
-    fused_row_passes<G, R, MODE, WIDE>(cols, q, reinterpret_cast<const float4 *>(b), reinterpret_cast<const float4 *>(d),
+    fused_row_passes<G, R, MODE, WIDE, EXACT>(cols, q, reinterpret_cast<const float4 *>(b), reinterpret_cast<const float4 *>(d),
                                        chunks, __ldg(row_offsets + row), __ldg(row_offsets + row + 1), 32, scale, lane,
                                        acc, run_max, run_sum);
     if constexpr (MODE == kSoftmax) {
@@ -407,6 +408,20 @@ void launch_fast(const int *ro, const int *ci, const float *c, const float *b, c
     if constexpr (G == 4 && R == 2) {
         if (wide) {  // rows of 32 floats, 32-byte aligned operands, a long launch: 256-bit loads
             launch_overlapped(fused_rows_kernel<G, R, MODE, false, true>, dlspm_ceil_div(M, warps), warps * 32, 0, st, ro, ci, c, b, d, e, M, chunks, scale);
+            return;
+        }
+    }
+    if constexpr (G == 8 && R >= 2) {
+        // Rows of exactly 64 or 128 floats: full passes without a test per nonzero and chunk, in fewer instructions and with
+        // their loads side by side (the kernel is bound by the latency of two dependent gathers a pass).  Tests / none:
+        // 4096 rows of a band and 5 %, d = 64 39.3 / 34.5 us, attention 16384 rows, 1 %, d = 128 210 / 197 us, 8000 rows, 2 %,
+        // d = 64 60.0 / 52.8 us, 2000 rows, d = 128 26.5 / 25.1 us.  Left with the tests: other widths (a build that asks
+        // for the chunks only, d = 100 43.7 / 46.4 us, d = 60 207 / 211 us), shared rows (500 rows 8.7 / 9.6 us), the layouts
+        // of other widths (20 registers more), and the SDDMM kernel (4096 rows at 10 %, inner dimension 64 29.5 / 30.1 us,
+        // 128 51.7 / 56.7 us at the registers of the build with the tests, more without that bound).  Held to 80 registers
+        // by the launch bounds instead of left alone (80 as well), d = 128 takes 213 us.
+        if (chunks == G * R) {
+            launch_overlapped(fused_rows_kernel<G, R, MODE, false, false, true>, dlspm_ceil_div(M, warps), warps * 32, 0, st, ro, ci, c, b, d, e, M, chunks, scale);
             return;
         }
     }

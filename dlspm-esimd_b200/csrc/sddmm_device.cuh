@@ -146,7 +146,7 @@ __device__ __forceinline__ float sddmm_pass(const float4 (&a)[R], const float4 *
 // lanes, where with blocks of G the first group worked through min(cnt, G) nonzeros alone.
 // Returns, on lane g*G + t, the dot product of nonzero sddmm_dealt_slot(G, g, t) of the pass.  Every
 // dot product is summed in the same order as in sddmm_pass, so the two give the same bits.
-template <int G, int R>
+template <int G, int R, bool FULL = false>
 __device__ __forceinline__ float sddmm_pass_dealt(const float4 (&a)[R], const float4 *__restrict__ rhs4,
                                                   int chunks, int col, int g, int t)
 {
@@ -156,12 +156,12 @@ __device__ __forceinline__ float sddmm_pass_dealt(const float4 (&a)[R], const fl
     for (int k = 0; k < G; k++) {
         const int c = __shfl_sync(0xffffffffu, col, k * NG + g);
         float acc = 0.f;
-        if (c >= 0) {
-            const float4 *brow = rhs4 + (size_t)c * (size_t)chunks;
+        if (FULL || c >= 0) {
+            const float4 *brow = rhs4 + (size_t)c * (size_t)(FULL ? G * R : chunks);
 #pragma unroll
             for (int r = 0; r < R; r++) {
                 const int idx = r * G + t;
-                if (idx < chunks) acc = dot4(a[r], __ldg(brow + idx), acc);
+                if (FULL || idx < chunks) acc = dot4(a[r], __ldg(brow + idx), acc);
             }
         }
         part[k] = acc;

@@ -56,6 +56,34 @@ def test_feature_dimensions(pkg, oracle, ctx, dev, N, softmax):
           run_attention(pkg, ctx, dev, M, K, N, ro, ci, q, k, v, scale, softmax))
 
 
+@pytest.mark.parametrize("N", [60, 64, 124, 128])
+@pytest.mark.parametrize("mode", ["plain", "scaled", "softmax"])
+def test_full_passes_of_unshared_rows(pkg, oracle, ctx, dev, N, mode):
+    """Enough rows that none is shared between warps, lengths around multiples of the 32 nonzeros of a pass: full passes
+    of rows of exactly 64 and 128 floats run without a test per nonzero, widths below with it.  Rows of k and v that no
+    pattern row refers to hold infinities."""
+    K = 200
+    edges = [0, 1, 31, 32, 33, 63, 64, 65, 95, 96, 97, 32, 64]
+    lengths = [edges[i % len(edges)] for i in range(5400)]
+    M = len(lengths)
+    ro, ci = csr_from_lengths(pkg, K - 2, lengths, seed=N)
+    q = dense(pkg, M, N, N, 11, kind=pkg.KIND_NORMAL)
+    k = dense(pkg, K, N, N, 12, kind=pkg.KIND_NORMAL)
+    v = dense(pkg, K, N, N, 13)
+    k[-2:], v[-2:] = np.inf, -np.inf
+    scale = 1.0 if mode == "plain" else 1.0 / np.sqrt(N)
+    if mode == "plain":
+        import torch
+
+        buf = torch.full((M * N,), float("nan"), device=dev)
+        ctx.fused(M, K, N, int(ci.size), *(to_dev(x, dev) for x in (ro, ci, q, k, v)), buf)
+        torch.cuda.synchronize()
+        out = buf.cpu().numpy().reshape(M, N)
+    else:
+        out = run_attention(pkg, ctx, dev, M, K, N, ro, ci, q, k, v, scale, mode == "softmax")
+    check(oracle, ro, ci, q, k[:-2], v[:-2], M, N, scale, mode == "softmax", out)
+
+
 @pytest.mark.parametrize("N", [64, 50])
 def test_row_length_edges_and_empty_rows(pkg, oracle, ctx, dev, N):
     K = 140
