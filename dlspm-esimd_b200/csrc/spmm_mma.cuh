@@ -38,8 +38,7 @@
 //                     row, into one of two stages; the entries come from registers loaded one chunk ahead.
 //   1 issuing warp    (of the even block) issues 24 multiplies a chunk; in the odd block it relays barriers.
 //   1 planning warp   lays the next tiles out (problem, place, the rows' entries) for all others.
-//   1 more warp       looks, with the planning one, whether columns ascend (launches of one problem).
-// (registers are handed out in groups of four warps; in launches over a table the last one is idle)
+// (registers are handed out in groups of four warps; the rest of the last group is idle)
 //
 // Rows whose columns are not strictly ascending, tiles with magnitudes that cannot be split, and sums that are
 // not finite are computed again from the CSR arrays with fp32 multiply-adds, so that such input gives what the
@@ -66,7 +65,6 @@ constexpr int kMmaCheckMost = 8192;  // problems of a launch whose columns may b
 constexpr uint32_t kMmaSmallColumn = 128, kMmaDenseColumn = 256, kMmaDenseStage = 128;
 static_assert(3 * kMmaDensePart <= (int)kMmaDenseStage && kMmaDenseColumn + kMmaStages * kMmaDenseStage <= 512, "tensor memory");
 constexpr int kMmaAhead = 4;    // tiles planned ahead
-constexpr int kMmaLookWarps = 2;
 constexpr int kMmaRing = 16;    // tiles whose marks (rows to compute again) can be alive at once
 constexpr int kMmaRegsLaunch = 72, kMmaRegsSum = 88, kMmaRegsOperand = 72, kMmaRegsIssue = 40;
 static_assert(kMmaThreads * kMmaRegsLaunch <= 65536 &&
@@ -106,7 +104,6 @@ struct MmaSmem {
     unsigned long long full[kMmaStages], empty[kMmaStages];  // operands written (both blocks) / multiplies done
     unsigned long long sum_full, sum_empty;                  // main accumulator complete / added by all sum warps
     unsigned long long small_full, small_empty;              // the same for the small products, once a tile
-    unsigned long long checked[kMmaAhead];                   // the order of a tile's columns has been looked at, by both blocks
     unsigned long long tile_full[kMmaAhead], tile_empty[kMmaAhead];  // tile planned / no longer read
     unsigned long long drain;                                // multiplies still running when a wait ran out
     MmaTile tile[kMmaAhead];
@@ -429,9 +426,9 @@ __device__ __forceinline__ void mma_mark_again(MmaSmem &sm, int ring, int bit, u
 }
 
 // One tile: every lane group of eight lanes owns one row of it, 4 * warp + group, and walks it once.  DEPTH: entries
-// of a row fetched ahead, in eights.  ORDER: looks whether columns ascend (a prepared batch looked when it was made, the
-// launch of one problem leaves it to mma_look).
-template <int DEPTH, bool TABLE, bool WIDE, bool ORDER>
+// of a row fetched ahead, in eights.  CHECK: columns may be out of order (a prepared batch looked at them when it was
+// made).
+template <int DEPTH, bool TABLE, bool WIDE, bool CHECK>
 __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, const MmaTile &t, unsigned rank, int warp, int lane, MmaStage &st,
                                                  MmaFetch &f, unsigned &slot)
 {
@@ -487,11 +484,11 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
                 const int q = cursor + l8;
                 bool take = false;
                 if (more && q < end) {
-                    const int col = __ldg(p.cols + q), before = ORDER ? __ldg(p.cols + q - 1) : -1;
+                    const int col = __ldg(p.cols + q), before = CHECK ? __ldg(p.cols + q - 1) : -1;
                     const float x = __ldg(p.values + q);
                     take = (unsigned)(col - k0) < (unsigned)kMmaChunk;
                     if (take) {
-                        if (ORDER && col <= before) bad = true;
+                        if (CHECK && col <= before) bad = true;
                         least = split_magnitude(x, least);
                         mma_store_entry(row, col - k0, x, swizzle, true);
                     }
@@ -510,7 +507,7 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
                 if (DEPTH > 5 && h >= turns) break;  // the whole warp
                 const int col = c[h] - k0;
                 const bool live = (unsigned)col < (unsigned)kMmaChunk;
-                if constexpr (ORDER) {
+                if constexpr (CHECK) {
                     int before = __shfl_up_sync(0xffffffffu, col, 1, 8);
                     if (l8 == 0) before = last;
                     if (h + 1 < DEPTH) last = __shfl_sync(0xffffffffu, col, 7, 8);
@@ -527,7 +524,7 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
     // Hands a stage over; `marks`: the tile's last one.
     auto hand_over = [&](bool marks) {
         if (marks) {
-            if (ORDER && cursor != end) bad = true;  // entries out of order were never reached
+            if (CHECK && cursor != end) bad = true;  // entries out of order were never reached
             const bool all = __any_sync(0xffffffffu, least < kSplitLeast);
             if (__any_sync(0xffffffffu, bad) || all) {
                 if (bad && own < t.rows) mma_mark_again(sm, t.ring, (int)(rank & 1u) * t.rows + own, rank);
@@ -570,7 +567,7 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
     return true;
 }
 
-template <bool TABLE, bool WIDE, bool DEEP, bool ORDER>
+template <bool TABLE, bool WIDE, bool DEEP, bool CHECK>
 __device__ __forceinline__ bool mma_operands(MmaSmem &sm, const MmaArgs &a, unsigned rank, int warp, int lane)
 {
     MmaStage st{0, 0u};
@@ -586,84 +583,18 @@ __device__ __forceinline__ bool mma_operands(MmaSmem &sm, const MmaArgs &a, unsi
         const MmaTile &t = walk.tile(sm);
         if (t.chunks == 0) break;
         if constexpr (DEEP) {
-            ok = mma_operand_tile<8, TABLE, WIDE, ORDER>(sm, a, t, rank, warp, lane, st, f, slot);
+            ok = mma_operand_tile<8, TABLE, WIDE, CHECK>(sm, a, t, rank, warp, lane, st, f, slot);
         } else {
             const int depth = mma_problem_of<TABLE>(t, a).depth;
-            if (depth == 1) ok = mma_operand_tile<1, TABLE, WIDE, ORDER>(sm, a, t, rank, warp, lane, st, f, slot);
-            else if (depth == 2) ok = mma_operand_tile<2, TABLE, WIDE, ORDER>(sm, a, t, rank, warp, lane, st, f, slot);
-            else ok = mma_operand_tile<5, TABLE, WIDE, ORDER>(sm, a, t, rank, warp, lane, st, f, slot);
+            if (depth == 1) ok = mma_operand_tile<1, TABLE, WIDE, CHECK>(sm, a, t, rank, warp, lane, st, f, slot);
+            else if (depth == 2) ok = mma_operand_tile<2, TABLE, WIDE, CHECK>(sm, a, t, rank, warp, lane, st, f, slot);
+            else ok = mma_operand_tile<5, TABLE, WIDE, CHECK>(sm, a, t, rank, warp, lane, st, f, slot);
         }
         __syncwarp();
         if (ok && lane == 0) walk.done(sm);
     }
     copy_async_wait<0>();
     return ok;
-}
-
-// ---- looking at the order of columns (launches of one problem) ---------------------------------------------------
-
-// Two warps, of which the first also plans the tiles.  The rows of a block's part of a tile lie one behind the other in the
-// CSR arrays, so their entries are walked as one run, whose descents must be starts of rows; another one marks its row.
-// (The operand warps hold the entries anyway, but bind the kernel, and the comparisons took them 32 of 390 instructions a
-// chunk: 8192 x 2048 at 10 %, N = 256 53.5 -> 52.0 us, 1024 x 4096, N = 1024 56.6 -> 55.3 us, 2048 x 4096 at 50 %, N = 2048 297 ->
-// 301 us.  The sum warps cannot take them over: 59.8 and 62.7 us, their latency holds up the multiplies.)
-template <bool TABLE, bool CHECK>
-__device__ __forceinline__ bool mma_look(MmaSmem &sm, const MmaArgs &a, unsigned rank, int which, int lane, MmaPlan &plan, bool more)
-{
-    constexpr int kAtOnce = 12;  // entries of a lane in flight
-    volatile int *abort = &sm.abort;
-    for (MmaWalk walk;; walk.n++) {
-        if (which == 0 && more) {
-            const unsigned n = walk.n + 1u;
-            if (!mbar_wait_suspended(&sm.tile_empty[n % kMmaAhead], ((n / kMmaAhead) & 1u) ^ 1u, abort)) return false;
-            more = mma_plan_tile<TABLE, CHECK>(sm, a, rank, lane, plan, n);
-        }
-        if (!walk.wait(sm)) return false;
-        const MmaTile &t = walk.tile(sm);
-        if (t.chunks == 0) return true;
-        const MmaProblem &p = mma_problem_of<TABLE>(t, a);
-        const int rows = max(1, min(t.rows, p.M - t.row0 - (int)(rank & 1u) * t.rows));
-        const int first = t.start[0], end = t.end[rows - 1];
-        const int shares = kMmaLookWarps * a.splits, each = (end - first + shares - 1) / shares;
-        const int from = first + min(each * (kMmaLookWarps * (int)(rank >> 1) + which), end - first), stop = min(from + each, end);
-        for (int at = from; at < stop; at += 32 * kAtOnce) {
-            int c[kAtOnce + 1];
-#pragma unroll
-            for (int j = 0; j <= kAtOnce; j++) {
-                const int q = at + 32 * j + lane;
-                c[j] = 0x7fffffff;
-                if (q < end && (j < kAtOnce || lane == 0)) c[j] = __ldg(p.cols + q);
-            }
-            unsigned descents = 0u;  // bit j: the entry behind c[j] is not larger
-#pragma unroll
-            for (int j = 0; j < kAtOnce; j++) {
-                int next = __shfl_down_sync(0xffffffffu, c[j], 1);
-                const int far = __shfl_sync(0xffffffffu, c[j + 1], 0);
-                if (lane == 31) next = far;
-                if (next <= c[j]) descents |= 1u << j;
-            }
-            while (descents) {
-                const int q = at + 32 * (__ffs(descents) - 1) + lane + 1;
-                descents &= descents - 1u;
-                if (q >= end) break;
-                int lo = 0, hi = rows - 1;  // the last row that starts at or in front of it
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (t.start[mid] <= q) lo = mid;
-                    else hi = mid - 1;
-                }
-                if (t.start[lo] != q) mma_mark_again(sm, t.ring, (int)(rank & 1u) * t.rows + lo, rank);
-            }
-            __syncwarp();
-        }
-        if (lane == 0) {  // (marks are fenced where they are made)
-            unsigned long long *bar = &sm.checked[walk.n % kMmaAhead];
-            mbar_arrive(bar);
-            mbar_arrive_cluster(cluster_map(smem_u32(bar), rank ^ 1u));
-            walk.done(sm);
-        }
-        __syncwarp();
-    }
 }
 
 // ---- issuing warp (of the even block) ----------------------------------------------------------
@@ -790,7 +721,7 @@ __device__ __forceinline__ void mma_mark_not_finite(MmaSmem &sm, int ring, const
 
 // Warp w: tensor-memory lanes 32 * (w % 4) .. + 31 (columns of C), accumulator columns 64 * (w / 4) .. + 63
 // (rows of the sparse matrix).
-template <bool TABLE, bool LOOK>
+template <bool TABLE>
 __device__ __forceinline__ bool mma_sums(MmaSmem &sm, const MmaArgs &a, unsigned rank, int warp, int lane)
 {
     volatile int *abort = &sm.abort;
@@ -838,7 +769,6 @@ __device__ __forceinline__ bool mma_sums(MmaSmem &sm, const MmaArgs &a, unsigned
             for (int j = 0; j < kMmaRows; j++)
                 if (j < rows) __stcs(c + (size_t)j * (size_t)N, acc[j]);
         }
-        if (LOOK && !mbar_wait_suspended(&sm.checked[walk.n % kMmaAhead], (walk.n / kMmaAhead) & 1u, abort)) return false;
         sum_warps_barrier();
         unsigned any = 0;
         for (int w = 0; w < kMmaMarkWords; w++) any |= *(volatile unsigned *)&sm.again[ring][w];
@@ -936,7 +866,6 @@ __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_c
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned rank = cluster_rank();
     constexpr int kIssueWarp = kMmaSumWarps + kMmaOperandWarps, kPlanWarp = kIssueWarp + 2;
-    constexpr bool kLook = CHECK && !TABLE;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kMmaStages; s++) {
             mbar_init(&sm.full[s], kMmaOperandWarps + (rank & 1u ? 0u : 1u));  // even block: plus the odd one's relay
@@ -948,8 +877,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_c
         mbar_init(&sm.small_empty, kMmaSumWarps + (rank & 1u ? 0u : 1u));
         for (int n = 0; n < kMmaAhead; n++) {
             mbar_init(&sm.tile_full[n], 1);
-            mbar_init(&sm.tile_empty[n], kMmaSumWarps + kMmaOperandWarps + (rank & 1u ? 2u : 1u) + (kLook ? kMmaLookWarps : 0));  // with the issuing warp or both relays
-            mbar_init(&sm.checked[n], 2 * kMmaLookWarps);
+            mbar_init(&sm.tile_empty[n], kMmaSumWarps + kMmaOperandWarps + (rank & 1u ? 2u : 1u));  // and the issuing warp or both relays
         }
         mbar_init(&sm.drain, 1);
         sm.abort = 0;
@@ -993,17 +921,13 @@ __global__ void __launch_bounds__(kMmaThreads, 1) spmm_mma_kernel(const __grid_c
         // nothing left to do
     } else if (warp < kMmaSumWarps) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kMmaRegsSum));
-        ok = mma_sums<TABLE, kLook>(sm, a, rank, warp, lane);
+        ok = mma_sums<TABLE>(sm, a, rank, warp, lane);
     } else if (warp < kIssueWarp) {
         if (kMmaRegsOperand != kMmaRegsLaunch) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kMmaRegsOperand));
-        ok = mma_operands<TABLE, WIDE, DEEP, TABLE && CHECK>(sm, a, rank, warp - kMmaSumWarps, lane);
+        ok = mma_operands<TABLE, WIDE, DEEP, CHECK>(sm, a, rank, warp - kMmaSumWarps, lane);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kMmaRegsIssue));
-        if constexpr (kLook) {
-            if (warp >= kPlanWarp) ok = mma_look<TABLE, CHECK>(sm, a, rank, warp - kPlanWarp, lane, plan, more);
-        } else if (warp == kPlanWarp && more) {
-            ok = mma_plan<TABLE, CHECK>(sm, a, rank, lane, plan, TABLE ? 0u : 1u);
-        }
+        if (warp == kPlanWarp && more) ok = mma_plan<TABLE, CHECK>(sm, a, rank, lane, plan, TABLE ? 0u : 1u);
         if (warp == kIssueWarp && (rank & 1u) == 0u) {
             const bool issuer = elect_one();
             ok = mma_issue(sm, rank, issuer, lane);
