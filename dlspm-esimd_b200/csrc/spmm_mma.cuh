@@ -291,8 +291,8 @@ __device__ __forceinline__ int mma_lower_bound(const int *__restrict__ cols, int
 // ---- operand warps ------------------------------------------------------------------------------------
 
 // The fetches of an operand warp's part of B, rows 16 * (warp / 4) .. + 15 of a chunk and columns 32 * (warp % 4) .. + 31 of
-// this block's, two chunks ahead of the conversion and across tiles.  Rows and columns past the end of B repeat its last
-// ones: no entry refers to such a row, and such a column is not stored.
+// this block's, two chunks ahead of the conversion and across tiles.  Rows and columns past the end of B are others of
+// its own: no entry refers to such a row, and such a column is not stored.
 struct MmaFetch {
     unsigned n;        // tile
     int left;          // its chunks to come; < 0: behind the last tile
@@ -325,7 +325,11 @@ __device__ __forceinline__ bool mma_fetch_tile(MmaFetch &f, MmaSmem &sm, const M
     const MmaProblem &p = mma_problem_of<TABLE>(t, a);
     f.left = t.chunks == 0 ? -1 : t.chunks;
     if (f.left < 0) return true;
-    const int n = min(t.n0 + 32 * (warp & 3) + (WIDE ? 4 * (lane & 7) : lane), p.N - (WIDE ? 4 : 1));
+    int n = t.n0 + 32 * (warp & 3) + (WIDE ? 4 * (lane & 7) : lane);
+    // Columns past the end: others instead, by steps of 32, so that the lanes of a request differ.  (Copies of one word to 32
+    // places are done one by one: all on the last column, 3000 x 1500 at 50 %, N = 770 took 227 us.)
+    if (n >= p.N) n = max(n - ((n - p.N) / 32 + 1) * 32, 0);
+    n = min(n, p.N - (WIDE ? 4 : 1));
     const int k = t.chunk0 * kMmaChunk + 16 * (warp >> 2);
     f.rows = p.K - k;
     f.row = 4u * (unsigned)p.N;
