@@ -29,8 +29,15 @@ struct SpmmArgs {
     int sm_count;
 };
 
+// Resident blocks per SM of the builds with batched loads.  Three leave 80 registers, which those need; one chunk of 16-byte
+// loads does with 64.  Speed against a plain loop whose loads were waited for one by one, with three / four blocks: 4800 x
+// 4096 at 5 %, N = 256 1.49 / 1.31, 5000 x 3000 at 10 %, N = 98 1.89 / 1.64, 8192 x 4096 at 5 %, N = 128 1.23 / 1.31.  Held by
+// their latency, long launches gain as well (they had a build of the plain loop in 32 and 44 registers before): 32768 x 8192 at
+// 2 %, N = 128 151 -> 126 us, 16000 x 8000 at 2 %, N = 256 161 -> 145, 6000 x 3000 at 2 %, N = 150 37.4 -> 28.4.
+template <int VEC, int U>
+constexpr int kLoneBlocks = VEC == 4 && U == 1 ? 4 : 3;
 template <int VEC, int U, bool STRICT, int J>
-__global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_rows_kernel(const SpmmArgs a)
+__global__ void __launch_bounds__(kWarpsPerCta * 32, J > 0 ? kLoneBlocks<VEC, U> : 0) spmm_rows_kernel(const SpmmArgs a)
 {
     grid_dependency_wait();
     __shared__ int2 stage[kWarpsPerCta][32];
@@ -47,13 +54,20 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_rows_kernel(const Spmm
                                        stage[warp]);
 }
 
-// Few long rows: the S warps of a group share one row, each taking every S-th run of 32 nonzeros;
-// the partial slabs are added in a fixed order through shared memory, so the result is deterministic
-// (but not in CSR order: this path is not used in strict mode).  8/S rows per thread block.
-template <int VEC, int U, int S>
-__global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_rows_split_kernel(const SpmmArgs a)
+// Few long rows: the S warps of a group share one row; the partial slabs are added in a fixed order through shared memory,
+// so the result is deterministic (but not in CSR order: this path is not used in strict mode).  8/S rows per thread block.
+// Such a launch is bound by the latency of a warp's loads, one after the other: the row's offsets, its pairs, then a batch
+// of rows of B after another, each about 0.4 us from L2.  Every warp therefore takes an equal share of the row, in whole
+// half (kTail = 2) or quarter batches, and asks for the next 32 pairs a step ahead.  Dealt out in runs of 32, 51 entries
+// were 32 / 19 / 0 / 0 on four warps.  Device time (launches in a graph), runs of 32 with the loads of a batch waited for
+// one by one (load_vec_if) / this: 512 x 512 at 10 %, N = 128 4.8 / 2.7 us, 64 x 4000 at 10 %, N = 128 14.8 / 5.8, 300 x 2000
+// at 5 %, N = 1024 16.5 / 10.0, 512 x 2048 at 5 %, N = 256 6.5 / 5.4, 1003 x 1531 at 20 %, N = 49 14.0 / 11.7.
+// BLOCKS: resident blocks per SM (0: what the compiler likes), see launch_rows_split.
+template <int VEC, int U, int S, int BLOCKS>
+__global__ void __launch_bounds__(kWarpsPerCta * 32, BLOCKS) spmm_rows_split_kernel(const SpmmArgs a)
 {
     grid_dependency_wait();
+    constexpr int J = kLoneBatch<VEC, U>;
     __shared__ int2 stage[kWarpsPerCta][32];
     __shared__ float part[kWarpsPerCta][U][32 * VEC];
     constexpr int kRows = kWarpsPerCta / S;
@@ -76,13 +90,18 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) spmm_rows_split_kernel(cons
     }
     if (active) {
         const int start = __ldg(a.row_offsets + row), end = __ldg(a.row_offsets + row + 1);
-        for (int base = start + 32 * split; base < end; base += 32 * S) {
-            const int p = base + lane;
-            int2 cv = make_int2(0, 0);
-            if (p < end) cv = make_int2(__ldg(a.cols + p), __float_as_int(__ldg(a.values + p)));
-            stage[warp][lane] = cv;
+        constexpr int kTail = VEC == 4 && U > 1 ? 4 : 2;
+        constexpr int kStep = J > 0 ? J / kTail : 4;
+        const float *values = a.values + start;
+        const int *cols = a.cols + start;
+        const int len = end - start, share = ((len + S - 1) / S + kStep - 1) / kStep * kStep;
+        const int last = min((split + 1) * share, len);
+        int2 next = spmm_first_pairs(values, cols, split * share, last, lane);
+        for (int base = split * share; base < last; base += 32) {
+            stage[warp][lane] = next;
             __syncwarp();
-            spmm_accumulate_staged<VEC, U, false, kLoneBatch<VEC, U>>(stage[warp], min(32, end - base), a.B, a.N, cidx, acc);
+            next = spmm_first_pairs(values, cols, base + 32, last, lane);
+            spmm_accumulate_staged<VEC, U, false, J, kTail>(stage[warp], min(32, last - base), a.B, a.N, cidx, acc);
             __syncwarp();
         }
     }
@@ -111,7 +130,17 @@ template <int VEC, int U, int S>
 void launch_rows_split(SpmmArgs a, int slabs, cudaStream_t st)
 {
     a.row_groups = dlspm_ceil_div(a.M, kWarpsPerCta / S);
-    launch_overlapped(spmm_rows_split_kernel<VEC, U, S>, (unsigned)((long long)a.row_groups * slabs), kWarpsPerCta * 32, 0, st, a);
+    // Registers keep loads in flight, blocks keep a second wave away: 80 registers while three blocks per SM hold the launch,
+    // 64 beyond that where the batch is one or two chunks of 16-byte loads (three / four blocks, in speed against before:
+    // 64 rows, N = 128 2.4 / 2.0, but 1024 rows, N = 128, 512 blocks 1.37 / 1.45; 512 rows, N = 256 0.96 / 1.19).  The
+    // others keep one build: 64 registers spill the narrower loads (2000 x 2000, N = 98 1.24 / 1.13; 400 rows, N = 197 1.40
+    // / 1.31), four chunks want 121 (300 rows, N = 1024 1.65 with two blocks, 1.55 with three), and one chunk of 8-byte loads
+    // takes 47 by itself (700 rows, N = 50 1.19, with 80 0.97, in two waves).
+    const long long blocks = (long long)a.row_groups * slabs;
+    constexpr int kFew = VEC == 2 && U == 1 ? 0 : VEC == 4 && U == 4 ? 2 : 3;
+    constexpr int kMany = VEC == 4 && U <= 2 ? 4 : kFew;
+    if (blocks <= 3LL * a.sm_count) launch_overlapped(spmm_rows_split_kernel<VEC, U, S, kFew>, (unsigned)blocks, kWarpsPerCta * 32, 0, st, a);
+    else launch_overlapped(spmm_rows_split_kernel<VEC, U, S, kMany>, (unsigned)blocks, kWarpsPerCta * 32, 0, st, a);
 }
 
 // Narrow dense operand (N <= 64 floats, 16-byte aligned rows): a full warp per row would leave most
@@ -231,22 +260,9 @@ void launch_subwarp(const SpmmArgs &a, bool strict, cudaStream_t st)
 template <int VEC, int U>
 void launch_rows(const SpmmArgs &a, int slabs, bool strict, cudaStream_t st)
 {
-    const long long tiles = (long long)a.row_groups * slabs;
-    const unsigned grid = (unsigned)tiles, block = kWarpsPerCta * 32;
-    // The narrow slabs exist in two builds: with the batched loads (74 to 76 registers, three
-    // resident blocks) for launches of a few waves, where the latency chain of a warp counts, and
-    // with the plain loop (32 and 44 registers) for long launches, where occupancy hides it.
-    // Measured: one-chunk slabs, 32768 x 8192 (9 waves) 0.71 -> 0.61 ms with the plain loop but
-    // 8192 x 8192 (2.3 waves) 0.19 -> 0.20 ms; two-chunk slabs, 32768 x 2048 413 -> 338 us.
-    const int waves = U == 1 ? 6 : 2;
-    const bool lone = kLoneBatch<VEC, U> > 0 && tiles <= (long long)waves * 3 * a.sm_count;
-    if (lone) {
-        if (strict) launch_overlapped(spmm_rows_kernel<VEC, U, true, kLoneBatch<VEC, U>>, grid, block, 0, st, a);
-        else launch_overlapped(spmm_rows_kernel<VEC, U, false, kLoneBatch<VEC, U>>, grid, block, 0, st, a);
-    } else {
-        if (strict) launch_overlapped(spmm_rows_kernel<VEC, U, true, 0>, grid, block, 0, st, a);
-        else launch_overlapped(spmm_rows_kernel<VEC, U, false, 0>, grid, block, 0, st, a);
-    }
+    const unsigned grid = (unsigned)((long long)a.row_groups * slabs), block = kWarpsPerCta * 32;
+    if (strict) launch_overlapped(spmm_rows_kernel<VEC, U, true, kLoneBatch<VEC, U>>, grid, block, 0, st, a);
+    else launch_overlapped(spmm_rows_kernel<VEC, U, false, kLoneBatch<VEC, U>>, grid, block, 0, st, a);
 }
 
 template <int VEC, int U>

@@ -30,6 +30,24 @@ __device__ __forceinline__ void load_vec(const float *__restrict__ p, float (&v)
     }
 }
 
+// The same load where `use` holds, zeros elsewhere.  Volatile: an ordinary load under a condition is moved down to the
+// product that needs it when that has the same condition, so that a batch's loads are waited for one after the other.
+template <int VEC>
+__device__ __forceinline__ void load_vec_if(const float *__restrict__ p, bool use, float (&v)[VEC])
+{
+    if constexpr (VEC == 4) {
+        asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %5, 0;\n mov.b32 %0, 0;\n mov.b32 %1, 0;\n mov.b32 %2, 0;\n mov.b32 %3, 0;\n"
+                     " @q ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n}"
+                     : "=&f"(v[0]), "=&f"(v[1]), "=&f"(v[2]), "=&f"(v[3]) : "l"(p), "r"((unsigned)use));
+    } else if constexpr (VEC == 2) {
+        asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %3, 0;\n mov.b32 %0, 0;\n mov.b32 %1, 0;\n @q ld.global.nc.v2.f32 {%0, %1}, [%2];\n}"
+                     : "=&f"(v[0]), "=&f"(v[1]) : "l"(p), "r"((unsigned)use));
+    } else {
+        asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n mov.b32 %0, 0;\n @q ld.global.nc.f32 %0, [%1];\n}"
+                     : "=&f"(v[0]) : "l"(p), "r"((unsigned)use));
+    }
+}
+
 template <int VEC>
 __device__ __forceinline__ void store_vec(float *__restrict__ p, const float (&v)[VEC])
 {
@@ -71,8 +89,9 @@ __device__ __forceinline__ float mad(float a, float b, float c)
 // Adds the products of `cnt` staged (column, value) pairs to the accumulators of one warp slab, in
 // the order of the pairs.  J = 0: the plain loop, unrolled four times.  J > 0: J nonzeros are taken
 // at once, all their loads first and their products afterwards (still in pair order), which keeps
-// J*U loads in flight per lane; a lone small matrix is bound by exactly that latency chain.
-template <int VEC, int U, bool STRICT, int J>
+// J*U loads in flight per lane; a lone small matrix is bound by exactly that latency chain.  What is left
+// of the pairs is taken J/TAIL at once.
+template <int VEC, int U, bool STRICT, int J, int TAIL = 4>
 __device__ __forceinline__ void spmm_accumulate_staged(const int2 *stage, int cnt, const float *__restrict__ B,
                                                        int N, const int (&cidx)[U], float (&acc)[U][VEC])
 {
@@ -113,7 +132,7 @@ __device__ __forceinline__ void spmm_accumulate_staged(const int2 *stage, int cn
                 const float *brow = B + (size_t)e.x * (size_t)N;
 #pragma unroll
                 for (int u = 0; u < U; u++)
-                    if (in[u]) load_vec<VEC>(brow + at[u], b[jj][u]);
+                    load_vec_if<VEC>(brow + at[u], in[u], b[jj][u]);
             }
 #pragma unroll
             for (int jj = 0; jj < J; jj++) {
@@ -126,8 +145,8 @@ __device__ __forceinline__ void spmm_accumulate_staged(const int2 *stage, int cn
                 }
             }
         }
-        // the rest, in batches of a quarter
-        constexpr int T = J / 4;
+        // the rest, in smaller batches
+        constexpr int T = J / TAIL;
         for (; j < cnt; j += T) {
             float b[T][U][VEC];
             float a[T];
@@ -139,7 +158,7 @@ __device__ __forceinline__ void spmm_accumulate_staged(const int2 *stage, int cn
                 const float *brow = B + (size_t)e.x * (size_t)N;
 #pragma unroll
                 for (int u = 0; u < U; u++)
-                    if (live && in[u]) load_vec<VEC>(brow + at[u], b[jj][u]);
+                    load_vec_if<VEC>(brow + at[u], live && in[u], b[jj][u]);
             }
 #pragma unroll
             for (int jj = 0; jj < T; jj++) {
@@ -157,11 +176,9 @@ __device__ __forceinline__ void spmm_accumulate_staged(const int2 *stage, int cn
     }
 }
 
-// Nonzeros taken at once by a lone launch (0: the plain unrolled loop): 8 loads in flight per lane
-// for the one- and two-chunk slabs of 16-byte loads.  Measured on lone matrices of 256 to 2048 rows: 512 x 512 at
-// 10 %, N = 128 went from 7.7 to 5.2 us, 1024 x 1024 at 30 % from 20.5 to 17.5 us; 16 nonzeros at
-// once (one-chunk) or 8 (two-chunk) lost again through registers.  Narrower loads need fewer registers each, so more
-// of them are in flight.  The grouped launch keeps the
+// Nonzeros taken at once by a lone launch (0: the plain unrolled loop): 32 registers of loads in flight per lane.  Four
+// chunks of 16-byte loads keep the plain loop, which has 4 to 16 loads in flight as it is (two nonzeros at once: 4096 x 4096
+// at 2 %, N = 1024 1.04 of the speed, 2048 x 512, N = 3136 0.96).  The grouped launch keeps the
 // plain loop for every width: it holds all three widths in one kernel, its occupancy is what
 // hides the latency there, and the batched loads would cost it registers.
 template <int VEC, int U>

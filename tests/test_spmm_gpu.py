@@ -105,6 +105,19 @@ def test_sweep_shapes_one_prepared_batch(pkg, oracle, ctx, dev, kernel):
         check(oracle, ro, ci, vals, B, M, N, Cd.cpu().numpy().reshape(M, N))
 
 
+@pytest.mark.parametrize("longest", [40, 300])  # two and eight warps per row
+@pytest.mark.parametrize("copies", [1, 5])  # launches that few and many resident blocks per SM hold
+@pytest.mark.parametrize("N", [7, 25, 49, 50, 98, 128, 132, 197, 256, 302, 516, 640])
+def test_rows_shared_between_warps(pkg, oracle, ctx, dev, N, copies, longest):
+    """Every row length up to a few shares of eight warps, in every width of loads and chunks: whole batches, their rests,
+    warps without a share, and a step beyond 32 pairs."""
+    lengths = np.tile(np.arange(longest), copies)
+    K = 500
+    ro, ci = csr_from_lengths(pkg, K, lengths, seed=N)
+    vals, B = dense(pkg, int(ci.size), 1, N, 2).reshape(-1), dense(pkg, K, N, N, 10)
+    check(oracle, ro, ci, vals, B, lengths.size, N, run_spmm(ctx, dev, lengths.size, K, N, ro, ci, vals, B))
+
+
 @pytest.mark.parametrize("N", [4, 8, 12, 16, 20, 32, 36, 48, 64])
 def test_narrow_dense_operand_many_rows(pkg, oracle, ctx, dev, N):
     """Enough rows for the several-rows-per-warp kernel (N <= 64): 4, 8 and 16 lanes per row, widths
