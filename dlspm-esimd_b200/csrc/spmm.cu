@@ -29,15 +29,16 @@ struct SpmmArgs {
     int sm_count;
 };
 
-// Resident blocks per SM of the builds with batched loads.  Three leave 80 registers, which those need; one chunk of 16-byte
-// loads does with 64.  Speed against a plain loop whose loads were waited for one by one, with three / four blocks: 4800 x
+// Resident blocks per SM.  Three leave 80 registers, which the batched loads need, and four chunks of the plain loop (for the
+// compiler's choice of 66: 4096 x 4096 at 2 %, N = 1024 90 -> 81 us, 1000 x 2560 at 2 %, N = 3136 44.8 -> 40.6); one chunk of
+// 16-byte loads does with 64.  Speed against a plain loop whose loads were waited for one by one, with three / four blocks: 4800 x
 // 4096 at 5 %, N = 256 1.49 / 1.31, 5000 x 3000 at 10 %, N = 98 1.89 / 1.64, 8192 x 4096 at 5 %, N = 128 1.23 / 1.31.  Held by
 // their latency, long launches gain as well (they had a build of the plain loop in 32 and 44 registers before): 32768 x 8192 at
 // 2 %, N = 128 151 -> 126 us, 16000 x 8000 at 2 %, N = 256 161 -> 145, 6000 x 3000 at 2 %, N = 150 37.4 -> 28.4.
 template <int VEC, int U>
 constexpr int kLoneBlocks = VEC == 4 && U == 1 ? 4 : 3;
 template <int VEC, int U, bool STRICT, int J>
-__global__ void __launch_bounds__(kWarpsPerCta * 32, J > 0 ? kLoneBlocks<VEC, U> : 0) spmm_rows_kernel(const SpmmArgs a)
+__global__ void __launch_bounds__(kWarpsPerCta * 32, kLoneBlocks<VEC, U>) spmm_rows_kernel(const SpmmArgs a)
 {
     grid_dependency_wait();
     __shared__ int2 stage[kWarpsPerCta][32];

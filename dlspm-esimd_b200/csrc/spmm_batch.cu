@@ -111,8 +111,12 @@ __device__ __forceinline__ void batched_rows_coarse(const BatchProblem &p, int s
 // total.
 // COARSE: the tiles of this launch cover 64 rows (each warp walks eight of them) instead of 8; a
 // build of its own, because the extra loop costs the common build registers it does not have.
+// The common build has 128 registers, so that the loads of four nonzeros are in flight in all three widths; two blocks per SM
+// with them do more than three or four with 64 to 80.  Left to the compiler (64) / 128: grouped calls of 9 to 180 problems
+// 314 / 194, 686 / 578, 1931 / 1813, 3086 / 2914 us, prepared batches, where the tensor cores do most, 0.98 to 1 of the time
+// (80 registers: group of 12 1.03 of the speed, 128 1.10).  The coarse tiles' rows are too short for it.
 template <bool STRICT, bool COARSE>
-__global__ void __launch_bounds__(kBatchWarps * 32)
+__global__ void __launch_bounds__(kBatchWarps * 32, COARSE ? 0 : 2)
 spmm_batched_kernel(const BatchProblem *__restrict__ problems, const long long *__restrict__ tile_start,
                     int count, unsigned long long *counter)
 {
