@@ -389,7 +389,8 @@ __device__ __forceinline__ void mma_store_dense(uint32_t dst, const float *raw, 
     tmem_store4(dst, x1);
     tmem_store4(dst + kMmaDensePart, x2);
     tmem_store4(dst + 2 * kMmaDensePart, x3);
-    if (small < kSplitSmall) {  // a zero, or a number that cannot be split
+    // a zero, or a number that cannot be split (asked by the whole warp: the wait for the stores is for a converged one)
+    if (__any_sync(0xffffffffu, small < kSplitSmall)) {
 #pragma unroll
         for (int i = 0; i < 8; i++) least = split_magnitude(d[i], least);
     }
@@ -534,6 +535,7 @@ __device__ __forceinline__ bool mma_operand_tile(MmaSmem &sm, const MmaArgs &a, 
                 if (bad && own < t.rows) mma_mark_again(sm, t.ring, (int)(rank & 1u) * t.rows + own, rank);
                 if (all)
                     for (int r = lane; r < 2 * t.rows; r += 32) mma_mark_again(sm, t.ring, r, rank);
+                __syncwarp();
             }
         }
         tmem_store_wait();

@@ -151,7 +151,7 @@ def test_many_tiles_per_cluster(pkg, oracle, ctx, dev):
         ctx.set_option(pkg.OPT_TILE_MIN_DENSITY, -1)
 
 
-@pytest.mark.parametrize("where", ["infinite", "tiny", "huge", "tiny rows", "tiny columns"])
+@pytest.mark.parametrize("where", ["infinite", "tiny", "huge", "tiny rows", "tiny columns", "zeros", "zeros, one tiny"])
 def test_numbers_that_cannot_be_split(pkg, oracle, ctx, dev, where):
     """Infinities and NaN reach the rows that refer to them and no others; magnitudes at the ends of the range keep
     their precision."""
@@ -181,6 +181,10 @@ def test_numbers_that_cannot_be_split(pkg, oracle, ctx, dev, where):
         else:
             for _ in range(2):
                 B[:, [3, 140, 141, 400]] *= np.float32(1e-28)
+    elif where.startswith("zeros"):  # in some columns of B, so that the lanes of a warp part, in the last rows of it too
+        B[np.arange(K)[:, None] % 5 == np.arange(N) % 7] = 0
+        if where == "zeros, one tiny":
+            B[K - 1, 77] = np.float32(1e-35)
     elif where == "tiny":
         vals = (vals * np.float32(1e-36)).astype(np.float32)
         B *= np.float32(1e20)
