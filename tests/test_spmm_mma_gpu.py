@@ -98,33 +98,76 @@ def test_lone_launches(pkg, oracle, ctx, dev, M, K, N, density, order):
     check(oracle, ro, ci, vals, B, M, N, lone_run(ctx, dev, M, K, N, ro, ci, vals, B, plan=True))
 
 
-@pytest.mark.parametrize("M,K,N", [(12900, 200, 1028), (130, 4097, 260)])
+def gather_run(ctx, dev, M, K, N, ro, ci, vals, B):
+    """The row-gather kernel whatever the sizes: a plan made when no row was sorted (entries may be permuted inside rows since)."""
+    import torch
+
+    out = torch.full((M, N), float("nan"), device=dev)
+    d = [to_dev(x, dev) for x in (vals, ro, ci, B)]
+    p = ctx.plan_create(M, K, int(ci.size), d[1], to_dev(np.concatenate([ci[s:e][::-1] for s, e in zip(ro, ro[1:])]), dev))
+    ctx.spmm_planned(p, N, *d, out)
+    torch.cuda.synchronize()
+    p.close()
+    return out.cpu().numpy()
+
+
+def looks_sorted(ro, ci, M):
+    """The kernel's look at the order of columns: eight entries from the middle of 32 rows."""
+    for row in (M * lane // 32 for lane in range(32)):
+        start, end = int(ro[row]), int(ro[row + 1])
+        c = ci[start + (end - start) // 2:end][:8]
+        if (np.diff(c) <= 0).any():
+            return False
+    return True
+
+
+@pytest.mark.parametrize("M,K,N", [(12900, 200, 1028), (9800, 200, 1029), (900, 4100, 300), (900, 4100, 301)])
 def test_order_of_columns_is_seen_in_every_tile_of_a_lone_launch(pkg, oracle, ctx, dev, M, K, N):
-    """More tiles for every pair of blocks than are planned ahead, and one tile in parts of K; empty rows among them.
-    Columns repeated at the start, in the middle and at the end of rows, and rows that run backwards."""
-    seed = M
+    """More tiles for every pair of blocks than are planned ahead, and one tile in four parts of K, with 16- and 4-byte
+    copies of B; empty rows among them.  Columns repeated at the start, in the middle and at the end of rows, rows that run
+    backwards, and columns exchanged or repeated where the parts of K meet.  The rows that the kernel looks at before it
+    multiplies are in order, so that no launch is left to its gather loop."""
+    seed = M + N
     rng = np.random.default_rng(seed)
     lengths = rng.integers(K // 4, K // 2, M)
     lengths[rng.integers(0, M, M // 8)] = 0
     lengths[:3] = 0
     lengths[-1] = 0
     ro, ci = csr_from_lengths(pkg, K, [int(x) for x in lengths], seed=seed)
-    for n, i in enumerate(i for i in range(M) if lengths[i]):
-        at = {0: 0, 1: int(lengths[i]) // 2, 2: int(lengths[i]) - 2}.get(n % 11)
-        if at is not None:
-            ci[ro[i] + at + 1] = ci[ro[i] + at]
-        elif n % 11 == 3:
-            ci[ro[i]:ro[i + 1]] = ci[ro[i]:ro[i + 1]][::-1].copy()
+    chunks = -(-K // 64)
+    seams = [64 * (chunks * part // 4) for part in (1, 2, 3)]
+    looked_at = {M * lane // 32 for lane in range(32)}
+    mixed = np.zeros(M, dtype=bool)
+    for n, i in enumerate(i for i in range(M) if lengths[i] and i not in looked_at):
+        start, end = int(ro[i]), int(ro[i + 1])
+        at = {0: start, 1: start + int(lengths[i]) // 2, 2: end - 2}.get(n % 11)
+        if n % 11 in (4, 5, 6):  # the last entry in front of a seam and the first one behind it
+            at = start + int(np.searchsorted(ci[start:end], seams[n % 11 - 4])) - 1
+            if not start <= at < end - 1:
+                continue
+        if n % 11 == 3:
+            ci[start:end] = ci[start:end][::-1].copy()
+        elif at is None:
+            continue
+        elif n % 22 in (4, 5, 6):
+            ci[at], ci[at + 1] = ci[at + 1], ci[at]
+        else:
+            ci[at + 1] = ci[at]
+        mixed[i] = True
+    assert looks_sorted(ro, ci, M) and mixed.sum() > M // 3
     vals = pkg.gen_dense_host(int(ci.size), seed, 2)
     B = dense(pkg, K, N, seed, 10)
     out = lone_run(ctx, dev, M, K, N, ro, ci, vals, B)
     check(oracle, ro, ci, vals, B, M, N, out)
     assert (out[lengths == 0] == 0).all()
+    # sums of split products do not have the bits of a chain of multiply-adds in a row of 50 entries and 300 columns or more
+    gathered = gather_run(ctx, dev, M, K, N, ro, ci, vals, B)
+    assert all((out[i] != gathered[i]).any() for i in range(M) if lengths[i] and not mixed[i]), "rows not multiplied"
 
 
 def test_many_tiles_per_cluster(pkg, oracle, ctx, dev):
     """More tiles for every pair of blocks than are planned ahead, of problems of different sizes, as a prepared batch
-    (columns known to ascend) and as a one-shot call (columns checked)."""
+    (columns known to ascend; the one-shot call: test_many_tiles_with_columns_out_of_order)."""
     import torch
 
     shapes = [(17 + 53 * i % 290, 40 + 31 * i % 90, 260 + 4 * (i % 3)) for i in range(120)]
@@ -140,12 +183,10 @@ def test_many_tiles_per_cluster(pkg, oracle, ctx, dev):
             keep.append((ro, ci, vals, B, out))
         batch = ctx.batch_create(arr)
         assert batch.info()[1] == len(shapes)
-        for launch in (batch.launch, lambda: ctx.spmm_batched(arr)):
-            launch()
-            torch.cuda.synchronize()
-            for (M, K, N), (ro, ci, vals, B, out) in zip(shapes, keep):
-                check(oracle, ro, ci, vals, B, M, N, out.cpu().numpy().reshape(M, N))
-                out.fill_(float("nan"))
+        batch.launch()
+        torch.cuda.synchronize()
+        for (M, K, N), (ro, ci, vals, B, out) in zip(shapes, keep):
+            check(oracle, ro, ci, vals, B, M, N, out.cpu().numpy().reshape(M, N))
         batch.close()
     finally:
         ctx.set_option(pkg.OPT_TILE_MIN_DENSITY, -1)
