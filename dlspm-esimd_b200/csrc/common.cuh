@@ -104,7 +104,7 @@ bool dlspm_spmm_mma_pays_alone(const dlspm_ctx *ctx, int M, int K, int N, int nn
 int dlspm_spmm_mma(dlspm_ctx *ctx, int M, int K, int N, int nnz, const float *values, const int *row_offsets, const int *cols,
                    const float *B, float *C, cudaStream_t st);
 
-// Whether the kernel's 32-bit offsets reach all of a problem.
+// Whether the kernel takes a problem of this size.
 bool dlspm_spmm_mma_fits(int K, int N, int nnz);
 // Which problems of a batch the tensor cores are the faster way for.
 void dlspm_spmm_mma_choose(int count, const dlspm_problem *problems, unsigned char *chosen);

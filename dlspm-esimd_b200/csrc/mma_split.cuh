@@ -80,14 +80,6 @@ __device__ __forceinline__ void split_one(float x, uint32_t &p1, uint32_t &p2, u
     p3 = bf16x2_bits(x, 0.f);
 }
 
-// Sixteen bytes that are not read again by this block: kept out of L1, which these kernels leave 28 KiB.
-__device__ __forceinline__ float4 load_once(const float *p)
-{
-    float4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-    return v;
-}
-
 // Stores by shared-memory address.
 __device__ __forceinline__ void store_shared(uint32_t at, uint32_t x, uint32_t y)
 {
@@ -248,7 +240,7 @@ __device__ __forceinline__ void tmem_add(float (&acc)[64], uint32_t addr, int co
 
 // Shared-memory operand descriptors.  Swizzled layouts repeat every 8 rows; byte offsets between repetitions:
 // `lead` and `stride` as in the canonical layouts of the PTX manual.
-constexpr uint64_t kSwizzle128 = 2, kSwizzle64 = 4;
+constexpr uint64_t kSwizzle128 = 2;
 __device__ __forceinline__ uint64_t mma_descriptor(uint32_t smem, unsigned lead, unsigned stride, uint64_t swizzle)
 {
     return (uint64_t)((smem & 0x3ffffu) >> 4) | ((uint64_t)(lead >> 4) << 16) | ((uint64_t)(stride >> 4) << 32) | (1ull << 46) |

@@ -289,8 +289,8 @@ void launch_rows_vec(SpmmArgs a, int split, bool strict, cudaStream_t st)
 
 // Warps per row for a lone matrix: with few rows one warp per (row, slab) leaves most of the device
 // idle and every warp walks its whole row as one latency chain, so rows are shared by 2, 4 or 8
-// warps until about 32 warps per SM exist or a warp would get fewer than 8 nonzeros.  Measured with
-// the bound at 64 / 16 / 8 nonzeros per warp (lone launches, warm L2): 512 x 512 at 10 %, N = 128:
+// warps until about 32 warps per SM exist or a warp would get fewer than 8 nonzeros.  Measured, when
+// rows were still dealt out in runs of 32, with the bound at 64 / 16 / 8 nonzeros per warp (lone launches, warm L2): 512 x 512 at 10 %, N = 128:
 // 17.3 / 13.1 / 7.6 us; 1024 x 1024 at 10 %, N = 128: 35.6 / - / 8.5 us; 512 x 2048 at 10 %,
 // N = 256: 47.8 / 12.8 / 12.8 us; nothing measured got slower by more than 10 %.
 int spmm_row_split(const dlspm_ctx *ctx, int M, int N, int nnz, int vec, bool strict)

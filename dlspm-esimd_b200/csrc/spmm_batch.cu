@@ -470,7 +470,7 @@ bool prefer_tiled(const dlspm_ctx *ctx, const dlspm_problem &q, int vec, bool so
 
 // Whether the automatic choice may take the tensor-core kernel for a problem.  The caller's density threshold, where one
 // is set, decides for the tiled kernels as a whole (without the estimate of dlspm_spmm_mma_choose, so the sizes the
-// kernel can address are tested here).
+// kernel takes are tested here).
 bool mma_eligible(const dlspm_ctx *ctx, const dlspm_problem &q, int vec)
 {
     if (ctx->spmm_kernel != 0 || vec != 4 || q.nnz == 0 || !dlspm_spmm_mma_fits(q.K, q.N, q.nnz)) return false;

@@ -65,18 +65,23 @@ int mma_splits(const dlspm_ctx *ctx, long long tiles, int K)
 
 }  // namespace
 
-// Byte offsets into B and into the CSR arrays are 32-bit in the kernel (and run up to two chunks past the end).
+// Byte offsets into the CSR arrays (up to two chunks past the end) and the step from request to request of B, four rows, are
+// 32-bit in the kernel.  B itself is addressed by 64-bit pointers; beyond 1e9 elements the kernel is not measured, and such
+// problems stay with the row-gather kernels.
 bool dlspm_spmm_mma_fits(int K, int N, int nnz)
 {
     return ((double)K + 4 * kMmaChunk) * N < 1e9 && nnz < 1000000000;
 }
 
 // Which problems of a batch the tensor cores are faster for: chosen[i], not 0 on entry where problem i may go there, becomes
-// its depth or 0.  A pair of blocks needs 1.5 us per chunk of 64 columns, more with more entries to scatter, and 3 us per
-// tile; the row-gather kernel 9 to 12 TFLOP/s.  Measured on batches of one shape with N = 3136, row-gather / tensor cores
-// in TFLOP/s: 1024 x 4096 at 50 % nonzeros 11 / 54, at 10 % 9.3 / 17, at 5 % equal; 2048 x 512 at 50 % 13.5 / 48, at 10 %
-// 11.4 / 12.5; 256 x 256 at 20 % 10.8 / 16.7, at 10 % equal.  A batch whose tiles are too few for the 74 pairs of blocks
-// takes as long as its longest tile: then none is chosen.
+// its depth or 0.  The constants are of a build that took 1.5 us per chunk of 64 columns, more with more entries to scatter,
+// and 3 us per tile; the present one takes 1.4 us per chunk at 10 % nonzeros and 1.9 at 50 % with 64 chunks a tile, tile
+// included (1.7 and 2.3 with eight chunks), so the estimate leaves problems near the line to the row-gather kernel (10 to 15
+// TFLOP/s).  Measured on batches of one shape with N = 3136, row-gather / tensor cores in TFLOP/s: 1024 x 4096 at 50 %
+// nonzeros 15.1 / 75.6, at 10 % 11.9 / 20.4, at 5 % 10.9 / 11.5 (left to the gather), at 2 % 10.2 / 4.9; 2048 x 512 at 50 %
+// 14.6 / 64.7, at 10 % 11.5 / 16.9, at 5 % 11.1 / 8.9; 512 x 2048 at 5 % 11.1 / 10.9; 256 x 256 at 20 % 11.4 / 23.6, at 10 %
+// 10.6 / 12.9 (left to the gather), at 5 % 8.5 / 6.7.  A batch whose tiles are too few for the 74 pairs of blocks takes as
+// long as its longest tile: then none is chosen.
 void dlspm_spmm_mma_choose(int count, const dlspm_problem *problems, unsigned char *chosen)
 {
     double all = 0.0, longest = 0.0, gather = 0.0;
@@ -99,9 +104,12 @@ void dlspm_spmm_mma_choose(int count, const dlspm_problem *problems, unsigned ch
 }
 
 // A matrix on its own: launch and first chunk 8.5 us, then 1.25 us per chunk and round of tiles; the row-gather
-// kernels 4 us and about 9.5, 6 or 3 TFLOP/s for rows of B that allow 16-, 8- or 4-byte loads.  Measured,
-// row-gather / tensor cores in us: 8192 x 2048 at 10 %, N = 256 90 / 53; 1024 x 4096 at 10 %, N = 1024 101 / 57, at
-// 50 %, N = 3136 1012 / 243; 512 x 2048 at 30 %, N = 256 equal; 256 x 512, N = 256 7.3 / 18.
+// kernels 4 us and about 9.5, 6 or 3 TFLOP/s for rows of B that allow 16-, 8- or 4-byte loads, which is what they did before
+// they issued a batch's loads together.  Measured (launches in a graph), row-gather / tensor cores in us: 8192 x 2048 at 10 %,
+// N = 256 74 / 52; 1024 x 4096 at 10 %, N = 1024 84 / 56, at 50 %, N = 3136 1276 / 298; 4096 x 4096 at 10 %, N = 256 85 / 57;
+// 1000 x 2000 at 20 %, N = 301 65 / 55; 512 x 2048 at 30 %, N = 256 24.3 / 25.0.  Near the line the tensor cores are the
+// slower way now (1024 x 1024 at 30 %, N = 512 34 / 41, 2048 x 2048 at 20 %, N = 200 43 / 55); the line stays where it was, since
+// sums there are three times as close to those in 64 bits as the gather's.
 bool dlspm_spmm_mma_pays_alone(const dlspm_ctx *ctx, int M, int K, int N, int nnz, int vec)
 {
     if (nnz == 0 || N < 32 || !dlspm_spmm_mma_fits(K, N, nnz)) return false;

@@ -29,8 +29,8 @@
 // N = 2048 327 -> 297 us, at 10 % 182 -> 180 us, a batch of 256 problems 5540 -> 5060 us, where the entries of the sparse rows
 // now find their lines in L1.  Measured and left: B's third part in shared memory and three stages (batch 5460 us; with
 // two chunks of raw B 5150 us); rows of B by bulk copies of 512 bytes from one warp (6680 us: it cannot issue them fast
-// enough); the entries by cp.async through rings of 128 per row (6560 us: more instructions); 37 to 70 KiB more for L1
-// (no change).
+// enough); the entries by cp.async through rings of 128 per row (6560 us: more instructions); two chunks of raw B instead
+// of three and the 32 KiB for L1 (5110 us).
 //
 // Roles of the 28 warps of a block:
 //   8 sum warps       add finished accumulators to their registers and write C.

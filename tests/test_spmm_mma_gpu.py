@@ -237,7 +237,7 @@ def test_numbers_that_cannot_be_split(pkg, oracle, ctx, dev, where):
 
 def test_problems_beyond_32_bit_offsets_stay_on_other_kernels(pkg, ctx, dev):
     """B of 2^30 elements and more, with a density threshold of the caller's (which takes the place of the estimate):
-    the byte offsets of such a B do not fit the tensor-core kernel."""
+    the tensor-core kernel does not take a B of that size."""
     import torch
 
     M, K, N, per_row = 64, (1 << 21) + 64, 512, 60
