@@ -42,11 +42,14 @@ COV = 0.4
 STREAM_PICK = 50
 FALLBACK_HBM_GBS = 6650.0
 # DRAM bytes per algorithmic byte of the two parts of a step, from one ncu capture each on the first 256 problems of the
-# batch (dram__bytes_read.sum + dram__bytes_write.sum over the algorithmic bytes of the problems the part served: 2.18 +
-# 0.61 GB for 3.06 GB on the row-gather kernel, whose last results are still in L2 when it ends; 5.62 + 0.53 GB for 2.52 GB
-# in the two builds of the tensor-core kernel, which read a B that L2 does not hold once per 128 rows).  Traffic grows with
-# the bytes of the problems processed, so the ratios are applied to the full launch.
-NCU_TRAFFIC_PER_ALGORITHMIC_BYTE = {"spmm_batched_kernel": 0.913, "spmm_mma_kernel": 2.44}
+# batch (dram__bytes_read.sum + dram__bytes_write.sum over the algorithmic bytes of the problems the part served: 0.86 +
+# 0.44 GB for 1.35 GB in the two builds of the row-gather kernel, whose last results are still in L2 when it ends; 2.07 + 0.56
+# GB for 2.52 GB in the two builds of the tensor-core kernel).  Traffic grows with the bytes of the problems processed, so the
+# ratios are applied to the full launch.
+NCU_TRAFFIC_PER_ALGORITHMIC_BYTE = {"spmm_batched_kernel": 0.958, "spmm_mma_kernel": 1.044}
+# Multiplies of bf16 parts per fp32 product of the tensor-core kernel: its roof is that share of the bf16 rate.
+SPLIT_PRODUCTS = 6
+FALLBACK_BF16_TFLOPS = 1590.0
 
 
 def log(*a):
@@ -289,10 +292,10 @@ def measured_peaks():
     if os.path.exists(path):
         try:
             d = json.load(open(path))
-            return float(d["hbm_gbs"]), "measured"
+            return float(d["hbm_gbs"]), float(d["bf16_tflops"]), "measured"
         except Exception:
             pass
-    return FALLBACK_HBM_GBS, "fallback"
+    return FALLBACK_HBM_GBS, FALLBACK_BF16_TFLOPS, "fallback"
 
 
 # ---- CPU baseline (the oracle: the reference's host loop, rows spread over the host threads) -----------------
@@ -1068,7 +1071,7 @@ def main():
     if args.tile_density is not None:
         ctx.set_option(pkg.OPT_TILE_MIN_DENSITY, args.tile_density)
     ctx.set_option(pkg.OPT_SPMM_KERNEL, args.spmm_kernel)
-    hbm_gbs, peak_kind = measured_peaks()
+    hbm_gbs, bf16_tflops, peak_kind = measured_peaks()
     fp32_tflops = ctx.measure_fp32_peak()
 
     t_setup = time.perf_counter()
@@ -1218,7 +1221,10 @@ def main():
         launch_avg_ms = dom["launch_ms"]
         achieved = dom["achieved_gbs"]
         dom_flops = dom["gflops"] * 1e6 * dom["launch_ms"]
-        t_roof_ms = max(dom["algorithmic_bytes_per_launch"] / (hbm_gbs * 1e9), dom_flops / (fp32_tflops * 1e12)) * 1e3
+        on_tensor_cores = dominant == "spmm_mma_kernel"
+        arithmetic_tflops = bf16_tflops / SPLIT_PRODUCTS if on_tensor_cores else fp32_tflops
+        t_hbm_ms = dom["algorithmic_bytes_per_launch"] / (hbm_gbs * 1e9) * 1e3
+        t_roof_ms = max(t_hbm_ms, dom_flops / (arithmetic_tflops * 1e12) * 1e3)
         line = {
             "metric": "spmm_batch_gflops", "value": value, "unit": "GFLOP/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_per_step,
@@ -1235,7 +1241,7 @@ def main():
                          "algorithmic_bytes_per_launch": dom["algorithmic_bytes_per_launch"],
                          "fp32_peak_tflops_measured": fp32_tflops,
                          "fp32_frac": dom["fp32_frac"],
-                         "binding_roof": "hbm" if dom["algorithmic_bytes_per_launch"] / (hbm_gbs * 1e9) >= dom_flops / (fp32_tflops * 1e12) else "fp32",
+                         "binding_roof": "hbm" if t_hbm_ms >= t_roof_ms else "bf16 tensor rate / 6" if on_tensor_cores else "fp32",
                          "roof_frac": t_roof_ms / launch_avg_ms,
                          "step_ms_rank0": step_avg_ms, "kernels": parts},
             "extras": extras,
